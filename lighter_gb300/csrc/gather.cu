@@ -8,7 +8,7 @@
 // whose left operand G (N x N) streams from HBM once per bounce while X
 // (N x R) stays in L2.
 //
-//   FP32        G in FP32, register-blocked SIMT GEMM              k_sgemm_bounce
+//   FP32        G in FP32, SIMT stream-K GEMM                       k_sgemm_bounce
 //   FP16/BF16   G in 16 bits on the tcgen05 tensor cores            k_umma_gather
 //               (FP32 accumulation in TMEM), with optional head/tail
 //               splits of X and of G (LTRG_REFINE_*) whose extra products
@@ -415,105 +415,204 @@ __global__ void __launch_bounds__(256) k_combine(u32 n, u32 ld, u32 R, u32 Rpad,
 
 // ----------------------------------------------------------------------------- FP32 SIMT gather
 
-// B_new = E + G X, G (n x n FP32), X (n x R FP32, row-major): 128 x 192 tile
-// per block, 16 x 16 threads with 8 x 12 outputs each, k tiles of 16 in two
-// shared-memory buffers (one barrier per tile); the next tile's global loads
-// are in flight in registers while the current tile is consumed.
-constexpr int SBM = 128, SBN = 192, SBK = 16;
-__global__ void __launch_bounds__(256) k_sgemm_bounce(u32 n, u32 R, const float* __restrict__ G,
-                                                      const float* __restrict__ X, const float* __restrict__ E,
-                                                      float* __restrict__ Bnew)
+// Partial sums of G X for FP32 (G n x n, row stride ldg a multiple of 4; X^T rows
+// of ldx floats, zero past n and past R). Bound by the FP32 pipes (G streams at a
+// fifth of HBM's rate), so the shape serves the multiply-adds:
+//  * both operands lie k-contiguous in shared memory (no transposition on the way
+//    in); a thread owns 16 rows ty + 8 i and TN columns tx + 16 j and reads four k at a
+//    time, 16 + TN 16-byte loads for 64 TN multiply-adds. A warp spans 4 x 8 threads,
+//    so with rows padded to 36 floats its loads touch 4 (G) or 8 (X) different rows
+//    on different banks.
+//  * 128 x (16 TN) tiles, k blocks of 32 in three cp.async stages, 128 threads, two
+//    blocks per SM.
+//  * the (tile, k block) units are cut into equal contiguous ranges, one per
+//    resident block, so the SMs stay filled whatever n and R are; a block writes the
+//    sums of each tile it touches into its slot of that tile and k_combine32 adds
+//    the slots in order (deterministic, and shorter sums than one range of n).
+// TN by R (sgemm_tn): the least padding wins, with a charge per tile for G's re-read.
+// Measured, n = 8192: R = 96 1541 -> 262 us a bounce (50 TFLOP/s; the 128 x 192 tile on
+// 64 blocks before), R = 192 515 us. Tried: fma.rn.f32x2 on k pairs 46 TFLOP/s (its
+// 64-bit operands cost the register ports what it saves in issue slots); 8 x 6 and
+// 8 x 12 per thread 47 and 49.
+constexpr int SGM = 128, SGK = 32, SGS = SGK + 4, SGStages = 3, SGThreads = 128, SGBlocksPerSM = 2;
+
+struct SgemmArgs {
+    u32 n, ldg, ldx, nkb;     // rows, strides of G and X^T, k blocks
+    u32 tiles_n, max_slots;
+    uint64_t total;           // (tile, k block) units
+    const float* G;
+    const float* XT;
+    float* partial;           // [tile][slot][SGM][16 TN]
+};
+
+// Which of `n_cta` equal ranges of `total` units holds unit u.
+__host__ __device__ __forceinline__ u32 range_of(uint64_t u, uint64_t total, u32 n_cta)
 {
-    __shared__ __align__(16) float As[2][SBK][SBM + 4];
-    __shared__ __align__(16) float Bs[2][SBK][SBN];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const u32 m0 = blockIdx.x * SBM, n0 = blockIdx.y * SBN;
-    // loader coordinates: A 128 rows x 16 k (row ar, k ak..ak+7); B 16 k x 192 (k bk, cols bc..bc+11)
-    const int ar = tid >> 1, ak = (tid & 1) * 8, bk = tid >> 4, bc = (tid & 15) * 12;
-    float pa[8], pb[12];
-    auto fetch = [&](u32 k0) {
-        const u32 gi = m0 + ar;
+    return (u32) (((u + 1) * n_cta + total - 1) / total - 1);
+}
+
+__device__ __forceinline__ void cp16(float* dst, const float* src, bool in)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(saddr(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+
+__device__ __forceinline__ float f4at(const float4& v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
+
+template <int TN>
+__global__ void __launch_bounds__(SGThreads, SGBlocksPerSM) k_sgemm_bounce(SgemmArgs a)
+{
+    constexpr int BN = 16 * TN, TM = SGM / 8, STAGE = (SGM + BN) * SGS, CG = SGM / 16, CX = BN / 16;
+    extern __shared__ __align__(16) float sm[];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int ty = (w >> 1) * 4 + (lane >> 3), tx = (w & 1) * 8 + (lane & 7);
+    const uint64_t lo = (uint64_t) blockIdx.x * a.total / gridDim.x, hi = (uint64_t) (blockIdx.x + 1) * a.total / gridDim.x;
+    // copies: 8 chunks of 16 bytes per row of a stage; this thread's are rows tid / 8 + 16 t
+    const int cr = tid >> 3, cc = (tid & 7) * 4;
+    u32 ft = (u32) (lo / a.nkb), fk = (u32) (lo % a.nkb);   // the next unit to fetch
+    const float* gp[CG];
+    bool gin[CG];
+    const float* xp;
+    auto seek = [&]() {
+        const u32 m0 = ft / a.tiles_n * SGM, n0 = ft % a.tiles_n * BN;
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const u32 gk = k0 + ak + t;
-            pa[t] = (gi < n && gk < n) ? __ldg(&G[(size_t) gi * n + gk]) : 0.0f;
+        for (int t = 0; t < CG; ++t) {
+            const u32 m = m0 + cr + 16 * t;
+            gin[t] = m < a.n;
+            gp[t] = a.G + (gin[t] ? (size_t) m * a.ldg : 0) + fk * SGK + cc;
         }
-        const u32 gk = k0 + bk;
+        xp = a.XT + (size_t) (n0 + cr) * a.ldx + fk * SGK + cc;
+    };
+    seek();
+    auto fetch = [&](int stage) {
+        float* S = sm + stage * STAGE + cr * SGS + cc;
+        const bool kin = fk * SGK + cc < a.ldg;
 #pragma unroll
-        for (int t = 0; t < 12; ++t) {
-            const u32 gc = n0 + bc + t;
-            pb[t] = (gk < n && gc < R) ? __ldg(&X[(size_t) gk * R + gc]) : 0.0f;
+        for (int t = 0; t < CG; ++t) {
+            cp16(S + 16 * t * SGS, gin[t] && kin ? gp[t] : a.G, gin[t] && kin);
+            gp[t] += SGK;
+        }
+#pragma unroll
+        for (int t = 0; t < CX; ++t) cp16(S + (SGM + 16 * t) * SGS, xp + (size_t) (16 * t) * a.ldx, true);
+        xp += SGK;
+        if (++fk == a.nkb) {
+            fk = 0;
+            ++ft;
+            seek();
         }
     };
-    auto stash = [&](int buf) {
+    float acc[TM][TN];
 #pragma unroll
-        for (int t = 0; t < 8; ++t) As[buf][ak + t][ar] = pa[t];
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int t = 0; t < 12; ++t) Bs[buf][bk][bc + t] = pb[t];
-    };
-    float acc[8][12];
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 12; ++j) acc[i][j] = 0.0f;
-    fetch(0);
-    stash(0);
-    __syncthreads();
-    int cur = 0;
-    for (u32 k0 = 0; k0 < n; k0 += SBK) {
-        const bool more = k0 + SBK < n;
-        if (more) fetch(k0 + SBK);
-#pragma unroll
-        for (int k = 0; k < SBK; ++k) {
-            const float4 a0 = *reinterpret_cast<const float4*>(&As[cur][k][ty * 8]);
-            const float4 a1 = *reinterpret_cast<const float4*>(&As[cur][k][ty * 8 + 4]);
-            const float4 b0 = *reinterpret_cast<const float4*>(&Bs[cur][k][tx * 12]);
-            const float4 b1 = *reinterpret_cast<const float4*>(&Bs[cur][k][tx * 12 + 4]);
-            const float4 b2 = *reinterpret_cast<const float4*>(&Bs[cur][k][tx * 12 + 8]);
-            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            const float bv[12] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w, b2.x, b2.y, b2.z, b2.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 12; ++j) acc[i][j] = __fmaf_rn(av[i], bv[j], acc[i][j]);
-        }
-        if (more) stash(cur ^ 1);
-        __syncthreads();
-        cur ^= 1;
+    for (int q = 0; q < SGStages - 1; ++q) {
+        if (lo + q < hi) fetch(q);
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
+    int stage = 0;
+    u32 ct = (u32) (lo / a.nkb), ck = (u32) (lo % a.nkb);   // the unit being summed
+    for (uint64_t u = lo; u < hi; ++u) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(SGStages - 2) : "memory");
+        __syncthreads();   // stage `stage` has landed, and everyone is done with the one refilled here
+        if (u + SGStages - 1 < hi) fetch(stage == 0 ? SGStages - 1 : stage - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float* As = sm + stage * STAGE + ty * SGS;
+        const float* Bs = sm + stage * STAGE + (SGM + tx) * SGS;
+#pragma unroll 2
+        for (int k = 0; k < SGK; k += 4) {
+            float4 b[TN];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const u32 gi = m0 + ty * 8 + i;
-        if (gi >= n) continue;
+            for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const float4*>(Bs + 16 * j * SGS + k);
 #pragma unroll
-        for (int j = 0; j < 12; ++j) {
-            const u32 gc = n0 + tx * 12 + j;
-            if (gc < R) {
-                const size_t o = (size_t) gi * R + gc;
-                Bnew[o] = E[o] + acc[i][j];
+            for (int i = 0; i < TM; ++i) {
+                const float4 av = *reinterpret_cast<const float4*>(As + 8 * i * SGS + k);
+#pragma unroll
+                for (int h = 0; h < 4; ++h)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) acc[i][j] = __fmaf_rn(f4at(av, h), f4at(b[j], h), acc[i][j]);
             }
+        }
+        stage = stage + 1 == SGStages ? 0 : stage + 1;
+        ++ck;
+        if (u + 1 == hi || ck == a.nkb) {   // the end of this block's part of the tile
+            const u32 slot = blockIdx.x - range_of((uint64_t) ct * a.nkb, a.total, gridDim.x);
+            float* P = a.partial + ((size_t) ct * a.max_slots + slot) * (SGM * BN);
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    P[(ty + 8 * i) * BN + tx + 16 * j] = acc[i][j];
+                    acc[i][j] = 0.0f;
+                }
+            ck = 0;
+            ++ct;
         }
     }
 }
 
-// X_j(r) = albedo_j(r mod 3) B_j(r), FP32 row-major.
-__global__ void k_make_x32(u32 n, u32 R, const float* __restrict__ albedo, const float* __restrict__ B,
-                           float* __restrict__ X)
+// One 32 (patches) x 32 (right-hand sides) tile of a bounce: B = E + the tile's
+// slots in order (no slots: B = E), and the next X^T[r][j] = albedo_j(r mod 3) B,
+// zero for j >= n or r >= R. B_out and xt may be null (not wanted).
+__global__ void __launch_bounds__(256) k_combine32(u32 n, u32 ldx, u32 R, u32 BN, u32 tiles_n, u32 nkb, uint64_t total,
+                                                   u32 n_cta, u32 max_slots, const float* __restrict__ partial,
+                                                   const float* __restrict__ E, const float* __restrict__ albedo,
+                                                   float* __restrict__ B_out, float* __restrict__ xt)
 {
-    const size_t t = blockIdx.x * (size_t) blockDim.x + threadIdx.x;
-    if (t >= (size_t) n * R) return;
-    const u32 j = (u32) (t / R), r = (u32) (t % R);
-    X[t] = albedo[3 * j + r % 3] * B[t];
+    __shared__ float tile[32][33];
+    const u32 j0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    // 32 divides the tile's rows and its BN columns: one product tile for the block
+    const u32 t = j0 / SGM * tiles_n + r0 / BN;
+    u32 cnt = 0;
+    if (partial && j0 < n)
+        cnt = range_of((uint64_t) (t + 1) * nkb - 1, total, n_cta) - range_of((uint64_t) t * nkb, total, n_cta) + 1;
+    const float* P = partial ? partial + (size_t) t * max_slots * (SGM * BN) + (size_t) (j0 % SGM) * BN + r0 % BN + tx : nullptr;
+    const u32 r = r0 + tx;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const u32 k = ty + 8 * i, j = j0 + k;
+        float x = 0.0f;
+        if (j < n && r < R) {
+            float v = 0.0f;
+            for (u32 s = 0; s < cnt; ++s) v += __ldg(&P[(size_t) s * (SGM * BN) + (size_t) k * BN]);
+            const float b = E[(size_t) j * R + r] + v;
+            if (B_out) B_out[(size_t) j * R + r] = b;
+            x = albedo[3 * j + r % 3] * b;
+        }
+        tile[k][tx] = x;
+    }
+    if (!xt) return;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const u32 rr = r0 + ty + 8 * i, j = j0 + tx;
+        if (j < ldx) xt[(size_t) rr * ldx + j] = tile[tx][ty + 8 * i];
+    }
+}
+
+// Column groups of 16 per tile (TN of k_sgemm_bounce) for R right-hand sides: the
+// least ceil(R / BN) (BN + 24). The 24 columns per tile stand for reading G once more.
+int sgemm_tn(u32 R)
+{
+    int best = 6;
+    u32 cost = UINT32_MAX;
+    for (int tn : {6, 4, 2}) {
+        const u32 bn = 16 * (u32) tn, c = (R + bn - 1) / bn * (bn + 24);
+        if (c < cost) { cost = c; best = tn; }
+    }
+    return best;
 }
 
 // ----------------------------------------------------------------------------- G preparation
 
-// G_ij = F_ij * area_j, in place.
-__global__ void k_scale_cols(u32 n, float* __restrict__ G, const float* __restrict__ area)
+// G_ij = F_ij * area_j, in place (row stride ldg; the padding columns stay 0).
+__global__ void k_scale_cols(u32 n, u32 ldg, float* __restrict__ G, const float* __restrict__ area)
 {
     const size_t t = blockIdx.x * (size_t) blockDim.x + threadIdx.x;
-    if (t >= (size_t) n * n) return;
-    G[t] *= area[t % n];
+    if (t >= (size_t) n * ldg) return;
+    const u32 j = (u32) (t % ldg);
+    if (j < n) G[t] *= area[j];
 }
 
 // *out = max |x| as float bits (non-negative floats order like their bits); *out starts at 0.
@@ -528,13 +627,13 @@ __global__ void k_absmax(const float* __restrict__ x, size_t count, u32* out)
 
 // hi = 16-bit 2^g_exp G (row stride ld, zero columns j >= n); lo = 16-bit residual when requested.
 template <class T>
-__global__ void k_g_to_16(u32 n, u32 ld, const float* __restrict__ G, T* __restrict__ hi, T* __restrict__ lo,
+__global__ void k_g_to_16(u32 n, u32 ld, u32 ldg, const float* __restrict__ G, T* __restrict__ hi, T* __restrict__ lo,
                           float gscale)
 {
     const size_t t = blockIdx.x * (size_t) blockDim.x + threadIdx.x;
     if (t >= (size_t) n * ld) return;
     const u32 i = (u32) (t / ld), j = (u32) (t % ld);
-    const float g = j < n ? G[(size_t) i * n + j] * gscale : 0.0f;
+    const float g = j < n ? G[(size_t) i * ldg + j] * gscale : 0.0f;
     const T h = to16<T>(g);
     hi[t] = h;
     if (lo) lo[t] = to16<T>(g - from16(h));
@@ -782,7 +881,8 @@ struct ltrg_Gather {
     int sm_count = 0;
     cudaStream_t st = nullptr;
     u32 n = 0, ld = 0;
-    DevBuf G32;                   // n x n FP32
+    u32 ldg = 0;                  // row stride of G32: n rounded up to 4 floats (16-byte rows), zeros past n
+    DevBuf G32;                   // n x ldg FP32
     DevBuf G16, G16lo;            // n x ld 16-bit head and residual
     int g16_kind = -1;            // precision held in G16 (-1: none)
     int g_exp = 0;                // G16 holds 2^g_exp G: max |G| maps below 2^14
@@ -792,7 +892,7 @@ struct ltrg_Gather {
     u32 kchunk = 0;               // k blocks per TMEM accumulation (0: whole range of a CTA)
     DevBuf rp_tab;                // rp_first[n_rp], rp_cnt[n_rp]
     // solve scratch
-    DevBuf partial, xh, xl, x32, btmp, err, emax;
+    DevBuf partial, xh, xl, x32, err, emax;
     DevBuf h_alb, h_E, h_out;     // device copies for the host-buffer entry point
     PinBuf pin_in, pin_out;       // its page-locked staging
     std::unique_ptr<StagePool> pool;   // its host copy threads (started by the first host-buffer solve)
@@ -810,7 +910,7 @@ struct ltrg_Gather {
         cudaSetDevice(device);
         cudaStreamSynchronize(st);
         DevBuf* all[] = {&G32,  &G16, &G16lo, &rp_tab, &partial, &xh,    &xl,
-                         &x32,  &btmp, &err,  &emax,   &h_alb,   &h_E,   &h_out};
+                         &x32,  &err,  &emax,   &h_alb,   &h_E,   &h_out};
         for (DevBuf* b : all) b->release();
         pin_in.release();
         pin_out.release();
@@ -867,27 +967,41 @@ void ltrg_Gather::solve(const float* alb, const float* E, u32 R, int bounces, in
     } evg{ev};
     double ms_convert = 0, ms_gemm = 0, ms_bounces = 0;
     int stages = 0, products = 1;
+    int32_t ctas32 = 0;
     uint64_t bytes_bounce = 0;
 
     if (!tc) {
-        // FP32: ping-pong between btmp and out so the last bounce lands in out
-        btmp.ensure((size_t) n * R * 4);
-        x32.ensure((size_t) n * R * 4);
-        float* cur = (bounces % 2 == 0) ? out : btmp.as<float>();
-        float* nxt = (bounces % 2 == 0) ? btmp.as<float>() : out;
-        GCK(cudaMemcpyAsync(cur, E, (size_t) n * R * 4, cudaMemcpyDeviceToDevice, s));
+        const int tn = sgemm_tn(R);
+        const u32 bn = 16 * (u32) tn, tiles_n = (R + bn - 1) / bn, tiles_m = (n + SGM - 1) / SGM;
+        const u32 skb = (ldg + SGK - 1) / SGK, ldx = skb * SGK;
+        const uint64_t total = (uint64_t) tiles_m * tiles_n * skb;
+        const u32 sg_cta = (u32) std::min<uint64_t>((uint64_t) sm_count * SGBlocksPerSM, total);
+        // slots: the most ranges that one tile's units can fall into
+        const u32 slots = (u32) std::min<uint64_t>(sg_cta, ((uint64_t) skb * sg_cta + total - 1) / total + 1);
+        partial.ensure((size_t) tiles_m * tiles_n * slots * SGM * bn * 4);
+        x32.ensure((size_t) tiles_n * bn * ldx * 4);
+        const dim3 cb(32, 8), cg((ldx + 31) / 32, tiles_n * bn / 32);
+        auto combine = [&](bool with_partial, bool last) {
+            k_combine32<<<cg, cb, 0, s>>>(n, ldx, R, bn, tiles_n, skb, total, sg_cta, slots,
+                                          with_partial ? partial.as<float>() : nullptr, E, alb, last ? out : nullptr,
+                                          last ? nullptr : x32.as<float>()); note_launch();
+            GCK(cudaGetLastError());
+        };
+        const SgemmArgs sa{n, ldg, ldx, skb, tiles_n, slots, total, G32.as<float>(), x32.as<float>(), partial.as<float>()};
+        auto kern = tn == 6 ? k_sgemm_bounce<6> : tn == 4 ? k_sgemm_bounce<4> : k_sgemm_bounce<2>;
+        const size_t sg_smem = (size_t) SGStages * (SGM + bn) * SGS * 4;
+        GCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sg_smem));
+        ctas32 = (int32_t) sg_cta;
         cudaEvent_t e0 = event();
+        combine(false, bounces == 0);
         std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ge;
         for (int b = 0; b < bounces; ++b) {
-            const size_t tot = (size_t) n * R;
-            k_make_x32<<<(unsigned) ((tot + 255) / 256), 256, 0, s>>>(n, R, alb, cur, x32.as<float>()); note_launch();
             cudaEvent_t g0 = event();
-            dim3 grid((n + SBM - 1) / SBM, (R + SBN - 1) / SBN);
-            k_sgemm_bounce<<<grid, 256, 0, s>>>(n, R, G32.as<float>(), x32.as<float>(), E, nxt); note_launch();
+            kern<<<sg_cta, SGThreads, sg_smem, s>>>(sa); note_launch();
             cudaEvent_t g1 = event();
             ge.push_back({g0, g1});
             GCK(cudaGetLastError());
-            std::swap(cur, nxt);
+            combine(true, b + 1 == bounces);
         }
         cudaEvent_t e1 = event();
         GCK(cudaStreamSynchronize(s));
@@ -906,10 +1020,10 @@ void ltrg_Gather::solve(const float* alb, const float* E, u32 R, int bounces, in
             const unsigned grid = (unsigned) ((tot + 255) / 256);
             const float gscale = ldexpf(1.0f, g_exp);
             if (precision == LTRG_F_FP16)
-                k_g_to_16<__half><<<grid, 256, 0, s>>>(n, ld, G32.as<float>(), G16.as<__half>(),
+                k_g_to_16<__half><<<grid, 256, 0, s>>>(n, ld, ldg, G32.as<float>(), G16.as<__half>(),
                                                        need_lo ? G16lo.as<__half>() : nullptr, gscale);
             else
-                k_g_to_16<__nv_bfloat16><<<grid, 256, 0, s>>>(n, ld, G32.as<float>(), G16.as<__nv_bfloat16>(),
+                k_g_to_16<__nv_bfloat16><<<grid, 256, 0, s>>>(n, ld, ldg, G32.as<float>(), G16.as<__nv_bfloat16>(),
                                                               need_lo ? G16lo.as<__nv_bfloat16>() : nullptr, gscale);
             note_launch();
             GCK(cudaGetLastError());
@@ -1015,7 +1129,7 @@ void ltrg_Gather::solve(const float* alb, const float* E, u32 R, int bounces, in
         stats->pairs = pairs;
         stats->tensor_cores = tc ? 1 : 0;
         stats->stages = stages;
-        stats->ctas = tc ? (int32_t) n_cta : (int32_t) (((n + SBM - 1) / SBM) * ((R + SBN - 1) / SBN));
+        stats->ctas = tc ? (int32_t) n_cta : ctas32;
         stats->products = tc ? products : 1;
     }
 }
@@ -1039,6 +1153,7 @@ LTRAPI ltrg_Gather* ltrg_GatherCreate(const float* tri_xyz, u32 n_tris, const fl
         GCK(cudaStreamCreateWithFlags(&g->st, cudaStreamNonBlocking));
         g->n = n;
         g->ld = (n + BK - 1) / BK * BK;
+        g->ldg = (n + 3) / 4 * 4;
         cudaStream_t st = g->st;
 
         // occluder BVH (one instance, every triangle casts shadows)
@@ -1091,16 +1206,16 @@ LTRAPI ltrg_Gather* ltrg_GatherCreate(const float* tri_xyz, u32 n_tris, const fl
         const float* da = (const float*) up(area, n * sizeof(float));
         u32* derr = (u32*) up(nullptr, 0);
         GCK(cudaMemsetAsync(derr, 0, 4, st));
-        g->G32.ensure((size_t) n * n * 4);
+        g->G32.ensure((size_t) n * g->ldg * 4);
 
         cudaEvent_t e0, e1;
         GCK(cudaEventCreate(&e0));
         GCK(cudaEventCreate(&e1));
         GCK(cudaEventRecord(e0, st));
         BvhView view = bin.n ? bvh.view() : BvhView{nullptr, nullptr, nullptr, nullptr, 0, 0};
-        RadFormFactors ff = radiosity_form_factors_f32(n, dp, dn, view, ErrFlag{derr}, links, g->G32.as<float>(), st);
-        const size_t nn2 = (size_t) n * n;
-        k_scale_cols<<<(unsigned) ((nn2 + 255) / 256), 256, 0, st>>>(n, g->G32.as<float>(), da); note_launch();
+        RadFormFactors ff = radiosity_form_factors_f32(n, g->ldg, dp, dn, view, ErrFlag{derr}, links, g->G32.as<float>(), st);
+        const size_t nn2 = (size_t) n * g->ldg;
+        k_scale_cols<<<(unsigned) ((nn2 + 255) / 256), 256, 0, st>>>(n, g->ldg, g->G32.as<float>(), da); note_launch();
         GCK(cudaGetLastError());
         GCK(cudaEventRecord(e1, st));
         u32* dgmax = (u32*) up(nullptr, 0);
@@ -1153,7 +1268,9 @@ LTRAPI LTRBOOL ltrg_GatherGetG(ltrg_Gather* g, float* out)
     std::lock_guard<std::mutex> lk(g->mu);
     if (cudaSetDevice(g->device) != cudaSuccess) return 0;
     if (cudaStreamSynchronize(g->st) != cudaSuccess) return 0;
-    if (cudaMemcpy(out, g->G32.p, (size_t) g->n * g->n * 4, cudaMemcpyDeviceToHost) != cudaSuccess) return 0;
+    if (cudaMemcpy2D(out, (size_t) g->n * 4, g->G32.p, (size_t) g->ldg * 4, (size_t) g->n * 4, g->n, cudaMemcpyDeviceToHost) !=
+        cudaSuccess)
+        return 0;
     return 1;
 }
 

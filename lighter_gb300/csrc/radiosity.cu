@@ -709,10 +709,10 @@ RadResult radiosity_solve_dev(const RadDevInputs& in, const RadSettings& rs, con
     return solve_t<float>(in, rs, bvh, err, st, total_out, abort_flag);
 }
 
-RadFormFactors radiosity_form_factors_f32(uint32_t n, const float4* pos, const float4* nrm, const BvhView& bvh,
+RadFormFactors radiosity_form_factors_f32(uint32_t n, size_t ld, const float4* pos, const float4* nrm, const BvhView& bvh,
                                           ErrFlag err, int links, float* F, cudaStream_t st)
 {
-    return build_ff<float>(n, n, pos, nrm, bvh, err, links, F, nullptr, nullptr, st);
+    return build_ff<float>(n, ld, pos, nrm, bvh, err, links, F, nullptr, nullptr, st);
 }
 
 RadResult radiosity_solve(const RadInputs& in, const RadSettings& rs, const BvhView& bvh, ErrFlag err, cudaStream_t st,

@@ -51,14 +51,14 @@ struct RadDevInputs {
 RadResult radiosity_solve_dev(const RadDevInputs& in, const RadSettings& rs, const BvhView& bvh, ErrFlag err,
                               cudaStream_t st, float4* total_out, std::atomic<bool>* abort_flag);
 
-// Only the form factors: F (n x n FP32, row-major) with the pair test and the
+// Only the form factors: F (n rows of ld >= n FP32, zero past n) with the pair test and the
 // `links` predicate, in two passes (pair tests, then the visibility rays of the
 // pairs that passed); returns the link and visibility-ray counts (synchronises
 // the stream).
 struct RadFormFactors {
     uint64_t links = 0, vis_rays = 0;
 };
-RadFormFactors radiosity_form_factors_f32(uint32_t n, const float4* pos, const float4* nrm, const BvhView& bvh,
+RadFormFactors radiosity_form_factors_f32(uint32_t n, size_t ld, const float4* pos, const float4* nrm, const BvhView& bvh,
                                           ErrFlag err, int links, float* F, cudaStream_t st);
 
 // Same from host vectors (uploads them first).
