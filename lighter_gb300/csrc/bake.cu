@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "bvh.cuh"
+#include "finalize.cuh"
 #include "radiosity.cuh"
 #include "reftree.hpp"
 #include "scene.hpp"
@@ -1526,55 +1527,39 @@ __device__ __forceinline__ int find_inst(const unsigned long long* off, int n_in
     return lo;
 }
 
-__global__ void k_scatter(u32 n_probe, u32 n_samples, const u32* __restrict__ sloc, const u32* __restrict__ sinst,
-                          const float4* __restrict__ lm, const unsigned long long* __restrict__ tex_off,
-                          float* __restrict__ img, unsigned char* __restrict__ mask)
-{
-    u32 s = n_probe + blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n_samples) return;
-    unsigned long long g = tex_off[sinst[s]] + sloc[s];
-    float4 c = lm[s];
-    img[3 * g + 0] = c.x;
-    img[3 * g + 1] = c.y;
-    img[3 * g + 2] = c.z;
-    mask[g] = 1;
-}
+// One lightmap of the finalize pass: its first texel, its size and its first tile.
+struct FinInst {
+    unsigned long long off;
+    u32 w, h, tile0, tiles_x;
+};
 
-// One extrapolating dilation sweep (lighter.cpp:884-943): `old` is the mask
-// before the sweep, `next` receives newly set texels; colours of texels set
-// in `old` are never written during the sweep, so reading them is race-free.
-__global__ void k_dilate(unsigned long long ntex, int n_inst, const unsigned long long* __restrict__ tex_off,
-                         const u32* __restrict__ inst_w, const u32* __restrict__ inst_h,
-                         const unsigned char* __restrict__ old, unsigned char* __restrict__ next, float* img)
+// Scatter, dilation sweeps and blur of every lightmap in one launch
+// (finalize.cuh): a block finds its lightmap and tile, and a covered texel's
+// colour is read straight from its sample (`scan` holds the covered texels
+// before each texel), so no scattered image or mask is written first. Bound by
+// L2 (the halo reads each texel 2.1 times at the default blur).
+__global__ void __launch_bounds__(kFinThreads) k_finalize(const FinInst* __restrict__ fi, int n, int ext, FinTaps taps,
+                                                          u32 n_probe, const u32* __restrict__ scan,
+                                                          const float4* __restrict__ lm, float* __restrict__ img)
 {
-    for (unsigned long long g = blockIdx.x * (unsigned long long) blockDim.x + threadIdx.x; g < ntex;
-         g += (unsigned long long) gridDim.x * blockDim.x) {
-        if (old[g]) continue;
-        int inst = find_inst(tex_off, n_inst, g);
-        unsigned long long base = tex_off[inst];
-        u32 w = inst_w[inst], h = inst_h[inst];
-        unsigned long long local = g - base;
-        u32 x = (u32) (local % w), y = (u32) (local / w);
-        auto isset = [&](u32 xx, u32 yy) { return xx < w && yy < h && old[base + xx + (unsigned long long) yy * w]; };
-        auto col = [&](u32 xx, u32 yy) {
-            const float* p = img + 3 * (base + xx + (unsigned long long) yy * w);
-            return mk(p[0], p[1], p[2]);
-        };
-        V3 c = mk(0, 0, 0);
-        int cnt = 0;
-        if (isset(x - 1, y)) { c += isset(x - 2, y) ? lerp3(col(x - 2, y), col(x - 1, y), 2.0f) : col(x - 1, y); cnt++; }
-        if (isset(x + 1, y)) { c += isset(x + 2, y) ? lerp3(col(x + 2, y), col(x + 1, y), 2.0f) : col(x + 1, y); cnt++; }
-        if (isset(x, y - 1)) { c += isset(x, y - 2) ? lerp3(col(x, y - 2), col(x, y - 1), 2.0f) : col(x, y - 1); cnt++; }
-        if (isset(x, y + 1)) { c += isset(x, y + 2) ? lerp3(col(x, y + 2), col(x, y + 1), 2.0f) : col(x, y + 1); cnt++; }
-        if (cnt) {
-            c = c / (float) cnt;
-            float* p = img + 3 * g;
-            p[0] = fmax_(c.x, 0.0f);
-            p[1] = fmax_(c.y, 0.0f);
-            p[2] = fmax_(c.z, 0.0f);
-            next[g] = 1;
-        }
+    extern __shared__ __align__(16) unsigned char smem[];
+    int lo = 0, hi = n - 1;   // the last lightmap with tile0 <= block
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (fi[mid].tile0 <= blockIdx.x) lo = mid; else hi = mid - 1;
     }
+    const FinInst f = fi[lo];
+    const u32 t = blockIdx.x - f.tile0;
+    const u32* sc = scan + f.off;
+    fin_tile((int) (t % f.tiles_x), (int) (t / f.tiles_x), (int) f.w, (int) f.h, ext, taps,
+             [&](size_t g, float* c) {
+                 const u32 k = sc[g];
+                 if (sc[g + 1] == k) return false;
+                 const float4 v = lm[n_probe + k];
+                 c[0] = v.x; c[1] = v.y; c[2] = v.z;
+                 return true;
+             },
+             img + 3 * f.off, smem);
 }
 
 // Row convolution with clamp-to-edge taps, written transposed
@@ -3305,32 +3290,38 @@ void run_bake(ltr_Scene* S)
 
     // ---- finalize (Int_Finalize)
     S->stage = "exporting lightmaps";
-    float* d_img = A.zeros<float>(3 * ntex);
-    unsigned char* d_maskA = A.zeros<unsigned char>(ntex);
-    unsigned char* d_maskB = A.alloc<unsigned char>(ntex);
-    if (n_cov) {
-        k_scatter<<<(n_cov + kThreads - 1) / kThreads, kThreads, 0, st>>>(n_probe, n_samples, d_sloc, d_sinst, d_lm,
-                                                                          d_tex_off, d_img, d_maskA); note_launch();
+    float* d_img = A.alloc<float>(3 * ntex);
+    const int blur_ext = cfg.blur_size && ntex ? (int) ceilf(cfg.blur_size) : 0;
+    std::vector<float> taps;
+    if (blur_ext) taps = gauss_taps(blur_ext, cfg.blur_size);
+    if (ntex) {
+        std::vector<FinInst> fin;
+        unsigned long long n_tiles = 0;
+        for (int i = 0; i < n_inst; ++i) {
+            if (!inst_w[i] || !inst_h[i]) continue;
+            const u32 tx = (inst_w[i] + kFinTile - 1) / kFinTile;
+            fin.push_back(FinInst{tex_off[i], inst_w[i], inst_h[i], (u32) n_tiles, tx});
+            n_tiles += (unsigned long long) tx * ((inst_h[i] + kFinTile - 1) / kFinTile);
+        }
+        if (n_tiles > 0x7fffffffull) throw std::runtime_error("too many lightmap tiles for one bake");
+        // a blur too wide for a tile's halo runs as separate convolutions below
+        const int fin_ext = blur_ext <= kFinMaxExt ? blur_ext : 0;
+        FinTaps ft = {};
+        if (fin_ext) memcpy(ft.k, taps.data(), taps.size() * sizeof(float));
+        const size_t smem = fin_smem(fin_ext);
+        if (smem > 48 * 1024) CK(cudaFuncSetAttribute(k_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+        FinInst* d_fin = A.upload(fin);
+        k_finalize<<<(unsigned) n_tiles, kFinThreads, smem, st>>>(d_fin, (int) fin.size(), fin_ext, ft, n_probe, d_scan,
+                                                                  d_lm, d_img); note_launch();
         CK(cudaGetLastError());
     }
-    if (ntex) {
-        for (int it = 0; it < 3; ++it) {
-            CK(cudaMemcpyAsync(d_maskB, d_maskA, ntex, cudaMemcpyDeviceToDevice, st));
-            k_dilate<<<blocks_for(ntex), kThreads, 0, st>>>(ntex, n_inst, d_tex_off, d_inst_w, d_inst_h, d_maskA,
-                                                            d_maskB, d_img); note_launch();
-            CK(cudaGetLastError());
-            std::swap(d_maskA, d_maskB);
-        }
-    }
-    if (cfg.blur_size && ntex) {
-        int ext = (int) ceilf(cfg.blur_size);
-        std::vector<float> taps = gauss_taps(ext, cfg.blur_size);
+    if (blur_ext > kFinMaxExt) {
         float* d_taps = A.upload(taps);
         float* d_tmp = A.alloc<float>(3 * ntex);
-        k_conv_t<<<blocks_for(ntex), kThreads, 0, st>>>(ntex, n_inst, d_tex_off, d_inst_w, d_inst_h, 0, ext, d_taps,
+        k_conv_t<<<blocks_for(ntex), kThreads, 0, st>>>(ntex, n_inst, d_tex_off, d_inst_w, d_inst_h, 0, blur_ext, d_taps,
                                                         d_img, d_tmp); note_launch();
         CK(cudaGetLastError());
-        k_conv_t<<<blocks_for(ntex), kThreads, 0, st>>>(ntex, n_inst, d_tex_off, d_inst_w, d_inst_h, 1, ext, d_taps,
+        k_conv_t<<<blocks_for(ntex), kThreads, 0, st>>>(ntex, n_inst, d_tex_off, d_inst_w, d_inst_h, 1, blur_ext, d_taps,
                                                         d_tmp, d_img); note_launch();
         CK(cudaGetLastError());
     }

@@ -1,0 +1,179 @@
+// The finalize step of a lightmap in one pass over its texels: three
+// extrapolating dilation sweeps, then the separable Gaussian blur
+// (lighter.cpp:880-961), for the bake (bake.cu) and for the entry point on
+// caller-owned buffers (noalloc.cu).
+//
+// As separate kernels (scatter, three mask copies and sweeps, two transposed
+// convolutions) the step was bound by launches on one lightmap and by eight
+// passes over memory on many. Here a block owns 32 x 32 texels and reads them
+// once with a halo of 6 + ext texels (a sweep looks two texels out, the blur
+// ext): sweeps and both convolutions run in shared memory, and the tile is
+// written once. The halo re-reads 2.1x the texels, from L2. One lightmap is a
+// block or two per SM, so a block's own chain of latencies is the time: 512
+// threads, four texels per thread read at once, and each thread remembers which
+// of its texels are uncovered, so a sweep touches no others. Measured: 512 x 512
+// at blur 0.5 13.3 us on the device and 16.4 us a call (30.9 and 53.6 as separate
+// kernels; 25.4 a call with 256 threads that rescan the region every sweep),
+// 1024 x 1024 33.8 us (90.5); a bake's stage on four 1024^2 lightmaps 0.34 -> 0.16 ms. The float
+// expressions and their order are those of the separate kernels, so the
+// results are the same bits.
+#pragma once
+
+#include "common.cuh"
+
+namespace lg {
+
+constexpr int kFinTile = 32, kFinThreads = 512;
+constexpr int kFinMaxExt = 16;   // largest ceil(blur_size) the tile's shared memory is laid out for
+
+struct FinTaps { float k[2 * kFinMaxExt + 1]; };
+
+// Region side (tile + halo) and shared memory: colours, masks, and the rows of
+// the first convolution.
+inline __host__ __device__ int fin_side(int ext) { return kFinTile + 2 * (6 + ext); }
+inline size_t fin_smem(int ext)
+{
+    const size_t s = (size_t) fin_side(ext);
+    return s * s * 12 + (s * s + 15) / 16 * 16 + (ext ? (size_t) kFinTile * (kFinTile + 2 * ext) * 12 : 0);
+}
+
+#ifdef __CUDACC__
+
+// One dilation of an unset texel from its set 4-neighbours, each extrapolated
+// linearly (2 c1 - c2) when the next texel out is set too; `m` and `col` point
+// at the texel in the region, `sweep` counts from 1, and a mask byte holds one
+// more than the sweep that set its texel (0: unset, or outside the image).
+// Returns whether the texel was set.
+__device__ __forceinline__ bool fin_dilate(unsigned char* m, float* col, int side, int sweep)
+{
+    V3 c = mk(0, 0, 0);
+    int cnt = 0;
+    auto isset = [&](int o) { const int v = m[o]; return v != 0 && v <= sweep; };
+    auto at = [&](int o) { return mk(col[3 * o], col[3 * o + 1], col[3 * o + 2]); };
+    const int dir[4] = {-1, 1, -side, side};
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+        const int o = dir[d];
+        if (isset(o)) {
+            c += isset(2 * o) ? lerp3(at(2 * o), at(o), 2.0f) : at(o);
+            cnt++;
+        }
+    }
+    if (!cnt) return false;
+    c = c / (float) cnt;
+    col[0] = fmax_(c.x, 0.0f);
+    col[1] = fmax_(c.y, 0.0f);
+    col[2] = fmax_(c.z, 0.0f);
+    m[0] = (unsigned char) (sweep + 1);
+    return true;
+}
+
+// Tile (bx, by) of a w x h image. load(g, c[3]) returns whether texel g (row
+// major) is covered and its colour; out receives the finished texels (row major,
+// not read). Every thread of the block calls it.
+template <class Load>
+__device__ __forceinline__ void fin_tile(int bx, int by, int w, int h, int ext, const FinTaps& taps, Load&& load,
+                                         float* __restrict__ out, unsigned char* smem)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kWarps = kFinThreads / 32;
+    const int halo = 6 + ext, side = fin_side(ext);
+    float* col = reinterpret_cast<float*>(smem);
+    unsigned char* msk = smem + (size_t) side * side * 12;
+    float* tmp = reinterpret_cast<float*>(msk + (side * side + 15) / 16 * 16);
+    const int x0 = bx * kFinTile - halo, y0 = by * kFinTile - halo;   // the region's corner
+    const int n = side * side;
+    // i / side for i < n: n < 2^13 and side < 2^7, so the rounded-up reciprocal of 20 bits is exact
+    const unsigned rcp = (0xfffffu + (unsigned) side) / (unsigned) side;
+    unsigned open = 0;   // bit k: this thread's texel k (threadIdx.x + k kFinThreads) is uncovered
+    constexpr int kBatch = 4;
+    for (int k0 = 0; k0 * kFinThreads < n; k0 += kBatch) {
+        float c[kBatch][3];
+        bool set[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            const int i = (int) threadIdx.x + (k0 + k) * kFinThreads;
+            const int y = (int) ((unsigned) i * rcp >> 20), gx = x0 + i - y * side, gy = y0 + y;
+            c[k][0] = c[k][1] = c[k][2] = 0.0f;
+            set[k] = false;
+            if (i < n && gx >= 0 && gx < w && gy >= 0 && gy < h) {
+                set[k] = load((size_t) gy * w + gx, c[k]);
+                if (!set[k]) open |= 1u << (k0 + k);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            const int i = (int) threadIdx.x + (k0 + k) * kFinThreads;
+            if (i < n) {
+                col[3 * i] = c[k][0]; col[3 * i + 1] = c[k][1]; col[3 * i + 2] = c[k][2];
+                msk[i] = set[k] ? 1 : 0;
+            }
+        }
+    }
+    if (__syncthreads_or(open != 0)) {   // some texel of the image in the region is uncovered
+        for (int s = 1; s <= 3; ++s) {
+            for (unsigned left = open; left; left &= left - 1) {
+                const int k = __ffs(left) - 1, i = (int) threadIdx.x + k * kFinThreads;
+                const int y = (int) ((unsigned) i * rcp >> 20), x = i - y * side;
+                if (x < 2 * s || y < 2 * s || x >= side - 2 * s || y >= side - 2 * s) continue;
+                if (fin_dilate(msk + i, col + 3 * i, side, s)) open &= ~(1u << k);
+            }
+            __syncthreads();
+        }
+    }
+    const int tx = bx * kFinTile + lane;
+    float* res = col;   // the finished tile: 32 rows of 96 floats
+    int res_stride = 3 * kFinTile;
+    if (ext) {
+        if (tx < w)
+            for (int r = warp; r < kFinTile + 2 * ext; r += kWarps) {   // rows, clamped at the image's edges
+                const int gy = by * kFinTile - ext + r;
+                if (gy < 0 || gy >= h) continue;
+                const float* row = col + 3 * ((gy - y0) * side - x0);
+                float s0 = 0, s1 = 0, s2 = 0;
+                for (int i = -ext; i <= ext; ++i) {
+                    int xx = tx + i;
+                    xx = xx < 0 ? 0 : (xx >= w ? w - 1 : xx);
+                    const float kq = taps.k[i + ext];
+                    s0 += row[3 * xx + 0] * kq;
+                    s1 += row[3 * xx + 1] * kq;
+                    s2 += row[3 * xx + 2] * kq;
+                }
+                float* o = tmp + 3 * (r * kFinTile + lane);
+                o[0] = s0; o[1] = s1; o[2] = s2;
+            }
+        __syncthreads();
+        if (tx < w)
+            for (int r = warp; r < kFinTile; r += kWarps) {   // columns
+                const int gy = by * kFinTile + r;
+                if (gy >= h) break;
+                float s0 = 0, s1 = 0, s2 = 0;
+                for (int i = -ext; i <= ext; ++i) {
+                    int yy = gy + i;
+                    yy = yy < 0 ? 0 : (yy >= h ? h - 1 : yy);
+                    const float kq = taps.k[i + ext];
+                    const float* q = tmp + 3 * ((yy - (by * kFinTile - ext)) * kFinTile + lane);
+                    s0 += q[0] * kq;
+                    s1 += q[1] * kq;
+                    s2 += q[2] * kq;
+                }
+                float* o = col + 3 * (r * kFinTile + lane);   // the colours are no longer needed
+                o[0] = s0; o[1] = s1; o[2] = s2;
+            }
+        __syncwarp();   // a warp writes out the rows it summed
+    } else {
+        res = col + 3 * (6 * side + 6);
+        res_stride = 3 * side;
+    }
+    const int cols = 3 * min(kFinTile, w - bx * kFinTile);
+    for (int r = warp; r < kFinTile; r += kWarps) {
+        const int gy = by * kFinTile + r;
+        if (gy >= h) break;
+        float* o = out + 3 * ((size_t) gy * w + (size_t) bx * kFinTile);
+        for (int c = lane; c < cols; c += 32) o[c] = res[r * res_stride + c];
+    }
+}
+
+#endif  // __CUDACC__
+
+}  // namespace lg
