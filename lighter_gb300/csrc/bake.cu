@@ -2435,9 +2435,8 @@ void run_bake(ltr_Scene* S)
     } join_reftree{reftree_thread};
 
     // ---- BVH: built on its own stream and host thread as soon as the triangle
-    // soup exists, while this thread prepares the raster records (the build
-    // reads its cluster count back now and then, which would hold this thread);
-    // the sample stage waits for it.
+    // soup exists, while this thread prepares the raster records; the sample
+    // stage waits for it.
     cudaEvent_t e_dev0 = clock.mark();   // the bake's first device work
     float* d_tri_xyz = A.upload(tri_xyz);
     u32* d_tri_meta = A.upload(tri_meta);
@@ -3376,7 +3375,9 @@ void run_bake(ltr_Scene* S)
 
     // ---- readback
     u32 err_words[8] = {0};
+    int bvh_status = 0;
     Counters cnt;
+    if (bvh.status) { CK(cudaMemcpyAsync(&bvh_status, bvh.status, sizeof(int), cudaMemcpyDeviceToHost, st)); note_d2h(sizeof(int)); }
     CK(cudaMemcpyAsync(err_words, d_err, sizeof(err_words), cudaMemcpyDeviceToHost, st)); note_d2h(sizeof(err_words));
     CK(cudaMemcpyAsync(&cnt, d_cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st)); note_d2h(sizeof(Counters));
     // Outputs land directly in the scene's page-locked buffer (kept across
@@ -3423,6 +3424,7 @@ void run_bake(ltr_Scene* S)
     // the host queues the whole bake and waits here; an ltr_Abort during that
     // wait stopped the trace kernels early, so their outputs are incomplete
     check_abort(S);
+    bvh_check_status(bvh_status);
     static const char* kStageName[4] = {"sample fixup", "direct light", "radiosity", "ambient occlusion"};
     for (int k = 0; k < 4; ++k) {
         if (!err_words[k]) continue;

@@ -12,6 +12,10 @@
 //      computes its box (atomic arrival counters);
 //   5. packing into 64-byte nodes that hold both child boxes, and
 //      triangles reordered into leaf order.
+// Pass 3 and 4 serve the radix builder, and a clustering tree too deep for the
+// walks; the default hierarchy is locally-ordered clustering (below). Everything
+// is queued on one stream without a host wait: what depends on a result (the
+// fallback to the radix hierarchy, a failed clustering) is decided on the device.
 // Leaves are triangle references: an oversized triangle may be split (on the
 // host, bake.cu) into several references with clipped boxes, each holding the
 // whole triangle, so every query still tests the original triangle.
@@ -19,6 +23,7 @@
 #include <cub/cub.cuh>
 #include <cfloat>
 
+#include <algorithm>
 #include <cstring>
 #include <stdexcept>
 #include <string>
@@ -65,8 +70,23 @@ __device__ __forceinline__ int prefix(const u32* codes, int n, int i, int j)
     return __clz(a ^ b);
 }
 
-__global__ void k_hierarchy(const u32* codes, int n, int* left, int* right, int* parent_int, int* parent_leaf)
+// The walks keep a stack of kStack entries (the 4-wide walk up to 3 per 4-wide
+// level): a clustering tree deeper than this is replaced by the radix hierarchy,
+// whose depth is bounded by the code and index bits.
+constexpr int kPlocMaxDepth = 40;
+
+// status[0]: 1 when the clustering failed; status[1]: depth of the deepest
+// internal node of its tree. `status` null: the radix hierarchy is the builder.
+__device__ __forceinline__ bool radix_wanted(const int* status)
 {
+    return !status || (status[0] == 0 && status[1] + 1 > kPlocMaxDepth);   // + 1: the leaves below that node
+}
+
+__global__ void k_hierarchy(const int* __restrict__ status, const u32* codes, int n, int* left, int* right,
+                            int* parent_int, int* parent_leaf)
+{
+    if (!radix_wanted(status)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) parent_int[0] = -1;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
     int d = (prefix(codes, n, i, i + 1) - prefix(codes, n, i, i - 1)) >= 0 ? 1 : -1;
@@ -109,9 +129,10 @@ __device__ __forceinline__ void read_box(const float* boxes, int k, float* b)
     for (int c = 0; c < 6; ++c) b[c] = __ldcg(boxes + 6 * (size_t) k + c);
 }
 
-__global__ void k_refit(const float* ref_box, const u32* ids, int n, const int* parent_leaf, const int* parent_int,
+__global__ void k_refit(const int* __restrict__ status, const float* ref_box, const u32* ids, int n, const int* parent_leaf, const int* parent_int,
                         const int* left, const int* right, float* leaf_box, float* int_box, u32* arrivals)
 {
+    if (!radix_wanted(status)) return;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float b[6];
@@ -135,11 +156,23 @@ __global__ void k_refit(const float* ref_box, const u32* ids, int n, const int* 
     }
 }
 
-__global__ void k_pack_nodes(int n_int, const int* left, const int* right, const float* leaf_box, const float* int_box,
-                             float4* nodes)
+// Nodes of the radix hierarchy; or, after a failed clustering, nodes whose boxes
+// no query enters, so that the kernels queued behind the build end at the root
+// (the failure itself reaches the host with their results).
+__global__ void k_pack_nodes(const int* __restrict__ status, int n_int, const int* left, const int* right,
+                             const float* leaf_box, const float* int_box, float4* nodes)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_int) return;
+    if (status && status[0] != 0) {
+        float4* o = nodes + 4 * (size_t) i;
+        o[0] = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX);
+        o[1] = make_float4(-FLT_MAX, -FLT_MAX, FLT_MAX, FLT_MAX);
+        o[2] = make_float4(FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX);
+        o[3] = make_float4(__int_as_float(~0), __int_as_float(~0), 0.0f, 0.0f);
+        return;
+    }
+    if (!radix_wanted(status)) return;
     int l = left[i], r = right[i];
     const float* L = l < 0 ? leaf_box + 6 * (size_t) (~l) : int_box + 6 * (size_t) l;
     const float* R = r < 0 ? leaf_box + 6 * (size_t) (~r) : int_box + 6 * (size_t) r;
@@ -174,27 +207,27 @@ __device__ __forceinline__ void put_slot(float4* o, int k, const float* box, int
     reinterpret_cast<int*>(&o[6])[k] = child;
 }
 
-// Node layout in bvh.cuh (8 float4). Child boxes are the binary tree's, which
-// are already inflated; a grandchild that is internal is referenced by its
-// 4-wide index (it lies at even depth too), a leaf by ~leaf.
-__global__ void k_pack4(int n_int, const int* __restrict__ flag, const int* __restrict__ idx4, const int* __restrict__ left,
-                        const int* __restrict__ right, const float* __restrict__ leaf_box, const float* __restrict__ int_box,
-                        float4* __restrict__ nodes4)
+// Node layout in bvh.cuh (8 float4), from the binary nodes. Child boxes are the
+// binary tree's, which are already inflated; a grandchild that is internal is
+// referenced by its 4-wide index (it lies at even depth too), a leaf by ~leaf.
+__global__ void k_pack4(int n_int, const int* __restrict__ flag, const int* __restrict__ idx4,
+                        const float4* __restrict__ nodes, float4* __restrict__ nodes4)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_int || !flag[i]) return;
     float4* o = nodes4 + 8 * (size_t) idx4[i];
     const float empty_box[6] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
     int k = 0;
-    const int kids[2] = {left[i], right[i]};
-    for (int c : kids) {
+    const float* f = reinterpret_cast<const float*>(nodes + 4 * (size_t) i);
+    for (int s = 0; s < 2; ++s) {
+        const int c = __float_as_int(f[12 + s]);
         if (c < 0) {
-            put_slot(o, k++, leaf_box + 6 * (size_t) (~c), c);
+            put_slot(o, k++, f + 6 * s, c);
         } else {
-            const int gk[2] = {left[c], right[c]};
-            for (int g : gk) {
-                const float* box = g < 0 ? leaf_box + 6 * (size_t) (~g) : int_box + 6 * (size_t) g;
-                put_slot(o, k++, box, g < 0 ? g : idx4[g]);
+            const float* g = reinterpret_cast<const float*>(nodes + 4 * (size_t) c);
+            for (int q = 0; q < 2; ++q) {
+                const int gc = __float_as_int(g[12 + q]);
+                put_slot(o, k++, g + 6 * q, gc < 0 ? gc : idx4[gc]);
             }
         }
     }
@@ -202,28 +235,23 @@ __global__ void k_pack4(int n_int, const int* __restrict__ flag, const int* __re
     o[7] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
-__global__ void k_pack_tris(int n, const u32* ids, const u32* ref_tri, const float* xyz, const u32* meta, const u32* local,
-                            float4* tris)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    u32 s = ref_tri[ids[i]];
-    const float* p = xyz + 9 * (size_t) s;
-    tris[3 * (size_t) i + 0] = make_float4(p[0], p[1], p[2], __uint_as_float(meta[s]));
-    tris[3 * (size_t) i + 1] = make_float4(p[3], p[4], p[5], __uint_as_float(local[s]));
-    tris[3 * (size_t) i + 2] = make_float4(p[6], p[7], p[8], __uint_as_float(s));
-}
-
 // Triangle-only terms of the two exact tests per leaf (layout in bvh.cuh),
 // computed with the expressions of seg_tri / point_tri_dist in common.cuh.
-__global__ void k_pack_records(int nleaf, const float4* __restrict__ tris, float4* __restrict__ srec,
-                               float4* __restrict__ drec)
+// And the triangles themselves, in leaf order.
+__global__ void k_pack_leaves(int nleaf, const u32* __restrict__ ids, const u32* __restrict__ ref_tri,
+                              const float* __restrict__ xyz, const u32* __restrict__ metas,
+                              const u32* __restrict__ local, float4* __restrict__ tris, float4* __restrict__ srec,
+                              float4* __restrict__ drec)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nleaf) return;
-    float4 a = tris[3 * (size_t) i], b = tris[3 * (size_t) i + 1], c = tris[3 * (size_t) i + 2];
-    V3 t0 = mk(a.x, a.y, a.z), t1 = mk(b.x, b.y, b.z), t2 = mk(c.x, c.y, c.z);
-    float meta = a.w;
+    const u32 src = ref_tri[ids[i]];
+    const float* p = xyz + 9 * (size_t) src;
+    V3 t0 = mk(p[0], p[1], p[2]), t1 = mk(p[3], p[4], p[5]), t2 = mk(p[6], p[7], p[8]);
+    const float meta = __uint_as_float(metas[src]);
+    tris[3 * (size_t) i + 0] = make_float4(t0.x, t0.y, t0.z, meta);
+    tris[3 * (size_t) i + 1] = make_float4(t1.x, t1.y, t1.z, __uint_as_float(local[src]));
+    tris[3 * (size_t) i + 2] = make_float4(t2.x, t2.y, t2.z, __uint_as_float(src));
     V3 u = t1 - t0, v = t2 - t0;
     V3 n = cross(u, v);
     float4* s = srec + 4 * (size_t) i;
@@ -259,8 +287,18 @@ __global__ void k_pack_records(int nleaf, const float4* __restrict__ tris, float
 // (every iteration merges), and a run of equal boxes pairs up (0,1), (2,3), ...
 // and halves each iteration instead of growing a chain.
 
+//
+// All iterations run in one launch: a cluster of kPlocCtas blocks, each owning a
+// contiguous run of the list, with two cluster barriers per iteration (merge
+// counts, then the compacted list), and one block alone in shared memory once the
+// list fits its threads. Bound by latency and by the neighbour search of the
+// first iterations. Launched kernel by kernel (as graphs of eight iterations and a
+// read-back of the count) the build of 44,652 references took 2.5 ms, of six 0.6 ms.
+
 constexpr int kPlocR = 16;
-constexpr int kPlocB = 256;
+constexpr int kPlocT = 1024;     // threads per block, clusters per tile
+constexpr int kPlocCtas = 8;     // blocks of the cluster
+constexpr int kPlocHalo = 2 * kPlocR;
 
 __device__ __forceinline__ float merged_area(const float* a, const float* b)
 {
@@ -270,135 +308,264 @@ __device__ __forceinline__ float merged_area(const float* a, const float* b)
     return ex * ey + ey * ez + ez * ex;
 }
 
-__global__ void k_leaf_boxes(const float* ref_box, const u32* ids, int n, float* leaf_box, int* cl, float* cbox)
+struct PlocArgs {
+    int n;
+    const float* ref_box;
+    const u32* ids;               // references in Morton order
+    float4* cl[2];                // clusters, 2 per entry: (mn.xyz, mx.x) (mx.yz, node or ~leaf, height)
+    u32* flags;                   // per cluster: partner << 2 | merges (lower half of its pair) << 1 | keeps its place
+    unsigned long long* totals;   // [parity][block]: merges << 32 | kept
+    float4* nodes;                // bvh.cuh's binary nodes
+    int* parent;                  // per internal node (may be null)
+    int* status;                  // see radix_wanted
+};
+
+// A cluster's boxes in shared memory: 16 + 8 bytes, read as two vectors.
+struct PlocBoxes {
+    float4 a[kPlocT + 2 * kPlocHalo];   // mn.xyz, mx.x
+    float2 b[kPlocT + 2 * kPlocHalo];   // mx.yz
+};
+
+__device__ __forceinline__ void ploc_box(const PlocBoxes& s, int k, float* o)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float b[6];
-    leaf_box_of(ref_box + 6 * (size_t) ids[i], b);
-    for (int c = 0; c < 6; ++c) {
-        leaf_box[6 * (size_t) i + c] = b[c];
-        cbox[6 * (size_t) i + c] = b[c];
-    }
-    cl[i] = ~i;
+    const float4 p = s.a[k];
+    const float2 q = s.b[k];
+    o[0] = p.x; o[1] = p.y; o[2] = p.z; o[3] = p.w; o[4] = q.x; o[5] = q.y;
 }
 
-// The cluster count and the next node number live on the device (state[0],
-// state[1]): the host launches every iteration's kernels for the count it last
-// read (an upper bound), and threads past the current count do nothing.
-__global__ void __launch_bounds__(kPlocB) k_ploc_nn(const int* __restrict__ state, const float* __restrict__ cbox,
-                                                    int* __restrict__ nn)
+// The nearest neighbour of cluster i (at slot k of the boxes) as a key that orders
+// its pairs: cost, then list distance, parity of the lower position, the lower
+// position (26 bits; bvh_build keeps longer lists away). ~0: none.
+__device__ __forceinline__ unsigned long long ploc_nearest(const PlocBoxes& s, int k, int i, int count)
 {
-    __shared__ float sb[(kPlocB + 2 * kPlocR) * 6];
-    const int count = state[0];
-    const int start = blockIdx.x * kPlocB;
-    if (start >= count) return;
-    for (int k = threadIdx.x; k < (kPlocB + 2 * kPlocR) * 6; k += blockDim.x) {
-        const long g = (long) start * 6 - kPlocR * 6 + k;
-        sb[k] = (g >= 0 && g < (long) count * 6) ? cbox[g] : 0.0f;
-    }
-    __syncthreads();
-    const int i = start + threadIdx.x;
-    if (i >= count) return;
-    const float* me = sb + 6 * (threadIdx.x + kPlocR);
-    float best = FLT_MAX;
-    int bj = -1, bd = 1 << 30, bpar = 2, bmin = 1 << 30;
+    float me[6];
+    ploc_box(s, k, me);
+    unsigned long long best = ~0ull;
     for (int d = -kPlocR; d <= kPlocR; ++d) {
         const int j = i + d;
         if (d == 0 || j < 0 || j >= count) continue;
-        const float c = merged_area(me, sb + 6 * (threadIdx.x + kPlocR + d));
-        const int ad = d < 0 ? -d : d, mn = min(i, j), par = mn & 1;
-        if (c < best || (c == best && (ad < bd || (ad == bd && (par < bpar || (par == bpar && mn < bmin)))))) {
-            best = c; bj = j; bd = ad; bpar = par; bmin = mn;
-        }
+        float o[6];
+        ploc_box(s, k + d, o);
+        const float c = merged_area(me, o);
+        if (!(c <= FLT_MAX)) continue;
+        const u32 mn = (u32) min(i, j);
+        const u32 tie = ((u32) (d < 0 ? -d : d) << 27) | ((mn & 1u) << 26) | mn;
+        const unsigned long long key = ((unsigned long long) __float_as_uint(c) << 32) | tie;
+        best = key < best ? key : best;
     }
-    nn[i] = bj;
+    return best;
 }
 
-// flags[i]: merge (high word: i < nn[i] and mutual), keep (low word: not the
-// upper half of a mutual pair); zero from the current count up to the bound
-// `ub` the scan runs over. A single cluster keeps itself (an iteration after
-// the root is done changes nothing).
-__global__ void k_ploc_flags(const int* __restrict__ state, int ub, const int* __restrict__ nn,
-                             unsigned long long* __restrict__ flags)
+__device__ __forceinline__ int ploc_partner(unsigned long long key, int i)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > ub) return;
-    const int count = state[0];
-    if (i >= count) { flags[i] = 0ull; return; }
-    if (count == 1) { flags[i] = 1ull; return; }
-    const int j = nn[i];
-    const bool mutual = j >= 0 && nn[j] == i;
-    const unsigned long long merge = (mutual && i < j) ? 1ull : 0ull;
-    const unsigned long long keep = (mutual && i > j) ? 0ull : 1ull;
-    flags[i] = (merge << 32) | keep;
+    if (key == ~0ull) return -1;
+    const int d = (int) ((u32) key >> 27), mn = (int) (key & 0x3ffffffull);
+    return mn == i ? i + d : mn;
 }
 
-__global__ void k_ploc_merge(const int* __restrict__ state, const int* __restrict__ nn, const unsigned long long* __restrict__ flags,
-                             const unsigned long long* __restrict__ scan, const int* __restrict__ cl,
-                             const float* __restrict__ cbox, int* __restrict__ ncl, float* __restrict__ ncbox,
-                             int* __restrict__ left, int* __restrict__ right, int* __restrict__ parent_int,
-                             float* __restrict__ int_box)
+// Exclusive ranks of two flags over the block's threads, and their totals (kept
+// in the low, merged in the high half word).
+__device__ __forceinline__ u32 ploc_scan(bool keep, bool merge, u32* wsum, u32& total)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int count = state[0], base = state[1];
-    if (i >= count) return;
-    const unsigned long long f = flags[i];
-    if (!(f & 0xffffffffull)) return;   // merged into its lower partner
-    const int pos = (int) (scan[i] & 0xffffffffull);
-    const float* a = cbox + 6 * (size_t) i;
-    if (f >> 32) {
-        const int j = nn[i];
-        const int id = base - 1 - (int) (scan[i] >> 32);
-        const float* b = cbox + 6 * (size_t) j;
-        const int ca = cl[i], cb = cl[j];
-        left[id] = ca;
-        right[id] = cb;
-        if (ca >= 0) parent_int[ca] = id;
-        if (cb >= 0) parent_int[cb] = id;
-        float u[6];
-        for (int c = 0; c < 3; ++c) {
-            u[c] = fminf(a[c], b[c]);
-            u[3 + c] = fmaxf(a[3 + c], b[3 + c]);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const u32 bk = __ballot_sync(0xffffffffu, keep), bm = __ballot_sync(0xffffffffu, merge);
+    const u32 below = (1u << lane) - 1u;
+    if (lane == 0) wsum[w] = (u32) __popc(bk) | ((u32) __popc(bm) << 16);
+    __syncthreads();
+    u32 v = wsum[lane];   // 32 warps
+    static_assert(kPlocT == 1024, "one warp total per lane");
+    u32 inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u32 t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    total = __shfl_sync(0xffffffffu, inc, 31);
+    const u32 before = __shfl_sync(0xffffffffu, inc - v, w);
+    __syncthreads();   // wsum may be written again
+    return before + ((u32) __popc(bk & below) | ((u32) __popc(bm & below) << 16));
+}
+
+// Clusters a (lower) and b become internal node `id`; returns the merged cluster.
+__device__ __forceinline__ void ploc_merge(const PlocArgs& p, int id, float4 a0, float4 a1, float4 b0, float4 b1,
+                                           float4& o0, float4& o1)
+{
+    const int ca = __float_as_int(a1.z), cb = __float_as_int(b1.z);
+    float4* nd = p.nodes + 4 * (size_t) id;
+    nd[0] = a0;
+    nd[1] = make_float4(a1.x, a1.y, b0.x, b0.y);
+    nd[2] = make_float4(b0.z, b0.w, b1.x, b1.y);
+    nd[3] = make_float4(a1.z, b1.z, 0.0f, 0.0f);
+    if (p.parent) {
+        if (ca >= 0) p.parent[ca] = id;
+        if (cb >= 0) p.parent[cb] = id;
+    }
+    o0 = make_float4(fminf(a0.x, b0.x), fminf(a0.y, b0.y), fminf(a0.z, b0.z), fmaxf(a0.w, b0.w));
+    o1 = make_float4(fmaxf(a1.x, b1.x), fmaxf(a1.y, b1.y), __int_as_float(id),
+                     __int_as_float(max(__float_as_int(a1.w), __float_as_int(b1.w)) + 1));
+}
+
+__device__ __forceinline__ void ploc_cluster_sync()
+{
+    __threadfence();
+    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+}
+
+__global__ void __cluster_dims__(kPlocCtas, 1, 1) __launch_bounds__(kPlocT) k_ploc(PlocArgs p)
+{
+    __shared__ PlocBoxes box;
+    __shared__ unsigned long long key[kPlocT + 2 * kPlocR];
+    __shared__ int2 ref[kPlocT];   // the tail's (node or ~leaf, height)
+    __shared__ u32 wsum[32];
+    const int tid = threadIdx.x, rank = blockIdx.x;
+    for (int i = rank * kPlocT + tid; i < p.n; i += kPlocCtas * kPlocT) {
+        float b[6];
+        leaf_box_of(p.ref_box + 6 * (size_t) p.ids[i], b);
+        p.cl[0][2 * (size_t) i] = make_float4(b[0], b[1], b[2], b[3]);
+        p.cl[0][2 * (size_t) i + 1] = make_float4(b[4], b[5], __int_as_float(~i), __int_as_float(-1));
+    }
+    ploc_cluster_sync();
+    int count = p.n, base = p.n - 1, cur = 0;
+    bool ok = true;
+    for (int par = 0; ok && count > kPlocT; par ^= 1) {
+        const float4* src = p.cl[cur];
+        float4* dst = p.cl[cur ^ 1];
+        const int tiles = (count + kPlocT - 1) / kPlocT, per = (tiles + kPlocCtas - 1) / kPlocCtas;
+        const int t0 = min(tiles, rank * per), t1 = min(tiles, t0 + per);
+        u32 kept = 0, merged = 0;
+        for (int t = t0; t < t1; ++t) {
+            const int start = t * kPlocT;
+            for (int k = tid; k < kPlocT + 2 * kPlocHalo; k += kPlocT) {
+                const int g = start - kPlocHalo + k;
+                if (g >= 0 && g < count) {
+                    const float4 a = __ldcg(src + 2 * (size_t) g), b = __ldcg(src + 2 * (size_t) g + 1);
+                    box.a[k] = a;
+                    box.b[k] = make_float2(b.x, b.y);
+                }
+            }
+            __syncthreads();
+            // neighbours of the tile's clusters and of kPlocR more on either side
+            for (int k = tid; k < kPlocT + 2 * kPlocR; k += kPlocT) {
+                const int i = start - kPlocR + k;
+                if (i >= 0 && i < count) key[k] = ploc_nearest(box, k + kPlocR, i, count);
+            }
+            __syncthreads();
+            const int i = start + tid;
+            bool keep = false, merge = false;
+            if (i < count) {
+                const int j = ploc_partner(key[tid + kPlocR], i);
+                const bool mutual = j >= 0 && ploc_partner(key[j - start + kPlocR], j) == i;
+                merge = mutual && i < j;
+                keep = !(mutual && i > j);
+                p.flags[i] = ((u32) j << 2) | (merge ? 2u : 0u) | (keep ? 1u : 0u);
+            }
+            kept += (u32) __syncthreads_count(keep);
+            merged += (u32) __syncthreads_count(merge);
         }
-        for (int c = 0; c < 6; ++c) {
-            int_box[6 * (size_t) id + c] = u[c];
-            ncbox[6 * (size_t) pos + c] = u[c];
+        if (tid == 0) p.totals[par * kPlocCtas + rank] = ((unsigned long long) merged << 32) | kept;
+        ploc_cluster_sync();
+        unsigned long long before = 0, total = 0;
+        for (int r = 0; r < kPlocCtas; ++r) {
+            const unsigned long long v = __ldcg(p.totals + par * kPlocCtas + r);
+            if (r < rank) before += v;
+            total += v;
         }
-        ncl[pos] = id;
-    } else {
-        for (int c = 0; c < 6; ++c) ncbox[6 * (size_t) pos + c] = a[c];
-        ncl[pos] = cl[i];
+        u32 pos = (u32) before, mrk = (u32) (before >> 32);
+        for (int t = t0; t < t1; ++t) {
+            const int i = t * kPlocT + tid;
+            const u32 f = i < count ? p.flags[i] : 0u;
+            u32 tot;
+            const u32 ex = ploc_scan((f & 1u) != 0, (f & 2u) != 0, wsum, tot);
+            if (f & 1u) {
+                float4 o0 = __ldcg(src + 2 * (size_t) i), o1 = __ldcg(src + 2 * (size_t) i + 1);
+                if (f & 2u) {
+                    const size_t j = f >> 2;
+                    ploc_merge(p, base - 1 - (int) (mrk + (ex >> 16)), o0, o1, __ldcg(src + 2 * j), __ldcg(src + 2 * j + 1),
+                               o0, o1);
+                }
+                float4* o = dst + 2 * (size_t) (pos + (ex & 0xffffu));
+                o[0] = o0;
+                o[1] = o1;
+            }
+            pos += tot & 0xffffu;
+            mrk += tot >> 16;
+        }
+        ploc_cluster_sync();
+        ok = (total >> 32) != 0;   // the least pair is always mutual: only unordered costs merge nothing
+        count = (int) (total & 0xffffffffull);
+        base -= (int) (total >> 32);
+        cur ^= 1;
+    }
+    if (rank != 0) return;
+    // the list fits this block's threads: one cluster per thread, in shared memory
+    float4 c0 = make_float4(0, 0, 0, 0), c1 = c0;
+    if (ok && tid < count) {
+        c0 = __ldcg(p.cl[cur] + 2 * (size_t) tid);
+        c1 = __ldcg(p.cl[cur] + 2 * (size_t) tid + 1);
+    }
+    while (ok && count > 1) {
+        if (tid < count) {
+            box.a[tid] = c0;
+            box.b[tid] = make_float2(c1.x, c1.y);
+            ref[tid] = make_int2(__float_as_int(c1.z), __float_as_int(c1.w));
+        }
+        __syncthreads();
+        if (tid < count) key[tid] = ploc_nearest(box, tid, tid, count);
+        __syncthreads();
+        bool keep = false, merge = false;
+        int j = -1;
+        if (tid < count) {
+            j = ploc_partner(key[tid], tid);
+            const bool mutual = j >= 0 && ploc_partner(key[j], j) == tid;
+            merge = mutual && tid < j;
+            keep = !(mutual && tid > j);
+        }
+        u32 tot;
+        const u32 ex = ploc_scan(keep, merge, wsum, tot);
+        if (merge) {
+            const float4 b0 = box.a[j];
+            const float2 q = box.b[j];
+            const int2 r = ref[j];
+            ploc_merge(p, base - 1 - (int) (ex >> 16), c0, c1, b0,
+                       make_float4(q.x, q.y, __int_as_float(r.x), __int_as_float(r.y)), c0, c1);
+        }
+        __syncthreads();   // partners read
+        if (keep) {
+            const u32 o = ex & 0xffffu;
+            box.a[o] = c0;
+            box.b[o] = make_float2(c1.x, c1.y);
+            ref[o] = make_int2(__float_as_int(c1.z), __float_as_int(c1.w));
+        }
+        __syncthreads();
+        ok = (tot >> 16) != 0;
+        count = (int) (tot & 0xffffu);
+        base -= (int) (tot >> 16);
+        if (tid < count) {
+            c0 = box.a[tid];
+            const float2 q = box.b[tid];
+            const int2 r = ref[tid];
+            c1 = make_float4(q.x, q.y, __int_as_float(r.x), __int_as_float(r.y));
+        }
+        __syncthreads();   // everyone holds its cluster before the boxes are written again
+    }
+    if (tid == 0) {
+        p.status[0] = ok && count == 1 && base == 0 ? 0 : 1;
+        p.status[1] = __float_as_int(c1.w);
     }
 }
 
-// state = (kept, base - merged) from the scan total at scan[ub]
-__global__ void k_ploc_state(int* __restrict__ state, const unsigned long long* __restrict__ scan, int ub)
-{
-    const unsigned long long tot = scan[ub];
-    state[1] -= (int) (tot >> 32);
-    state[0] = (int) (tot & 0xffffffffull);
-}
-
-// depth (edges from the root) of the deepest internal node
-__global__ void k_max_depth(int n_int, const int* __restrict__ parent_int, int* __restrict__ maxd)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_int) return;
-    int d = 0;
-    for (int p = parent_int[i]; p >= 0 && d < 4096; p = parent_int[p]) ++d;
-    atomicMax(maxd, d);
-}
-
-template <class T>
-T* alloc(size_t count, cudaStream_t st, size_t& bytes)
-{
-    void* p = nullptr;
-    if (count == 0) count = 1;
-    BVH_CHECK(cudaMallocAsync(&p, count * sizeof(T), st));
-    bytes += count * sizeof(T);
-    return (T*) p;
-}
+// Parts of one device allocation, 256-byte aligned: a first pass adds up the
+// sizes, a second one hands out the addresses.
+struct Carve {
+    char* base = nullptr;
+    size_t at = 0;
+    template <class T> T* take(size_t count)
+    {
+        T* p = base ? reinterpret_cast<T*>(base + at) : nullptr;
+        at += (count * sizeof(T) + 255) / 256 * 256;
+        return p;
+    }
+};
 
 }  // namespace
 
@@ -409,21 +576,66 @@ void bvh_build(const BvhBuildInput& in, BvhStorage& out, void* stream)
     out.n_tris = n;
     out.bytes = 0;
     if (n <= 0) { out.root = 0; return; }
-    const int n_int = n > 1 ? n - 1 : 0;
-    out.root = n > 1 ? 0 : ~0;
+    const int n_int = n - 1;
+    out.root = n_int > 0 ? 0 : ~0;
+    out.root4 = out.root;   // the root is binary node 0 (both builders), at depth 0: 4-wide node 0
+    // list positions take 26 bits of the clustering's keys
+    const bool ploc = in.builder != 1 && n_int > 0 && n < (1 << 26);
+    const bool wide = n >= kWideTreeMin;
 
-    size_t scratch_bytes = 0;
-    u32* codes = alloc<u32>(n, st, scratch_bytes);
-    u32* codes2 = alloc<u32>(n, st, scratch_bytes);
-    u32* ids = alloc<u32>(n, st, scratch_bytes);
-    u32* ids2 = alloc<u32>(n, st, scratch_bytes);
-    int* left = alloc<int>(n_int, st, scratch_bytes);
-    int* right = alloc<int>(n_int, st, scratch_bytes);
-    int* parent_int = alloc<int>(n_int, st, scratch_bytes);
-    int* parent_leaf = alloc<int>(n, st, scratch_bytes);
-    float* leaf_box = alloc<float>(6 * (size_t) n, st, scratch_bytes);
-    float* int_box = alloc<float>(6 * (size_t) n_int, st, scratch_bytes);
-    u32* arrivals = alloc<u32>(n_int, st, scratch_bytes);
+    size_t sort_bytes = 0, scan_bytes = 0;
+    BVH_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (u32*) nullptr, (u32*) nullptr, (u32*) nullptr,
+                                              (u32*) nullptr, n, 0, 30, st));
+    if (wide)
+        BVH_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (int*) nullptr, (int*) nullptr, n_int + 1, st));
+
+    // what the walks read, in one allocation
+    auto layout = [&](Carve& c) {
+        out.status = c.take<int>(2);
+        out.nodes = c.take<float4>(4 * (size_t) std::max(n_int, 1));
+        out.tris = c.take<float4>(3 * (size_t) n);
+        out.srec = c.take<float4>(4 * (size_t) n);
+        out.drec = c.take<float4>(8 * (size_t) n);
+        out.nodes4 = wide ? c.take<float4>(8 * (size_t) n_int) : nullptr;   // at most one per binary node
+    };
+    Carve size;
+    layout(size);
+    BVH_CHECK(cudaMallocAsync(&out.mem, size.at, st));
+    out.bytes = size.at;
+    Carve fill{(char*) out.mem, 0};
+    layout(fill);
+
+    // build scratch, in another
+    u32 *codes, *codes2, *ids, *ids2, *arrivals, *flags;
+    int *left, *right, *parent_int, *parent_leaf, *flag4, *idx4;
+    float *leaf_box, *int_box;
+    float4* cl[2];
+    unsigned long long* totals;
+    char *sort_tmp, *scan_tmp;
+    auto scratch = [&](Carve& c) {
+        codes = c.take<u32>(n); codes2 = c.take<u32>(n); ids = c.take<u32>(n); ids2 = c.take<u32>(n);
+        left = c.take<int>(n); right = c.take<int>(n); parent_int = c.take<int>(n); parent_leaf = c.take<int>(n);
+        leaf_box = c.take<float>(6 * (size_t) n);
+        int_box = c.take<float>(6 * (size_t) n);
+        arrivals = c.take<u32>(n);
+        sort_tmp = c.take<char>(sort_bytes);
+        for (float4*& p : cl) p = c.take<float4>(ploc ? 2 * (size_t) n : 0);
+        flags = c.take<u32>(ploc ? n : 0);
+        totals = c.take<unsigned long long>(2 * kPlocCtas);
+        flag4 = c.take<int>(wide ? n : 0);
+        idx4 = c.take<int>(wide ? n : 0);
+        scan_tmp = c.take<char>(scan_bytes);
+    };
+    Carve ssize;
+    scratch(ssize);
+    void* smem = nullptr;
+    BVH_CHECK(cudaMallocAsync(&smem, ssize.at, st));
+    struct FreeScratch {
+        void* p; cudaStream_t s;
+        ~FreeScratch() { cudaFreeAsync(p, s); }
+    } free_scratch{smem, st};
+    Carve sfill{(char*) smem, 0};
+    scratch(sfill);
 
     const int B = 256;
     float3 mn = make_float3(in.scene_min[0], in.scene_min[1], in.scene_min[2]);
@@ -431,159 +643,48 @@ void bvh_build(const BvhBuildInput& in, BvhStorage& out, void* stream)
     float3 inv_ext = make_float3(ex > 0 ? 1.0f / ex : 0.0f, ey > 0 ? 1.0f / ey : 0.0f, ez > 0 ? 1.0f / ez : 0.0f);
     k_morton<<<(n + B - 1) / B, B, 0, st>>>(in.ref_box, n, mn, inv_ext, codes, ids); note_launch();
     BVH_CHECK(cudaGetLastError());
-
-    size_t temp_bytes = 0;
-    BVH_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, codes, codes2, ids, ids2, n, 0, 30, st));
-    void* temp = alloc<char>(temp_bytes, st, scratch_bytes);
-    BVH_CHECK(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, codes, codes2, ids, ids2, n, 0, 30, st));
-
-    // The walks keep a stack of kStack entries (the 4-wide walk up to 3 per
-    // 4-wide level): a PLOC tree deeper than kPlocMaxDepth is replaced by the
-    // radix hierarchy, whose depth is bounded by the code and index bits.
-    constexpr int kPlocMaxDepth = 40;
-    bool use_radix = in.builder == 1 || n_int == 0;
-    if (!use_radix) {
-        size_t pb = 0;
-        int* cl = alloc<int>(n, st, pb);
-        int* ncl = alloc<int>(n, st, pb);
-        float* cbox = alloc<float>(6 * (size_t) n, st, pb);
-        float* ncbox = alloc<float>(6 * (size_t) n, st, pb);
-        int* nn = alloc<int>(n, st, pb);
-        unsigned long long* flags = alloc<unsigned long long>(n + 1, st, pb);
-        unsigned long long* scan = alloc<unsigned long long>(n + 1, st, pb);
-        int* maxd = alloc<int>(1, st, pb);
-        unsigned long long h_tot = 0;   // scan total: merges << 32 | kept
-        size_t tb = 0;
-        BVH_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, tb, flags, scan, n + 1, st));
-        void* ptmp = alloc<char>(tb, st, pb);
-        BVH_CHECK(cudaMemsetAsync(parent_int, 0xff, sizeof(int) * n_int, st));
-        k_leaf_boxes<<<(n + B - 1) / B, B, 0, st>>>(in.ref_box, ids2, n, leaf_box, cl, cbox); note_launch();
-        BVH_CHECK(cudaGetLastError());
-        int* state = alloc<int>(2, st, pb);   // device: cluster count, next node number
-        {
-            const int init[2] = {n, n_int};
-            BVH_CHECK(cudaMemcpyAsync(state, init, sizeof(init), cudaMemcpyHostToDevice, st));
-        }
-        int count = n, base = n_int;   // as last read back
-        std::string fail;
-        // Clustering steps run in blocks of kItersPerRead between reads of the
-        // cluster count. A block is launched as one CUDA graph, captured once per
-        // build with launch bounds for all n clusters: the kernels take the live
-        // count from `state` (threads past it exit or write zero flags), so the
-        // same graph serves every block; the even number of steps per block
-        // returns the cluster buffers to their roles at its start. One graph
-        // launch replaces 48 small launches (with the scan's two) and their gaps.
-        constexpr int kItersPerRead = 8;
-        static_assert(kItersPerRead % 2 == 0, "a block must end with the cluster buffers in their starting roles");
-        cudaGraphExec_t block = nullptr;
-        struct BlockGuard {
-            cudaGraphExec_t& g;
-            ~BlockGuard() { if (g) cudaGraphExecDestroy(g); }
-        } block_guard{block};
-        {
-            const int ub = n;
-            BVH_CHECK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            cudaError_t ce = cudaSuccess;
-            for (int k = 0; k < kItersPerRead && ce == cudaSuccess; ++k) {
-                k_ploc_nn<<<(ub + kPlocB - 1) / kPlocB, kPlocB, 0, st>>>(state, cbox, nn);
-                k_ploc_flags<<<(ub + 1 + B - 1) / B, B, 0, st>>>(state, ub, nn, flags);
-                size_t tb2 = tb;
-                if (ce == cudaSuccess) ce = cudaGetLastError();
-                if (ce == cudaSuccess) ce = cub::DeviceScan::ExclusiveSum(ptmp, tb2, flags, scan, ub + 1, st);
-                k_ploc_merge<<<(ub + B - 1) / B, B, 0, st>>>(state, nn, flags, scan, cl, cbox, ncl, ncbox, left, right,
-                                                             parent_int, int_box);
-                k_ploc_state<<<1, 1, 0, st>>>(state, scan, ub);
-                if (ce == cudaSuccess) ce = cudaGetLastError();
-                std::swap(cl, ncl);
-                std::swap(cbox, ncbox);
-            }
-            cudaGraph_t graph = nullptr;
-            const cudaError_t ee = cudaStreamEndCapture(st, &graph);
-            if (ce == cudaSuccess) ce = ee;
-            if (ce == cudaSuccess) ce = cudaGraphInstantiate(&block, graph, 0);
-            if (graph) cudaGraphDestroy(graph);
-            BVH_CHECK(ce);
-        }
-        for (int it = 0; count > 1;) {
-            if (it >= 4 * n + 64) { fail = "bvh: clustering made no progress"; break; }
-            BVH_CHECK(cudaGraphLaunch(block, st));
-            for (int k = 0; k < 4 * kItersPerRead; ++k) note_launch();   // the graph's own kernels
-            it += kItersPerRead;
-            int hs[2] = {0, 0};
-            BVH_CHECK(cudaMemcpyAsync(hs, state, sizeof(hs), cudaMemcpyDeviceToHost, st));
-            note_d2h(sizeof(hs));
-            BVH_CHECK(cudaStreamSynchronize(st));
-            // every merge takes one cluster and one node number, so the next
-            // number is count - 1; with more than one cluster every iteration merges
-            if (hs[0] < 1 || hs[0] >= count || hs[1] != hs[0] - 1) { fail = "bvh: clustering step inconsistent"; break; }
-            count = hs[0];
-            base = hs[1];
-        }
-        if (fail.empty() && base != 0) fail = "bvh: clustering left " + std::to_string(base) + " nodes unnumbered";
-        int depth = 0;
-        if (fail.empty()) {
-            BVH_CHECK(cudaMemsetAsync(maxd, 0, sizeof(int), st));
-            k_max_depth<<<(n_int + B - 1) / B, B, 0, st>>>(n_int, parent_int, maxd); note_launch();
-            BVH_CHECK(cudaGetLastError());
-            BVH_CHECK(cudaMemcpyAsync(&depth, maxd, sizeof(int), cudaMemcpyDeviceToHost, st)); note_d2h(sizeof(int));
-            BVH_CHECK(cudaStreamSynchronize(st));
-        }
-        void* pp[] = {cl, ncl, cbox, ncbox, nn, flags, scan, maxd, ptmp, state};
-        for (void* p : pp) BVH_CHECK(cudaFreeAsync(p, st));
-        if (!fail.empty()) {
-            void* ptrs[] = {codes, codes2, ids, ids2, left, right, parent_int, parent_leaf, leaf_box, int_box, arrivals, temp};
-            for (void* p : ptrs) cudaFreeAsync(p, st);
-            throw std::runtime_error(fail);
-        }
-        use_radix = depth + 1 > kPlocMaxDepth;   // + 1: the leaves below the deepest internal node
-    }
-    if (use_radix) {
-        if (n_int > 0) {
-            BVH_CHECK(cudaMemsetAsync(parent_int, 0xff, sizeof(int) * n_int, st));
-            BVH_CHECK(cudaMemsetAsync(arrivals, 0, sizeof(u32) * n_int, st));
-            k_hierarchy<<<(n_int + B - 1) / B, B, 0, st>>>(codes2, n, left, right, parent_int, parent_leaf); note_launch();
-            BVH_CHECK(cudaGetLastError());
-        }
-        k_refit<<<(n + B - 1) / B, B, 0, st>>>(in.ref_box, ids2, n, parent_leaf, parent_int, left, right, leaf_box, int_box,
-                                                arrivals); note_launch();
+    BVH_CHECK(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, codes, codes2, ids, ids2, n, 0, 30, st));
+    BVH_CHECK(cudaMemsetAsync(out.status, 0, 2 * sizeof(int), st));
+    if (wide) BVH_CHECK(cudaMemsetAsync(parent_int, 0xff, sizeof(int) * n_int, st));
+    if (ploc) {
+        PlocArgs pa;
+        pa.n = n;
+        pa.ref_box = in.ref_box;
+        pa.ids = ids2;
+        pa.cl[0] = cl[0];
+        pa.cl[1] = cl[1];
+        pa.flags = flags;
+        pa.totals = totals;
+        pa.nodes = out.nodes;
+        pa.parent = wide ? parent_int : nullptr;
+        pa.status = out.status;
+        k_ploc<<<kPlocCtas, kPlocT, 0, st>>>(pa); note_launch();
         BVH_CHECK(cudaGetLastError());
     }
-
-    out.nodes = alloc<float4>(4 * (size_t) (n_int > 0 ? n_int : 1), st, out.bytes);
-    out.tris = alloc<float4>(3 * (size_t) n, st, out.bytes);
     if (n_int > 0) {
-        k_pack_nodes<<<(n_int + B - 1) / B, B, 0, st>>>(n_int, left, right, leaf_box, int_box, out.nodes); note_launch();
+        const int* status = ploc ? out.status : nullptr;
+        BVH_CHECK(cudaMemsetAsync(arrivals, 0, sizeof(u32) * n_int, st));
+        k_hierarchy<<<(n_int + B - 1) / B, B, 0, st>>>(status, codes2, n, left, right, parent_int, parent_leaf); note_launch();
+        k_refit<<<(n + B - 1) / B, B, 0, st>>>(status, in.ref_box, ids2, n, parent_leaf, parent_int, left, right, leaf_box,
+                                                int_box, arrivals); note_launch();
+        k_pack_nodes<<<(n_int + B - 1) / B, B, 0, st>>>(status, n_int, left, right, leaf_box, int_box, out.nodes); note_launch();
         BVH_CHECK(cudaGetLastError());
     }
-    // 4-wide nodes (at most one per binary node)
-    out.nodes4 = alloc<float4>(8 * (size_t) (n_int > 0 ? n_int : 1), st, out.bytes);
-    out.root4 = n_int > 0 ? 0 : ~0;   // the root is binary node 0 (both builders), at depth 0: 4-wide node 0
-    if (n_int > 0) {
-        int* flag = alloc<int>(n_int + 1, st, scratch_bytes);
-        int* idx4 = alloc<int>(n_int + 1, st, scratch_bytes);
-        k_even_depth<<<(n_int + 1 + B - 1) / B, B, 0, st>>>(n_int, parent_int, flag); note_launch();
+    if (wide) {
+        k_even_depth<<<(n_int + 1 + B - 1) / B, B, 0, st>>>(n_int, parent_int, flag4); note_launch();
         BVH_CHECK(cudaGetLastError());
-        size_t tb4 = 0;
-        BVH_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, tb4, flag, idx4, n_int + 1, st));
-        void* t4 = alloc<char>(tb4, st, scratch_bytes);
-        BVH_CHECK(cub::DeviceScan::ExclusiveSum(t4, tb4, flag, idx4, n_int + 1, st));
-        k_pack4<<<(n_int + B - 1) / B, B, 0, st>>>(n_int, flag, idx4, left, right, leaf_box, int_box, out.nodes4);
-        note_launch();
+        BVH_CHECK(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, flag4, idx4, n_int + 1, st));
+        k_pack4<<<(n_int + B - 1) / B, B, 0, st>>>(n_int, flag4, idx4, out.nodes, out.nodes4); note_launch();
         BVH_CHECK(cudaGetLastError());
-        BVH_CHECK(cudaFreeAsync(flag, st));
-        BVH_CHECK(cudaFreeAsync(idx4, st));
-        BVH_CHECK(cudaFreeAsync(t4, st));
     }
-    k_pack_tris<<<(n + B - 1) / B, B, 0, st>>>(n, ids2, in.ref_tri, in.tri_xyz, in.tri_meta, in.tri_local,
-                                                out.tris); note_launch();
+    k_pack_leaves<<<(n + B - 1) / B, B, 0, st>>>(n, ids2, in.ref_tri, in.tri_xyz, in.tri_meta, in.tri_local, out.tris,
+                                                  out.srec, out.drec); note_launch();
     BVH_CHECK(cudaGetLastError());
-    out.srec = alloc<float4>(4 * (size_t) n, st, out.bytes);
-    out.drec = alloc<float4>(8 * (size_t) n, st, out.bytes);
-    k_pack_records<<<(n + B - 1) / B, B, 0, st>>>(n, out.tris, out.srec, out.drec); note_launch();
-    BVH_CHECK(cudaGetLastError());
+}
 
-    void* ptrs[] = {codes, codes2, ids, ids2, left, right, parent_int, parent_leaf, leaf_box, int_box, arrivals, temp};
-    for (void* p : ptrs) BVH_CHECK(cudaFreeAsync(p, st));
+void bvh_check_status(int status)
+{
+    if (status) throw std::runtime_error("bvh: clustering step inconsistent");
 }
 
 // Copies the topology back and checks that a walk from the root reaches every
@@ -625,18 +726,8 @@ std::string bvh_validate(const BvhStorage& s, void* stream)
 
 void bvh_free(BvhStorage& s, void* stream)
 {
-    cudaStream_t st = (cudaStream_t) stream;
-    if (s.nodes) cudaFreeAsync(s.nodes, st);
-    if (s.nodes4) cudaFreeAsync(s.nodes4, st);
-    s.nodes4 = nullptr;
-    if (s.tris) cudaFreeAsync(s.tris, st);
-    if (s.srec) cudaFreeAsync(s.srec, st);
-    if (s.drec) cudaFreeAsync(s.drec, st);
-    s.nodes = nullptr;
-    s.tris = nullptr;
-    s.srec = nullptr;
-    s.drec = nullptr;
-    s.n_tris = 0;
+    if (s.mem) cudaFreeAsync(s.mem, (cudaStream_t) stream);
+    s = BvhStorage();
 }
 
 }  // namespace lg

@@ -25,6 +25,7 @@
 namespace lg {
 
 constexpr int kStack = 64;
+constexpr int kWideTreeMin = 1 << 18;        // leaves from which the 4-wide nodes are built and used (see walk_segment4)
 constexpr int kNoChild = (int) 0x80000000;   // empty slot of a 4-wide node
 constexpr u32 kOccluderBit = 0x80000000u;
 constexpr u32 kInstMask = 0x3fffffffu;
@@ -44,7 +45,7 @@ struct BvhView {
                             // plane test that skips hopeless leaves is off)
 };
 
-// 4-wide nodes, used by the any-hit walk: the binary nodes at even depth with
+// 4-wide nodes, used by the any-hit walk of trees of kWideTreeMin leaves and more: the binary nodes at even depth with
 // their grandchildren as children (2-4 per node), 8 float4 = 128 B:
 //   (min.x of children 0-3) (max.x) (min.y) (max.y) (min.z) (max.z)
 //   (child 0-3 as int bits: >= 0 4-wide node, < 0 leaf ~t, kNoChild empty) (-)
@@ -744,21 +745,27 @@ struct BvhBuildInput {
 };
 
 struct BvhStorage {
+    void* mem = nullptr;       // the allocation that holds the arrays below
+    int* status = nullptr;     // device: [0] nonzero when the build failed (see bvh_check_status)
     float4* nodes = nullptr;   // 4 per internal node
     float4* tris = nullptr;    // 3 per leaf
     float4* srec = nullptr;    // 4 per leaf
     float4* drec = nullptr;    // 8 per leaf
-    float4* nodes4 = nullptr;  // 8 per 4-wide node
+    float4* nodes4 = nullptr;  // 8 per 4-wide node; built from kWideTreeMin leaves on
     int n_tris = 0;
     int root = 0;
     int root4 = 0;
     size_t bytes = 0;
-    void* scratch = nullptr;   // build scratch, freed by bvh_free
     BvhView view() const { BvhView v = {nodes, tris, srec, drec, n_tris, root, nodes4, root4, 0, INFINITY}; return v; }
 };
 
-// Builds into `out` on `stream` (allocations with cudaMallocAsync on that stream).
+// Builds into `out` on `stream` (allocations with cudaMallocAsync on that stream)
+// without waiting for it. A clustering that cannot go on (unordered costs: boxes
+// with NaN or infinities) leaves a tree no query enters and a nonzero
+// status[0], which the caller reads back with its results.
 void bvh_build(const BvhBuildInput& in, BvhStorage& out, void* stream);
+// Throws when `status` (a build's status[0], read back) says that it failed.
+void bvh_check_status(int status);
 void bvh_free(BvhStorage& s, void* stream);
 std::string bvh_validate(const BvhStorage& s, void* stream);
 

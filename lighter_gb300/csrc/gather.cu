@@ -1222,6 +1222,8 @@ LTRAPI ltrg_Gather* ltrg_GatherCreate(const float* tri_xyz, u32 n_tris, const fl
         GCK(cudaMemsetAsync(dgmax, 0, 4, st));
         k_absmax<<<1024, 256, 0, st>>>(g->G32.as<float>(), nn2, dgmax); note_launch();
         u32 herr = 0, hgmax = 0;
+        int hbvh = 0;
+        if (bin.n) GCK(cudaMemcpyAsync(&hbvh, bvh.status, sizeof(int), cudaMemcpyDeviceToHost, st));
         GCK(cudaMemcpyAsync(&hgmax, dgmax, 4, cudaMemcpyDeviceToHost, st));
         GCK(cudaMemcpyAsync(&herr, derr, 4, cudaMemcpyDeviceToHost, st));
         GCK(cudaStreamSynchronize(st));
@@ -1229,6 +1231,7 @@ LTRAPI ltrg_Gather* ltrg_GatherCreate(const float* tri_xyz, u32 n_tris, const fl
         cudaEventElapsedTime(&ms, e0, e1);
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
+        bvh_check_status(hbvh);
         if (herr) throw std::runtime_error("form-factor traversal error word " + std::to_string(herr));
         float gmax;
         memcpy(&gmax, &hgmax, 4);

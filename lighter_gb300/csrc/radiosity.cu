@@ -580,8 +580,7 @@ RadFormFactors build_ff(u32 n, size_t ld, const float4* pos, const float4* nrm, 
         RCK(cudaGetDevice(&dev));
         RCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         unsigned grid = (unsigned) std::min<unsigned long long>((unsigned long long) sms * 8, (n_cand + 127) / 128);
-        // the 4-wide walk for trees of 256k references and more (see walk_segment4)
-        if (bvh.n_tris >= (1 << 18))
+        if (bvh.n_tris >= kWideTreeMin)   // see walk_segment4
             k_ff_visibility<T, true><<<grid, 128, 0, st>>>(ld, pos, bvh, err, links, F, cand, n_cand, counts + 2, counts);
         else
             k_ff_visibility<T, false><<<grid, 128, 0, st>>>(ld, pos, bvh, err, links, F, cand, n_cand, counts + 2, counts);

@@ -93,8 +93,11 @@ LTRAPI LTRBOOL ltrdbg_TraceSegments(const float* tri_xyz, u32 n_tris, const floa
             TCK(cudaMemcpyAsync(out_r, dout, (size_t) n_segs * 4, cudaMemcpyDeviceToHost, st));
         }
         u32 herr = 0;
+        int hbvh = 0;
+        if (built) TCK(cudaMemcpyAsync(&hbvh, bvh.status, sizeof(int), cudaMemcpyDeviceToHost, st));
         TCK(cudaMemcpyAsync(&herr, derr, 4, cudaMemcpyDeviceToHost, st));
         TCK(cudaStreamSynchronize(st));
+        bvh_check_status(hbvh);
         if (herr) throw std::runtime_error("traversal error word set");
     } catch (const std::exception& e) {
         fprintf(stderr, "ltrdbg_TraceSegments: %s\n", e.what());
