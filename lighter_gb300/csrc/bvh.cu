@@ -24,6 +24,7 @@
 #include <cfloat>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <stdexcept>
 #include <string>
@@ -288,17 +289,22 @@ __global__ void k_pack_leaves(int nleaf, const u32* __restrict__ ids, const u32*
 // and halves each iteration instead of growing a chain.
 
 //
-// All iterations run in one launch: a cluster of kPlocCtas blocks, each owning a
+// All iterations run in one launch: one thread-block cluster, each block owning a
 // contiguous run of the list, with two cluster barriers per iteration (merge
 // counts, then the compacted list), and one block alone in shared memory once the
-// list fits its threads. Bound by latency and by the neighbour search of the
-// first iterations. Launched kernel by kernel (as graphs of eight iterations and a
-// read-back of the count) the build of 44,652 references took 2.5 ms, of six 0.6 ms.
+// list fits its threads. Bound by the neighbour search of the first iterations
+// (about 20 instructions per pair) and by the latency of the later ones, so the
+// search is straight-line code over sentinel-padded boxes, and the blocks are as
+// many as a cluster takes: 16 where the device can place such a cluster, 8
+// otherwise, fewer for short lists (ploc_launch). Measured, whole kernel: 44,652
+// references 539 us with 8 blocks and a bounds-checked search -> 264 us, the 1.8k-triangle
+// level (22k references) 328 -> 185 us, a 34-triangle room 33 -> 18 us. Launched kernel by kernel (as graphs of eight
+// iterations and a read-back of the count) the same builds took 2.5 and 1.6 ms.
 
 constexpr int kPlocR = 16;
-constexpr int kPlocT = 1024;     // threads per block, clusters per tile
-constexpr int kPlocCtas = 8;     // blocks of the cluster
-constexpr int kPlocHalo = 2 * kPlocR;
+constexpr int kPlocT = 1024;           // threads per block
+constexpr int kPlocMaxCtas = 16;
+constexpr int kPlocOwn = kPlocT - 2 * kPlocR;   // most clusters a block merges at a time (its threads' less the halo's)
 
 __device__ __forceinline__ float merged_area(const float* a, const float* b)
 {
@@ -314,46 +320,53 @@ struct PlocArgs {
     const u32* ids;               // references in Morton order
     float4* cl[2];                // clusters, 2 per entry: (mn.xyz, mx.x) (mx.yz, node or ~leaf, height)
     u32* flags;                   // per cluster: partner << 2 | merges (lower half of its pair) << 1 | keeps its place
-    unsigned long long* totals;   // [parity][block]: merges << 32 | kept
+    unsigned long long* totals;   // [parity][kPlocMaxCtas]: merges << 32 | kept
     float4* nodes;                // bvh.cuh's binary nodes
     int* parent;                  // per internal node (may be null)
     int* status;                  // see radix_wanted
 };
 
-// A cluster's boxes in shared memory: 16 + 8 bytes, read as two vectors.
+// Clusters' boxes in shared memory (16 + 8 bytes, read as two vectors), kPlocR
+// slots more on either side. A slot without a cluster holds a box whose merged
+// area with any other is infinite.
 struct PlocBoxes {
-    float4 a[kPlocT + 2 * kPlocHalo];   // mn.xyz, mx.x
-    float2 b[kPlocT + 2 * kPlocHalo];   // mx.yz
+    float4 a[kPlocT + 2 * kPlocR];   // mn.xyz, mx.x
+    float2 b[kPlocT + 2 * kPlocR];   // mx.yz
+    __device__ __forceinline__ void none(int k)
+    {
+        a[k] = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, FLT_MAX);
+        b[k] = make_float2(FLT_MAX, FLT_MAX);
+    }
+    __device__ __forceinline__ void get(int k, float* o) const
+    {
+        const float4 p = a[k];
+        const float2 q = b[k];
+        o[0] = p.x; o[1] = p.y; o[2] = p.z; o[3] = p.w; o[4] = q.x; o[5] = q.y;
+    }
 };
 
-__device__ __forceinline__ void ploc_box(const PlocBoxes& s, int k, float* o)
-{
-    const float4 p = s.a[k];
-    const float2 q = s.b[k];
-    o[0] = p.x; o[1] = p.y; o[2] = p.z; o[3] = p.w; o[4] = q.x; o[5] = q.y;
-}
-
-// The nearest neighbour of cluster i (at slot k of the boxes) as a key that orders
-// its pairs: cost, then list distance, parity of the lower position, the lower
-// position (26 bits; bvh_build keeps longer lists away). ~0: none.
-__device__ __forceinline__ unsigned long long ploc_nearest(const PlocBoxes& s, int k, int i, int count)
+// The nearest neighbour of cluster i (at slot k) as a key that orders its pairs:
+// cost (a non-negative float's bits), then list distance, parity of the lower
+// position, the lower position (26 bits; bvh_build keeps longer lists away).
+// ~0: none (no finite cost).
+__device__ __forceinline__ unsigned long long ploc_nearest(const PlocBoxes& s, int k, int i)
 {
     float me[6];
-    ploc_box(s, k, me);
+    s.get(k, me);
+    const u32 same = ((u32) (i & 1) << 26) | (u32) i, flip = same ^ (1u << 26);
     unsigned long long best = ~0ull;
+#pragma unroll
     for (int d = -kPlocR; d <= kPlocR; ++d) {
-        const int j = i + d;
-        if (d == 0 || j < 0 || j >= count) continue;
+        if (d == 0) continue;
         float o[6];
-        ploc_box(s, k + d, o);
+        s.get(k + d, o);
         const float c = merged_area(me, o);
-        if (!(c <= FLT_MAX)) continue;
-        const u32 mn = (u32) min(i, j);
-        const u32 tie = ((u32) (d < 0 ? -d : d) << 27) | ((mn & 1u) << 26) | mn;
+        // lower position i (d > 0) or i + d, whose parity differs from i's when d is odd
+        const u32 tie = d > 0 ? same + ((u32) d << 27) : ((d & 1) ? flip : same) + (u32) d + ((u32) -d << 27);
         const unsigned long long key = ((unsigned long long) __float_as_uint(c) << 32) | tie;
         best = key < best ? key : best;
     }
-    return best;
+    return (u32) (best >> 32) <= __float_as_uint(FLT_MAX) ? best : ~0ull;
 }
 
 __device__ __forceinline__ int ploc_partner(unsigned long long key, int i)
@@ -411,14 +424,14 @@ __device__ __forceinline__ void ploc_cluster_sync()
     asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
 }
 
-__global__ void __cluster_dims__(kPlocCtas, 1, 1) __launch_bounds__(kPlocT) k_ploc(PlocArgs p)
+__global__ void __launch_bounds__(kPlocT) k_ploc(PlocArgs p)
 {
     __shared__ PlocBoxes box;
-    __shared__ unsigned long long key[kPlocT + 2 * kPlocR];
+    __shared__ unsigned long long key[kPlocT];
     __shared__ int2 ref[kPlocT];   // the tail's (node or ~leaf, height)
     __shared__ u32 wsum[32];
-    const int tid = threadIdx.x, rank = blockIdx.x;
-    for (int i = rank * kPlocT + tid; i < p.n; i += kPlocCtas * kPlocT) {
+    const int tid = threadIdx.x, rank = blockIdx.x, ctas = gridDim.x;
+    for (int i = rank * kPlocT + tid; i < p.n; i += ctas * kPlocT) {
         float b[6];
         leaf_box_of(p.ref_box + 6 * (size_t) p.ids[i], b);
         p.cl[0][2 * (size_t) i] = make_float4(b[0], b[1], b[2], b[3]);
@@ -428,33 +441,32 @@ __global__ void __cluster_dims__(kPlocCtas, 1, 1) __launch_bounds__(kPlocT) k_pl
     int count = p.n, base = p.n - 1, cur = 0;
     bool ok = true;
     for (int par = 0; ok && count > kPlocT; par ^= 1) {
-        const float4* src = p.cl[cur];
-        float4* dst = p.cl[cur ^ 1];
-        const int tiles = (count + kPlocT - 1) / kPlocT, per = (tiles + kPlocCtas - 1) / kPlocCtas;
-        const int t0 = min(tiles, rank * per), t1 = min(tiles, t0 + per);
+        const float4* src = cur ? p.cl[1] : p.cl[0];
+        float4* dst = cur ? p.cl[0] : p.cl[1];
+        // this block's run [r0, r1), in tiles of `own` clusters: thread t stands for
+        // cluster start - kPlocR + t, and merges it when it lies in the tile
+        const int run = (count + ctas - 1) / ctas, r0 = min(count, rank * run), r1 = min(count, r0 + run);
+        const int tiles = (r1 - r0 + kPlocOwn - 1) / kPlocOwn, own = tiles ? (r1 - r0 + tiles - 1) / tiles : 0;
         u32 kept = 0, merged = 0;
-        for (int t = t0; t < t1; ++t) {
-            const int start = t * kPlocT;
-            for (int k = tid; k < kPlocT + 2 * kPlocHalo; k += kPlocT) {
-                const int g = start - kPlocHalo + k;
-                if (g >= 0 && g < count) {
-                    const float4 a = __ldcg(src + 2 * (size_t) g), b = __ldcg(src + 2 * (size_t) g + 1);
-                    box.a[k] = a;
-                    box.b[k] = make_float2(b.x, b.y);
-                }
+        for (int t = 0; t < tiles; ++t) {
+            const int start = r0 + t * own, end = min(r1, start + own), i = start - kPlocR + tid;
+            {
+                const int g0 = i - kPlocR, g1 = g0 + kPlocT;   // slots tid and, for the last ones, tid + kPlocT
+                const bool in0 = g0 >= 0 && g0 < count, two = tid < 2 * kPlocR, in1 = two && g1 < count;
+                float4 a0, b0, a1, b1;
+                if (in0) { a0 = __ldcg(src + 2 * (size_t) g0); b0 = __ldcg(src + 2 * (size_t) g0 + 1); }
+                if (in1) { a1 = __ldcg(src + 2 * (size_t) g1); b1 = __ldcg(src + 2 * (size_t) g1 + 1); }
+                if (in0) { box.a[tid] = a0; box.b[tid] = make_float2(b0.x, b0.y); } else box.none(tid);
+                if (in1) { box.a[tid + kPlocT] = a1; box.b[tid + kPlocT] = make_float2(b1.x, b1.y); }
+                else if (two) box.none(tid + kPlocT);
             }
             __syncthreads();
-            // neighbours of the tile's clusters and of kPlocR more on either side
-            for (int k = tid; k < kPlocT + 2 * kPlocR; k += kPlocT) {
-                const int i = start - kPlocR + k;
-                if (i >= 0 && i < count) key[k] = ploc_nearest(box, k + kPlocR, i, count);
-            }
+            if (i >= 0 && i < min(count, end + kPlocR)) key[tid] = ploc_nearest(box, tid + kPlocR, i);
             __syncthreads();
-            const int i = start + tid;
             bool keep = false, merge = false;
-            if (i < count) {
-                const int j = ploc_partner(key[tid + kPlocR], i);
-                const bool mutual = j >= 0 && ploc_partner(key[j - start + kPlocR], j) == i;
+            if (i >= start && i < end) {
+                const int j = ploc_partner(key[tid], i);
+                const bool mutual = j >= 0 && ploc_partner(key[tid + j - i], j) == i;
                 merge = mutual && i < j;
                 keep = !(mutual && i > j);
                 p.flags[i] = ((u32) j << 2) | (merge ? 2u : 0u) | (keep ? 1u : 0u);
@@ -462,18 +474,18 @@ __global__ void __cluster_dims__(kPlocCtas, 1, 1) __launch_bounds__(kPlocT) k_pl
             kept += (u32) __syncthreads_count(keep);
             merged += (u32) __syncthreads_count(merge);
         }
-        if (tid == 0) p.totals[par * kPlocCtas + rank] = ((unsigned long long) merged << 32) | kept;
+        if (tid == 0) p.totals[par * kPlocMaxCtas + rank] = ((unsigned long long) merged << 32) | kept;
         ploc_cluster_sync();
         unsigned long long before = 0, total = 0;
-        for (int r = 0; r < kPlocCtas; ++r) {
-            const unsigned long long v = __ldcg(p.totals + par * kPlocCtas + r);
+        for (int r = 0; r < ctas; ++r) {
+            const unsigned long long v = __ldcg(p.totals + par * kPlocMaxCtas + r);
             if (r < rank) before += v;
             total += v;
         }
         u32 pos = (u32) before, mrk = (u32) (before >> 32);
-        for (int t = t0; t < t1; ++t) {
-            const int i = t * kPlocT + tid;
-            const u32 f = i < count ? p.flags[i] : 0u;
+        for (int t = 0; t < tiles; ++t) {
+            const int start = r0 + t * own, end = min(r1, start + own), i = start - kPlocR + tid;
+            const u32 f = i >= start && i < end ? p.flags[i] : 0u;
             u32 tot;
             const u32 ex = ploc_scan((f & 1u) != 0, (f & 2u) != 0, wsum, tot);
             if (f & 1u) {
@@ -498,19 +510,23 @@ __global__ void __cluster_dims__(kPlocCtas, 1, 1) __launch_bounds__(kPlocT) k_pl
     }
     if (rank != 0) return;
     // the list fits this block's threads: one cluster per thread, in shared memory
+    // (cluster t at slot t + kPlocR)
+    const float4* last = cur ? p.cl[1] : p.cl[0];
     float4 c0 = make_float4(0, 0, 0, 0), c1 = c0;
     if (ok && tid < count) {
-        c0 = __ldcg(p.cl[cur] + 2 * (size_t) tid);
-        c1 = __ldcg(p.cl[cur] + 2 * (size_t) tid + 1);
+        c0 = __ldcg(last + 2 * (size_t) tid);
+        c1 = __ldcg(last + 2 * (size_t) tid + 1);
     }
+    if (tid < kPlocR) box.none(tid);
     while (ok && count > 1) {
         if (tid < count) {
-            box.a[tid] = c0;
-            box.b[tid] = make_float2(c1.x, c1.y);
+            box.a[tid + kPlocR] = c0;
+            box.b[tid + kPlocR] = make_float2(c1.x, c1.y);
             ref[tid] = make_int2(__float_as_int(c1.z), __float_as_int(c1.w));
         }
+        if (tid < kPlocR) box.none(count + kPlocR + tid);
         __syncthreads();
-        if (tid < count) key[tid] = ploc_nearest(box, tid, tid, count);
+        if (tid < count) key[tid] = ploc_nearest(box, tid + kPlocR, tid);
         __syncthreads();
         bool keep = false, merge = false;
         int j = -1;
@@ -523,8 +539,8 @@ __global__ void __cluster_dims__(kPlocCtas, 1, 1) __launch_bounds__(kPlocT) k_pl
         u32 tot;
         const u32 ex = ploc_scan(keep, merge, wsum, tot);
         if (merge) {
-            const float4 b0 = box.a[j];
-            const float2 q = box.b[j];
+            const float4 b0 = box.a[j + kPlocR];
+            const float2 q = box.b[j + kPlocR];
             const int2 r = ref[j];
             ploc_merge(p, base - 1 - (int) (ex >> 16), c0, c1, b0,
                        make_float4(q.x, q.y, __int_as_float(r.x), __int_as_float(r.y)), c0, c1);
@@ -532,8 +548,8 @@ __global__ void __cluster_dims__(kPlocCtas, 1, 1) __launch_bounds__(kPlocT) k_pl
         __syncthreads();   // partners read
         if (keep) {
             const u32 o = ex & 0xffffu;
-            box.a[o] = c0;
-            box.b[o] = make_float2(c1.x, c1.y);
+            box.a[o + kPlocR] = c0;
+            box.b[o + kPlocR] = make_float2(c1.x, c1.y);
             ref[o] = make_int2(__float_as_int(c1.z), __float_as_int(c1.w));
         }
         __syncthreads();
@@ -541,8 +557,8 @@ __global__ void __cluster_dims__(kPlocCtas, 1, 1) __launch_bounds__(kPlocT) k_pl
         count = (int) (tot & 0xffffu);
         base -= (int) (tot >> 16);
         if (tid < count) {
-            c0 = box.a[tid];
-            const float2 q = box.b[tid];
+            c0 = box.a[tid + kPlocR];
+            const float2 q = box.b[tid + kPlocR];
             const int2 r = ref[tid];
             c1 = make_float4(q.x, q.y, __int_as_float(r.x), __int_as_float(r.y));
         }
@@ -552,6 +568,42 @@ __global__ void __cluster_dims__(kPlocCtas, 1, 1) __launch_bounds__(kPlocT) k_pl
         p.status[0] = ok && count == 1 && base == 0 ? 0 : 1;
         p.status[1] = __float_as_int(c1.w);
     }
+}
+
+// Blocks of the clustering's cluster for n references: one per full block of
+// them (a longer list per block costs more than the wider barrier), up to the
+// largest cluster that the current device can place.
+cudaError_t ploc_launch(const PlocArgs& pa, cudaStream_t st)
+{
+    static std::atomic<int> largest[64];   // per device, 0 = not asked yet
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.blockDim = dim3(kPlocT);
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int most = dev < 64 ? largest[dev].load() : 8;
+    if (!most) {
+        most = 8;   // the portable limit
+        if (cudaFuncSetAttribute(k_ploc, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+            int fit = 0;
+            at.val.clusterDim.x = kPlocMaxCtas;
+            cfg.gridDim = dim3(kPlocMaxCtas);
+            if (cudaOccupancyMaxActiveClusters(&fit, k_ploc, &cfg) == cudaSuccess && fit > 0) most = kPlocMaxCtas;
+        }
+        cudaGetLastError();   // an answer of "no" is not an error of the build
+        largest[dev].store(most);
+    }
+    int ctas = 1;
+    while (ctas < most && ctas * kPlocT < pa.n) ctas *= 2;
+    at.val.clusterDim.x = (unsigned) ctas;
+    cfg.gridDim = dim3((unsigned) ctas);
+    return cudaLaunchKernelEx(&cfg, k_ploc, pa);
 }
 
 // Parts of one device allocation, 256-byte aligned: a first pass adds up the
@@ -621,7 +673,7 @@ void bvh_build(const BvhBuildInput& in, BvhStorage& out, void* stream)
         sort_tmp = c.take<char>(sort_bytes);
         for (float4*& p : cl) p = c.take<float4>(ploc ? 2 * (size_t) n : 0);
         flags = c.take<u32>(ploc ? n : 0);
-        totals = c.take<unsigned long long>(2 * kPlocCtas);
+        totals = c.take<unsigned long long>(2 * kPlocMaxCtas);
         flag4 = c.take<int>(wide ? n : 0);
         idx4 = c.take<int>(wide ? n : 0);
         scan_tmp = c.take<char>(scan_bytes);
@@ -658,8 +710,7 @@ void bvh_build(const BvhBuildInput& in, BvhStorage& out, void* stream)
         pa.nodes = out.nodes;
         pa.parent = wide ? parent_int : nullptr;
         pa.status = out.status;
-        k_ploc<<<kPlocCtas, kPlocT, 0, st>>>(pa); note_launch();
-        BVH_CHECK(cudaGetLastError());
+        BVH_CHECK(ploc_launch(pa, st)); note_launch();
     }
     if (n_int > 0) {
         const int* status = ploc ? out.status : nullptr;
