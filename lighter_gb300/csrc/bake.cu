@@ -530,14 +530,23 @@ __device__ __forceinline__ float inv_shadow(const BvhView& bvh, V3 from, V3 to, 
     return res;
 }
 
+// A lane takes part in a step of the warp's sphere traces while it is at most this
+// far (along its segment) ahead of the hindmost one: lanes that ran ahead through
+// open space would drag the shared walk through two places at once. Any value gives
+// the same results; the trace kernel of the benchmark's level, of the terrain and
+// of a 1.8k-triangle level took 17.0, 48.8 and 1.87 ms without a bound, 13.8, 36.8 and 1.38
+// with 2 m, 12.8, 37.1 and 1.35 with 8 m, 13.1, 38.1 and 1.35 with 16 m.
+constexpr float kMarchLead = 8.0f;
+
 // inv_shadow for the 32 lanes of a warp at once (every lane calls it; `has`
-// marks the lanes with a pair): each step runs one warp_distance for all lanes
-// still marching, so the lanes walk the BVH together instead of 32 divergent
-// walks. Every lane makes the same queries (points and radii) as inv_shadow
-// and gets the same distances, so the factor is inv_shadow's bit for bit.
+// marks the lanes with a pair): each step runs one warp_distance for the lanes
+// still marching near the hindmost, so the lanes walk the BVH together instead of 32
+// divergent walks. Every lane makes the same queries (points and radii) as
+// inv_shadow and gets the same distances, so the factor is inv_shadow's bit for bit.
 __device__ __forceinline__ float inv_shadow_warp(const BvhView& bvh, bool has, V3 from, V3 to, float k, ErrFlag err,
                                                  u32& nq, u32& nv, u32& nt)
 {
+    const unsigned full = 0xffffffffu;
     V3 rd = mk(0, 0, 0);
     float maxt = 0.0f;
     if (has) {
@@ -547,27 +556,29 @@ __device__ __forceinline__ float inv_shadow_warp(const BvhView& bvh, bool has, V
     float res = 1.0f;
     float reach = kMaxPenumbraSize;
     float t = 0.001f;
-    bool active = has && t < maxt;
-    while (__any_sync(0xffffffffu, active)) {
+    bool marching = has && t < maxt;
+    while (__any_sync(full, marching)) {
+        const float hind = redux_min(marching ? t : INFINITY);
+        const bool active = marching && t <= hind + kMarchLead;
         const V3 p = from + rd * t;
         const float r0 = fminf(kMaxPenumbraSize, reach * 1.0001f + 1e-5f);
         float h = warp_distance(bvh, p, r0, active, err, nv, nt);
         if (active) ++nq;
         const bool again = active && !(h < r0) && r0 < kMaxPenumbraSize;
-        if (__any_sync(0xffffffffu, again)) {
+        if (__any_sync(full, again)) {
             const float h2 = warp_distance(bvh, p, kMaxPenumbraSize, again, err, nv, nt);
             if (again) { h = h2; ++nq; }
         }
         if (active) {
             if (h < 0.001f) {
                 res = 0.0f;
-                active = false;
+                marching = false;
             } else {
                 res = fmin_(res, h / fmin_(t * k, kMaxPenumbraSize));
                 const float step = fmin_(h, kMaxPenumbraStep);
                 reach = h + step;
                 t += step;
-                active = t < maxt;
+                marching = t < maxt;
             }
         }
     }
@@ -839,7 +850,15 @@ __device__ __forceinline__ void direct_pair_warp(const DirectArgs& a, bool has, 
     }
     const float vis = a.shadow_mode == 1 ? sampled_vis_warp(a, has, L, t)
                                          : inv_shadow_warp(a.bvh, has, t.from, t.to, L.radius, a.err, nq, nv, nt);
-    if (has) direct_pair_finish(a, w, L, t, vis);
+    // The light and its terms are evaluated again (through an index the compiler
+    // cannot see through) instead of being kept across the trace: eight registers
+    // less there, which is a fifth block of 128 threads per SM (terrain 37.0 -> 33.3 ms).
+    asm volatile("" : "+r"(w));
+    if (has) {
+        L = a.lights[w / a.n_samples];
+        light_terms(a, L, w % a.n_samples, t);
+        direct_pair_finish(a, w, L, t, vis);
+    }
 }
 
 // Outputs of one traced pair from its shadow factor.
@@ -901,6 +920,8 @@ __device__ __forceinline__ void direct_trace_body(const DirectArgs& a, const u32
                 c_traced += a.shadow_mode == 1 ? (unsigned) a.lights[w / a.n_samples].ns : 1u;
                 c_pairs += 1;
                 c_nq += nq;
+            }
+            if (lane == 0) {   // the warp's walks, counted by every lane
                 c_nv += nv;
                 c_nt += nt;
             }
@@ -1374,7 +1395,7 @@ __global__ void k_direct_batch_offsets(const DirectJob* __restrict__ jobs, int n
 __device__ __forceinline__ void flush_direct(Counters* c, unsigned long long& tr, unsigned long long& nq,
                                              unsigned long long& nv, unsigned long long& nt, unsigned long long& np)
 {
-    if (c && tr) {
+    if (c && (tr | nv)) {
         atomicAdd(&c->shadow_pairs, np);
         atomicAdd(&c->shadow_evals, tr);
         atomicAdd(&c->distance_queries, nq);
@@ -1427,8 +1448,10 @@ __global__ void k_direct_trace_batch(const DirectJob* __restrict__ jobs, int n, 
             c_pairs += 1;
         }
         c_nq += nq;
-        c_nv += nv;
-        c_nt += nt;
+        if (!kPacket || lane == 0) {   // a packet's walks are counted by every lane
+            c_nv += nv;
+            c_nt += nt;
+        }
     }
     if (cur >= 0) flush_direct(a.counters, c_traced, c_nq, c_nv, c_nt, c_pairs);
 }

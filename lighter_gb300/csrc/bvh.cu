@@ -157,6 +157,25 @@ __global__ void k_refit(const int* __restrict__ status, const float* ref_box, co
     }
 }
 
+// Binary node i (layout in bvh.cuh) from its children's boxes (min xyz, max xyz) and refs.
+__device__ __forceinline__ void put_node(float4* nodes, size_t i, const float* L, int l, const float* R, int r)
+{
+    float4* o = nodes + 4 * i;
+    o[0] = make_float4(L[0], R[0], L[1], R[1]);
+    o[1] = make_float4(L[2], R[2], L[3], R[3]);
+    o[2] = make_float4(L[4], R[4], L[5], R[5]);
+    o[3] = make_float4(__int_as_float(l), __int_as_float(r), 0.0f, 0.0f);
+}
+
+// Child s (0 left, 1 right) of binary node i: its box; returns its ref.
+__device__ __forceinline__ int get_child(const float4* nodes, size_t i, int s, float* box)
+{
+    const float* f = reinterpret_cast<const float*>(nodes + 4 * i);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) box[c] = f[2 * c + s];
+    return __float_as_int(f[12 + s]);
+}
+
 // Nodes of the radix hierarchy; or, after a failed clustering, nodes whose boxes
 // no query enters, so that the kernels queued behind the build end at the root
 // (the failure itself reaches the host with their results).
@@ -166,22 +185,15 @@ __global__ void k_pack_nodes(const int* __restrict__ status, int n_int, const in
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_int) return;
     if (status && status[0] != 0) {
-        float4* o = nodes + 4 * (size_t) i;
-        o[0] = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX);
-        o[1] = make_float4(-FLT_MAX, -FLT_MAX, FLT_MAX, FLT_MAX);
-        o[2] = make_float4(FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX);
-        o[3] = make_float4(__int_as_float(~0), __int_as_float(~0), 0.0f, 0.0f);
+        const float none[6] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
+        put_node(nodes, i, none, ~0, none, ~0);
         return;
     }
     if (!radix_wanted(status)) return;
     int l = left[i], r = right[i];
     const float* L = l < 0 ? leaf_box + 6 * (size_t) (~l) : int_box + 6 * (size_t) l;
     const float* R = r < 0 ? leaf_box + 6 * (size_t) (~r) : int_box + 6 * (size_t) r;
-    float4* o = nodes + 4 * (size_t) i;
-    o[0] = make_float4(L[0], L[1], L[2], L[3]);
-    o[1] = make_float4(L[4], L[5], R[0], R[1]);
-    o[2] = make_float4(R[2], R[3], R[4], R[5]);
-    o[3] = make_float4(__int_as_float(l), __int_as_float(r), 0.0f, 0.0f);
+    put_node(nodes, i, L, l, R, r);
 }
 
 // ---- 4-wide nodes: the binary nodes at even depth, with their grandchildren as children
@@ -219,16 +231,15 @@ __global__ void k_pack4(int n_int, const int* __restrict__ flag, const int* __re
     float4* o = nodes4 + 8 * (size_t) idx4[i];
     const float empty_box[6] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
     int k = 0;
-    const float* f = reinterpret_cast<const float*>(nodes + 4 * (size_t) i);
     for (int s = 0; s < 2; ++s) {
-        const int c = __float_as_int(f[12 + s]);
+        float box[6];
+        const int c = get_child(nodes, i, s, box);
         if (c < 0) {
-            put_slot(o, k++, f + 6 * s, c);
+            put_slot(o, k++, box, c);
         } else {
-            const float* g = reinterpret_cast<const float*>(nodes + 4 * (size_t) c);
             for (int q = 0; q < 2; ++q) {
-                const int gc = __float_as_int(g[12 + q]);
-                put_slot(o, k++, g + 6 * q, gc < 0 ? gc : idx4[gc]);
+                const int gc = get_child(nodes, c, q, box);
+                put_slot(o, k++, box, gc < 0 ? gc : idx4[gc]);
             }
         }
     }
@@ -404,11 +415,8 @@ __device__ __forceinline__ void ploc_merge(const PlocArgs& p, int id, float4 a0,
                                            float4& o0, float4& o1)
 {
     const int ca = __float_as_int(a1.z), cb = __float_as_int(b1.z);
-    float4* nd = p.nodes + 4 * (size_t) id;
-    nd[0] = a0;
-    nd[1] = make_float4(a1.x, a1.y, b0.x, b0.y);
-    nd[2] = make_float4(b0.z, b0.w, b1.x, b1.y);
-    nd[3] = make_float4(a1.z, b1.z, 0.0f, 0.0f);
+    const float boxa[6] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y}, boxb[6] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y};
+    put_node(p.nodes, id, boxa, ca, boxb, cb);
     if (p.parent) {
         if (ca >= 0) p.parent[ca] = id;
         if (cb >= 0) p.parent[cb] = id;

@@ -4,9 +4,12 @@
 // lighter_math.cpp:804-1044, lighter.cpp:112-289).
 //
 // Layout in HBM (built by bvh.cu, LBVH with single-triangle leaves):
-//   nodes : 4 x float4 per internal node (64 B, one 128-byte line pair):
-//           n0 = (L.min.xyz, L.max.x)  n1 = (L.max.yz, R.min.xy)
-//           n2 = (R.min.z, R.max.xyz)  n3 = (int L, int R, -, -)
+//   nodes : 4 x float4 per internal node (64 B, one 128-byte line pair), each
+//           plane of both children side by side so that one packed instruction
+//           works on the two:
+//           n0 = (L.min.x, R.min.x, L.min.y, R.min.y)
+//           n1 = (L.min.z, R.min.z, L.max.x, R.max.x)
+//           n2 = (L.max.y, R.max.y, L.max.z, R.max.z)  n3 = (int L, int R, -, -)
 //           child >= 0: internal node; child < 0: leaf holding triangle ~child.
 //   tris  : 3 x float4 per leaf (triangle reference) in leaf order:
 //           (P1.xyz, meta) (P2.xyz, local index) (P3.xyz, build index)
@@ -144,8 +147,8 @@ __device__ __forceinline__ NodeBoxes load_node(const BvhView& b, int n)
     const float4* p = b.nodes + 4 * n;
     float4 n0 = __ldg(p), n1 = __ldg(p + 1), n2 = __ldg(p + 2), n3 = __ldg(p + 3);
     NodeBoxes o;
-    o.lmin = mk(n0.x, n0.y, n0.z); o.lmax = mk(n0.w, n1.x, n1.y);
-    o.rmin = mk(n1.z, n1.w, n2.x); o.rmax = mk(n2.y, n2.z, n2.w);
+    o.lmin = mk(n0.x, n0.z, n1.x); o.lmax = mk(n1.z, n2.x, n2.z);
+    o.rmin = mk(n0.y, n0.w, n1.y); o.rmax = mk(n1.w, n2.y, n2.w);
     o.l = __float_as_int(n3.x); o.r = __float_as_int(n3.y);
     return o;
 }
@@ -504,10 +507,11 @@ __device__ __forceinline__ float bvh_distance(const BvhView& b, V3 p, float d0, 
 // test of the walk against its own query. The walk visits a superset of the
 // nodes each lane's own walk would visit, and a subtree is dropped only when,
 // for every lane, it lies beyond that lane's current limit, so every lane gets
-// exactly the result of the per-lane query. The stack is warp-uniform and
-// lives in registers spread over the lanes (entry i in lane i % 32, slot
-// i / 32; 64 entries, more than the tree's depth). Every lane of the warp
-// must call these (converged).
+// exactly the result of the per-lane query. A lane that takes no part, or has its
+// answer, holds a negative limit that no box meets, so the walk needs no other
+// mask. The stack is warp-uniform and lives in registers spread over the lanes
+// (entry i in lane i % 32, slot i / 32; 64 entries, more than the tree's depth).
+// Every lane of the warp must call these (converged).
 
 // Pushes `n` on the warp's stack (or records error bit 0 past 64 entries).
 __device__ __forceinline__ void wstack_push(int& s0, int& s1, int& sp, int n, ErrFlag err)
@@ -527,43 +531,97 @@ __device__ __forceinline__ int wstack_pop(int s0, int s1, int& sp)
     return __shfl_sync(0xffffffffu, sp < 32 ? s0 : s1, sp & 31);
 }
 
-// The child a warp enters first when the lanes reach both: the one more of
-// those lanes find nearer.
-__device__ __forceinline__ bool warp_left_first(bool hl, bool hr, bool lnear)
+// The least of the lanes' values, in every lane.
+__device__ __forceinline__ float redux_min(float v)
 {
-    const unsigned both = __ballot_sync(0xffffffffu, hl && hr);
-    const unsigned ln = __ballot_sync(0xffffffffu, hl && hr && lnear);
-    return 2 * __popc(ln) >= __popc(both);
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
 }
 
+// The child a warp enters first when lanes reach both (ml: the left, mr: the
+// right): the one more of the lanes that reach both find nearer.
+__device__ __forceinline__ bool warp_left_first(unsigned ml, unsigned mr, bool lnear)
+{
+    const unsigned both = ml & mr, near = __ballot_sync(0xffffffffu, lnear) & both;
+    return 2 * __popc(near) >= __popc(both);
+}
+
+// A node with both children's planes as pairs (left in the low half).
+struct NodePairs { F2 mnx, mny, mnz, mxx, mxy, mxz; int l, r; };
+
+__device__ __forceinline__ NodePairs load_pairs(const BvhView& b, int n)
+{
+    const ulonglong2* p = reinterpret_cast<const ulonglong2*>(b.nodes + 4 * n);
+    const ulonglong2 n0 = __ldg(p), n1 = __ldg(p + 1), n2 = __ldg(p + 2);
+    const int2 n3 = __ldg(reinterpret_cast<const int2*>(p + 3));
+    return NodePairs{n0.x, n0.y, n1.x, n1.y, n2.x, n2.y, n3.x, n3.y};
+}
+
+// box_d2 of both children: the distances along an axis of the point pp (both halves) ...
+__device__ __forceinline__ F2 gap_pair(F2 mn, F2 mx, F2 pp, F2 minus1)
+{
+    float a0, a1, b0, b1;
+    f2_get(f2_fma(pp, minus1, mn), a0, a1);   // mn - p
+    f2_get(f2_fma(mx, minus1, pp), b0, b1);   // p - mx
+    return f2_make(max3(a0, b0, 0.0f), max3(a1, b1, 0.0f));
+}
+
+// ... and slab of both children, inv and the negated o * inv in both halves.
+struct SlabPairs {
+    F2 ix, iy, iz, ox, oy, oz;
+    __device__ __forceinline__ SlabPairs(V3 inv, V3 o)
+        : ix(f2_make(inv.x, inv.x)), iy(f2_make(inv.y, inv.y)), iz(f2_make(inv.z, inv.z)),
+          ox(f2_make(-(o.x * inv.x), -(o.x * inv.x))), oy(f2_make(-(o.y * inv.y), -(o.y * inv.y))),
+          oz(f2_make(-(o.z * inv.z), -(o.z * inv.z)))
+    {
+    }
+    __device__ __forceinline__ void test(const NodePairs& n, float tlimit, bool& hl, bool& hr, float& tl, float& tr) const
+    {
+        float ax, bx, cx, dx, ay, by, cy, dy, az, bz, cz, dz;
+        f2_get(f2_fma(n.mnx, ix, ox), ax, bx);
+        f2_get(f2_fma(n.mxx, ix, ox), cx, dx);
+        f2_get(f2_fma(n.mny, iy, oy), ay, by);
+        f2_get(f2_fma(n.mxy, iy, oy), cy, dy);
+        f2_get(f2_fma(n.mnz, iz, oz), az, bz);
+        f2_get(f2_fma(n.mxz, iz, oz), cz, dz);
+        tl = fmaxf(max3(fminf(ax, cx), fminf(ay, cy), fminf(az, cz)), 0.0f);
+        tr = fmaxf(max3(fminf(bx, dx), fminf(by, dy), fminf(bz, dz)), 0.0f);
+        hl = tl <= fminf(min3(fmaxf(ax, cx), fmaxf(ay, cy), fmaxf(az, cz)), tlimit);
+        hr = tr <= fminf(min3(fmaxf(bx, dx), fmaxf(by, dy), fmaxf(bz, dz)), tlimit);
+    }
+};
+
 // bvh_distance for the active lanes: min(d0, min over occluder triangles of
-// the exact point-triangle distance), each lane with its own point and radius.
+// the exact point-triangle distance), each lane with its own point and radius;
+// d0 for the other lanes. nv and nt count the walk's nodes and exact tests (in every lane).
 __device__ __forceinline__ float warp_distance(const BvhView& b, V3 p, float d0, bool active, ErrFlag err, u32& nv,
                                                u32& nt)
 {
-    float dist = d0;
-    const unsigned am = __ballot_sync(0xffffffffu, active);
-    if (b.n_tris <= 0 || !am) return dist;
-    // the walk's node and leaf fetches are counted once for the warp, by its lowest active lane
-    const bool counter = (int) (threadIdx.x & 31) == __ffs(am) - 1;
+    const unsigned full = 0xffffffffu;
+    if (b.n_tris <= 0 || !__any_sync(full, active)) return d0;
+    float dist = active ? d0 : -INFINITY;
+    float lim = active ? d0 * d0 : -1.0f;
+    const F2 px = f2_make(p.x, p.x), py = f2_make(p.y, p.y), pz = f2_make(p.z, p.z), minus1 = f2_make(-1.0f, -1.0f);
     int s0 = 0, s1 = 0, sp = 0;
     int cur = b.root;
     for (;;) {
         if (cur >= 0) {
-            const NodeBoxes nb = load_node(b, cur);
-            if (counter) ++nv;
-            const float lim = dist * dist;
-            const float dl = box_d2(nb.lmin, nb.lmax, p), dr = box_d2(nb.rmin, nb.rmax, p);
-            const bool hl = active && dl <= lim, hr = active && dr <= lim;
-            const unsigned ml = __ballot_sync(0xffffffffu, hl), mr = __ballot_sync(0xffffffffu, hr);
+            const NodePairs nd = load_pairs(b, cur);
+            ++nv;
+            const F2 gx = gap_pair(nd.mnx, nd.mxx, px, minus1), gy = gap_pair(nd.mny, nd.mxy, py, minus1),
+                     gz = gap_pair(nd.mnz, nd.mxz, pz, minus1);
+            float dl, dr;
+            f2_get(f2_fma(gx, gx, f2_fma(gy, gy, f2_mul(gz, gz))), dl, dr);
+            const unsigned ml = __ballot_sync(full, dl <= lim), mr = __ballot_sync(full, dr <= lim);
             if (ml && mr) {
-                const bool lfirst = warp_left_first(hl, hr, dl <= dr);
-                wstack_push(s0, s1, sp, lfirst ? nb.r : nb.l, err);
-                cur = lfirst ? nb.l : nb.r;
+                const bool lfirst = warp_left_first(ml, mr, dl <= dr);
+                wstack_push(s0, s1, sp, lfirst ? nd.r : nd.l, err);
+                cur = lfirst ? nd.l : nd.r;
                 continue;
             }
-            if (ml) { cur = nb.l; continue; }
-            if (mr) { cur = nb.r; continue; }
+            if (ml) { cur = nd.l; continue; }
+            if (mr) { cur = nd.r; continue; }
         } else {
             const int t = ~cur;
             const float4* r = b.drec + 8 * (size_t) t;
@@ -572,16 +630,16 @@ __device__ __forceinline__ float warp_distance(const BvhView& b, V3 p, float d0,
                 // The exact test returns the plane distance pd or more (less rounding,
                 // at most dist_margin), so a lane whose limit is below pd - margin
                 // cannot take a smaller distance from this triangle; the warp runs the
-                // test only if some lane can (then for every lane, as before).
+                // test only if some lane can (then for every lane).
                 const float4 f0 = __ldg(r);
                 // a skip test only: fused multiply-adds move pd by far less than the margin
                 const float pd = fabsf(__fmaf_rn(f0.x, p.x, __fmaf_rn(f0.y, p.y, __fmaf_rn(f0.z, p.z, -f0.w))));
-                const bool may = active && !(pd > dist + b.dist_margin);
-                if (__any_sync(0xffffffffu, may)) {
-                    if (counter) ++nt;
-                    if (active) {
-                        const float nd = point_tri_dist_rec(b, t, p);
-                        if (nd < dist) dist = nd;
+                if (__any_sync(full, !(pd > dist + b.dist_margin))) {
+                    ++nt;
+                    const float nd = point_tri_dist_rec(b, t, p);
+                    if (nd < dist) {
+                        dist = nd;
+                        lim = dist * dist;
                     }
                 }
             }
@@ -589,42 +647,41 @@ __device__ __forceinline__ float warp_distance(const BvhView& b, V3 p, float d0,
         if (sp == 0) break;
         cur = wstack_pop(s0, s1, sp);
     }
-    return dist;
+    return active ? dist : d0;
 }
 
 // bvh_any_hit for the active lanes' segments: a lane stops searching at its
 // first occluder hit (r < 1); the walk ends when no lane searches any more.
 __device__ __forceinline__ bool warp_any_hit(const BvhView& b, V3 o, V3 e, bool active, ErrFlag err)
 {
+    const unsigned full = 0xffffffffu;
     bool hit = false;
-    bool searching = active && b.n_tris > 0;
-    if (!__any_sync(0xffffffffu, searching)) return false;
-    const V3 d = e - o;
-    const V3 inv = inv_dir(d);
-    const V3 oinv = mk(o.x * inv.x, o.y * inv.y, o.z * inv.z);
+    if (b.n_tris <= 0 || !__any_sync(full, active)) return false;
+    const SlabPairs seg(inv_dir(e - o), o);
+    float tlimit = active ? 1.0f : -1.0f;
     int s0 = 0, s1 = 0, sp = 0;
     int cur = b.root;
     for (;;) {
         if (cur >= 0) {
-            const NodeBoxes nb = load_node(b, cur);
+            const NodePairs nd = load_pairs(b, cur);
+            bool hl, hr;
             float tl, tr;
-            const bool hl = searching && slab(nb.lmin, nb.lmax, oinv, inv, 1.0f, tl);
-            const bool hr = searching && slab(nb.rmin, nb.rmax, oinv, inv, 1.0f, tr);
-            const unsigned ml = __ballot_sync(0xffffffffu, hl), mr = __ballot_sync(0xffffffffu, hr);
+            seg.test(nd, tlimit, hl, hr, tl, tr);
+            const unsigned ml = __ballot_sync(full, hl), mr = __ballot_sync(full, hr);
             if (ml && mr) {
-                const bool lfirst = warp_left_first(hl, hr, tl <= tr);
-                wstack_push(s0, s1, sp, lfirst ? nb.r : nb.l, err);
-                cur = lfirst ? nb.l : nb.r;
+                const bool lfirst = warp_left_first(ml, mr, tl <= tr);
+                wstack_push(s0, s1, sp, lfirst ? nd.r : nd.l, err);
+                cur = lfirst ? nd.l : nd.r;
                 continue;
             }
-            if (ml) { cur = nb.l; continue; }
-            if (mr) { cur = nb.r; continue; }
-        } else if (searching) {
+            if (ml) { cur = nd.l; continue; }
+            if (mr) { cur = nd.r; continue; }
+        } else if (tlimit > 0.0f) {
             u32 meta;
             const float r = seg_leaf(b, o, e, ~cur, meta);
-            if ((meta & kOccluderBit) && r < 1.0f) { hit = true; searching = false; }
+            if ((meta & kOccluderBit) && r < 1.0f) { hit = true; tlimit = -1.0f; }
         }
-        if (sp == 0 || !__any_sync(0xffffffffu, searching)) break;
+        if (sp == 0 || !__any_sync(full, tlimit > 0.0f)) break;
         cur = wstack_pop(s0, s1, sp);
     }
     return hit;
@@ -635,30 +692,29 @@ __device__ __forceinline__ bool warp_any_hit(const BvhView& b, V3 o, V3 e, bool 
 // visiting order), each lane shrinking its own limit.
 __device__ __forceinline__ float warp_closest(const BvhView& b, V3 o, V3 e, bool active, ErrFlag err)
 {
+    const unsigned full = 0xffffffffu;
     float best = kNoHit;
     int bt = -1;
-    if (b.n_tris <= 0 || !__any_sync(0xffffffffu, active)) return best;
-    const V3 d = e - o;
-    const V3 inv = inv_dir(d);
-    const V3 oinv = mk(o.x * inv.x, o.y * inv.y, o.z * inv.z);
-    float tlimit = 1.0f;
+    if (b.n_tris <= 0 || !__any_sync(full, active)) return best;
+    const SlabPairs seg(inv_dir(e - o), o);
+    float tlimit = active ? 1.0f : -1.0f;
     int s0 = 0, s1 = 0, sp = 0;
     int cur = b.root;
     for (;;) {
         if (cur >= 0) {
-            const NodeBoxes nb = load_node(b, cur);
+            const NodePairs nd = load_pairs(b, cur);
+            bool hl, hr;
             float tl, tr;
-            const bool hl = active && slab(nb.lmin, nb.lmax, oinv, inv, tlimit, tl);
-            const bool hr = active && slab(nb.rmin, nb.rmax, oinv, inv, tlimit, tr);
-            const unsigned ml = __ballot_sync(0xffffffffu, hl), mr = __ballot_sync(0xffffffffu, hr);
+            seg.test(nd, tlimit, hl, hr, tl, tr);
+            const unsigned ml = __ballot_sync(full, hl), mr = __ballot_sync(full, hr);
             if (ml && mr) {
-                const bool lfirst = warp_left_first(hl, hr, tl <= tr);
-                wstack_push(s0, s1, sp, lfirst ? nb.r : nb.l, err);
-                cur = lfirst ? nb.l : nb.r;
+                const bool lfirst = warp_left_first(ml, mr, tl <= tr);
+                wstack_push(s0, s1, sp, lfirst ? nd.r : nd.l, err);
+                cur = lfirst ? nd.l : nd.r;
                 continue;
             }
-            if (ml) { cur = nb.l; continue; }
-            if (mr) { cur = nb.r; continue; }
+            if (ml) { cur = nd.l; continue; }
+            if (mr) { cur = nd.r; continue; }
         } else if (active) {
             const int t = ~cur;
             u32 meta;
@@ -689,21 +745,19 @@ __device__ __forceinline__ float warp_closest_inst(const BvhView& b, V3 o, V3 e,
         *local_out = bl;
         return best;
     }
-    const V3 d = e - o;
-    const V3 inv = inv_dir(d);
-    const V3 oinv = mk(o.x * inv.x, o.y * inv.y, o.z * inv.z);
-    float tlimit = 1.0f;
+    const SlabPairs seg(inv_dir(e - o), o);
+    float tlimit = active ? 1.0f : -1.0f;
     int s0 = 0, s1 = 0, sp = 0;
     int cur = b.root;
     for (;;) {
         if (cur >= 0) {
-            const NodeBoxes nb = load_node(b, cur);
+            const NodePairs nb = load_pairs(b, cur);
+            bool hl, hr;
             float tl, tr;
-            const bool hl = active && slab(nb.lmin, nb.lmax, oinv, inv, tlimit, tl);
-            const bool hr = active && slab(nb.rmin, nb.rmax, oinv, inv, tlimit, tr);
+            seg.test(nb, tlimit, hl, hr, tl, tr);
             const unsigned ml = __ballot_sync(0xffffffffu, hl), mr = __ballot_sync(0xffffffffu, hr);
             if (ml && mr) {
-                const bool lfirst = warp_left_first(hl, hr, tl <= tr);
+                const bool lfirst = warp_left_first(ml, mr, tl <= tr);
                 wstack_push(s0, s1, sp, lfirst ? nb.r : nb.l, err);
                 cur = lfirst ? nb.l : nb.r;
                 continue;

@@ -75,6 +75,17 @@ HD V2 normalized2(V2 a)
 }
 
 #ifdef __CUDACC__
+// Two floats in a 64-bit register pair: sm_100's packed arithmetic does both
+// halves with one instruction, each rounded like the scalar one. And its
+// three-operand min and max.
+typedef unsigned long long F2;
+__device__ __forceinline__ F2 f2_make(float a, float b) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void f2_get(F2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ float max3(float a, float b, float c) { float r; asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
+__device__ __forceinline__ float min3(float a, float b, float c) { float r; asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
+
 HD V3 ld3(const float4& f) { return mk(f.x, f.y, f.z); }
 HD float4 st4(V3 v, float w) { return make_float4(v.x, v.y, v.z, w); }
 #endif
