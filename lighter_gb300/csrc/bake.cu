@@ -57,26 +57,6 @@ void ck(cudaError_t e, const char* what, int line)
 constexpr int kThreads = 256;
 constexpr u32 kNoLoc = 0xffffffffu;
 
-// f(begin, end) over [0, n) in contiguous chunks on up to 16 host threads
-// (one thread below 2 * grain items).
-template <class F>
-void parallel_for(size_t n, size_t grain, F&& f)
-{
-    size_t nt = std::min<size_t>({(size_t) 16, (size_t) std::max(1u, std::thread::hardware_concurrency()),
-                                  (n + grain - 1) / std::max<size_t>(grain, 1)});
-    if (nt <= 1) {
-        if (n) f((size_t) 0, n);
-        return;
-    }
-    const size_t chunk = (n + nt - 1) / nt;
-    std::vector<std::thread> th;
-    for (size_t t = 0; t < nt; ++t) {
-        const size_t b = t * chunk, e = std::min(n, b + chunk);
-        if (b < e) th.emplace_back([&f, b, e]() { f(b, e); });
-    }
-    for (auto& x : th) x.join();
-}
-
 // f(i) for i in [0, n) on up to 16 host threads taking items one at a time;
 // the first exception is rethrown after all threads end.
 template <class F>
@@ -122,6 +102,17 @@ struct DLight {
     int ns, soff;   // LTRG_SHADOW_SAMPLED: shadow samples of the light at lsmp[soff .. soff + ns)
 };
 
+// A vertex of an instance: world position, world normal, first texture
+// coordinates, lightmap-space position.
+constexpr int kVert = 10;
+
+// The triangles of one part of one instance among all raster records.
+struct RasterSeg {
+    u32 first;        // its first record
+    u32 inst, part;
+    u32 voff, ioff;   // its first vertex and its first index
+};
+
 // Raster record of one triangle (RasterizeInstance, lighter.cpp:32-66):
 //   [0..5] lightmap-space p1,p2,p3  [6..14] world pos  [15..23] world normal
 //   [24..29] uv1  [30] part  [31] sample area
@@ -140,6 +131,76 @@ __device__ __forceinline__ void warp_add(unsigned long long* dst, unsigned long 
 }
 
 // ----------------------------------------------------------------------------- raster
+
+// Raster records of all triangles, in instance / part / triangle order, and their
+// per-pass texel boxes (x, y, width, height) and box areas (RasterizeInstance and the
+// set-up of RasterizeTriangle2D_x2_ex, lighter.cpp:32-66, lighter_math.cpp:251-267).
+// One thread per triangle; bound by its 128-byte record's write. The host loops this
+// replaced, with the upload of their 200 bytes per triangle instead of the 40-byte vertices,
+// took 16 of the terrain bake's 24 ms before its first trace.
+__global__ void k_raster_setup(u32 n, const RasterSeg* __restrict__ segs, int n_segs, const float* __restrict__ verts,
+                               const u32* __restrict__ idx, const u32* __restrict__ inst_w, const u32* __restrict__ inst_h,
+                               float margin0, float margin1, float* __restrict__ rt, u32* __restrict__ rinst,
+                               int4* __restrict__ bbox0, int4* __restrict__ bbox1, unsigned long long* __restrict__ area0,
+                               unsigned long long* __restrict__ area1)
+{
+    const u32 k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k > n) return;
+    if (k == n) {   // the scans' last entry
+        area0[n] = area1[n] = 0;
+        return;
+    }
+    int lo = 0, hi = n_segs - 1;   // the last part with first <= k (empty parts precede the one that starts there too)
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (segs[mid].first <= k) lo = mid; else hi = mid - 1;
+    }
+    const RasterSeg g = segs[lo];
+    const u32 t = g.ioff + (k - g.first) * 3;
+    const float* v[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) v[c] = verts + (size_t) kVert * (g.voff + idx[t + c]);
+    V3 P[3], N[3];
+    V2 T[3], L[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        P[c] = mk(v[c][0], v[c][1], v[c][2]);
+        N[c] = mk(v[c][3], v[c][4], v[c][5]);
+        T[c] = mk2(v[c][6], v[c][7]);
+        L[c] = mk2(v[c][8], v[c][9]);
+    }
+    const float lmarea = tri_area2(L[0], L[1], L[2]), coarea = tri_area3(P[0], P[1], P[2]);
+    const float sa = lmarea > 0 ? coarea / lmarea : 0;
+    float4* o = reinterpret_cast<float4*>(rt + (size_t) k * kRT);
+    o[0] = make_float4(L[0].x, L[0].y, L[1].x, L[1].y);
+    o[1] = make_float4(L[2].x, L[2].y, P[0].x, P[0].y);
+    o[2] = make_float4(P[0].z, P[1].x, P[1].y, P[1].z);
+    o[3] = make_float4(P[2].x, P[2].y, P[2].z, N[0].x);
+    o[4] = make_float4(N[0].y, N[0].z, N[1].x, N[1].y);
+    o[5] = make_float4(N[1].z, N[2].x, N[2].y, N[2].z);
+    o[6] = make_float4(T[0].x, T[0].y, T[1].x, T[1].y);
+    o[7] = make_float4(T[2].x, T[2].y, (float) g.part, sa);
+    rinst[k] = g.inst;
+    const int w = (int) inst_w[g.inst], h = (int) inst_h[g.inst];
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+        const float mg = pass ? margin1 : margin0;
+        int maxX = (int) (fmax_(L[0].x, fmax_(L[1].x, L[2].x)) + mg);
+        int minX = (int) (fmin_(L[0].x, fmin_(L[1].x, L[2].x)) - mg);
+        int maxY = (int) (fmax_(L[0].y, fmax_(L[1].y, L[2].y)) + mg);
+        int minY = (int) (fmin_(L[0].y, fmin_(L[1].y, L[2].y)) - mg);
+        bool empty = maxX < 0 || minX >= w || maxY < 0 || minY >= h;
+        if (minX < 0) minX = 0;
+        if (maxX >= w) maxX = w - 1;
+        if (minY < 0) minY = 0;
+        if (maxY >= h) maxY = h - 1;
+        if (cross2(L[1] - L[0], L[2] - L[0]) == 0) empty = true;
+        if (maxX < minX || maxY < minY) empty = true;
+        const int4 b = empty ? make_int4(0, 0, 1, 0) : make_int4(minX, minY, maxX - minX + 1, maxY - minY + 1);
+        (pass ? bbox1 : bbox0)[k] = b;
+        (pass ? area1 : area0)[k] = (unsigned long long) b.z * (unsigned long long) b.w;
+    }
+}
 
 // Texel (x, y) is covered by the triangle when it lies within `margin` of all
 // three edges for either winding (lighter_math.cpp:281-300).
@@ -160,9 +221,10 @@ __device__ __forceinline__ bool raster_inside(const float* r, int x, int y, floa
 
 __global__ void k_raster_mark(int pass, float margin, const float* __restrict__ rt, const u32* __restrict__ rinst,
                               const int4* __restrict__ bbox, const unsigned long long* __restrict__ off, int ntri,
-                              unsigned long long nwork, const unsigned long long* __restrict__ tex_off,
-                              const u32* __restrict__ inst_w, u32* __restrict__ keys)
+                              const unsigned long long* __restrict__ tex_off, const u32* __restrict__ inst_w,
+                              u32* __restrict__ keys)
 {
+    const unsigned long long nwork = off[ntri];   // texels of all boxes
     for (unsigned long long w = blockIdx.x * (unsigned long long) blockDim.x + threadIdx.x; w < nwork;
          w += (unsigned long long) gridDim.x * blockDim.x) {
         int lo = 0, hi = ntri - 1;   // largest k with off[k] <= w
@@ -1772,12 +1834,13 @@ void check_abort(ltr_Scene* s)
 // Row-vector transform and normal matrix of Job_PreXForm_Inner (lighter.cpp:292-341,
 // lighter_int.hpp:511-545). The 2x2 minors keep the operand order of the
 // 4x4 cofactor expansion of Mat4::InvertTo applied to [R 0; 0 1].
-void prexform(ltr_Scene* S, HostInst* mi)
+// `vert` receives the instance's vertices, kVert floats each.
+void prexform(ltr_Scene* S, HostInst* mi, float* vert)
 {
     const float* m = mi->matrix;   // m[r*4+c]
     ltr_Mesh* me = mi->mesh;
     size_t nv = me->pos.size();
-    mi->vpos.resize(nv); mi->vnrm.resize(nv); mi->vtex.resize(nv); mi->ltex.resize(nv);
+    mi->vpos.resize(nv);
     const float a0 = m[0], a1 = m[1], a2 = m[2], a4 = m[4], a5 = m[5], a6 = m[6], a8 = m[8], a9 = m[9], a10 = m[10];
     float c[16] = {0};
     c[0] = a5 * a10 - a9 * a6;
@@ -1806,9 +1869,12 @@ void prexform(ltr_Scene* S, HostInst* mi)
                          v.x * m[1] + v.y * m[5] + v.z * m[9] + m[13] * 1.0f,
                          v.x * m[2] + v.y * m[6] + v.z * m[10] + m[14] * 1.0f);
         V3 n = me->nrm[i];
-        mi->vnrm[i] = normalized(mk(n.x * inv[0] + n.y * inv[1] + n.z * inv[2] + inv[3] * 0.0f,
+        const V3 wn = normalized(mk(n.x * inv[0] + n.y * inv[1] + n.z * inv[2] + inv[3] * 0.0f,
                                     n.x * inv[4] + n.y * inv[5] + n.z * inv[6] + inv[7] * 0.0f,
                                     n.x * inv[8] + n.y * inv[9] + n.z * inv[10] + inv[11] * 0.0f));
+        float* o = vert + (size_t) kVert * i;
+        o[0] = mi->vpos[i].x; o[1] = mi->vpos[i].y; o[2] = mi->vpos[i].z;
+        o[3] = wn.x; o[4] = wn.y; o[5] = wn.z;
     }
     float area = 0.0f;
     for (const HostPart& p : me->parts) {
@@ -1826,8 +1892,9 @@ void prexform(ltr_Scene* S, HostInst* mi)
     mi->h = size[1];
     float fw = (float) mi->w, fh = (float) mi->h;
     for (size_t i = 0; i < nv; ++i) {
-        mi->vtex[i] = me->tex1[i];
-        mi->ltex[i] = mk2(me->tex2[i].x * fw - 0.5f, me->tex2[i].y * fh - 0.5f);
+        float* o = vert + (size_t) kVert * i;
+        o[6] = me->tex1[i].x; o[7] = me->tex1[i].y;
+        o[8] = me->tex2[i].x * fw - 0.5f; o[9] = me->tex2[i].y * fh - 0.5f;
     }
 }
 
@@ -2315,7 +2382,11 @@ void run_bake(ltr_Scene* S)
     S->stage = "transforming spatial data";
     const int n_inst = (int) S->insts.size();
     // instances in parallel: the reference too calls size_fn from its pool threads
-    parallel_items(n_inst - 1, [&](int k) { prexform(S, S->insts[k + 1]); });
+    std::vector<size_t> vert_off(n_inst + 1, 0);   // each instance's first vertex
+    for (int i = 0; i < n_inst; ++i)
+        vert_off[i + 1] = vert_off[i] + (S->insts[i]->container ? 0 : S->insts[i]->mesh->pos.size());
+    std::unique_ptr<float[]> verts(new float[kVert * std::max<size_t>(vert_off[n_inst], 1)]);
+    parallel_items(n_inst - 1, [&](int k) { prexform(S, S->insts[k + 1], verts.get() + kVert * vert_off[k + 1]); });
     check_abort(S);
 
     // ---- host: triangle soup of shadow parts (Job_ColInfo) + instance boxes
@@ -2583,16 +2654,15 @@ void run_bake(ltr_Scene* S)
         }
     }
 
-    // Raster records and per-pass bounding boxes (RasterizeInstance /
-    // RasterizeTriangle2D_x2_ex set-up, lighter.cpp:32-66, lighter_math.cpp:251-267).
+    // Raster inputs: which records each part's triangles are, the vertices, and the
+    // meshes' indices (once per mesh).
     TRACE("light culling done");
-    // Raster records (kRT floats per triangle, in instance / part / triangle
-    // order) and their bounding boxes, filled in parallel over the triangles.
     std::vector<unsigned long long> tex_off(n_inst + 1, 0);
     std::vector<u32> inst_w(n_inst, 0), inst_h(n_inst, 0);
     unsigned long long ntex = 0;
-    struct Seg { int inst; u32 part; size_t first; };   // a part's triangles start at record `first`
-    std::vector<Seg> segs;
+    std::vector<RasterSeg> segs;
+    std::vector<u32> indices;
+    std::unordered_map<const ltr_Mesh*, u32> index_off;
     size_t n_rec = 0;
     for (int i = 0; i < n_inst; ++i) {
         HostInst* mi = S->insts[i];
@@ -2601,78 +2671,24 @@ void run_bake(ltr_Scene* S)
         inst_w[i] = mi->w;
         inst_h[i] = mi->h;
         ntex += (unsigned long long) mi->w * mi->h;
+        auto at = index_off.find(mi->mesh);
+        if (at == index_off.end()) {
+            at = index_off.emplace(mi->mesh, (u32) indices.size()).first;
+            indices.insert(indices.end(), mi->mesh->idx.begin(), mi->mesh->idx.end());
+        }
         for (u32 part = 0; part < mi->mesh->parts.size(); ++part) {
-            segs.push_back(Seg{i, part, n_rec});
-            n_rec += mi->mesh->parts[part].icount / 3;
+            const HostPart& p = mi->mesh->parts[part];
+            segs.push_back(RasterSeg{(u32) n_rec, (u32) i, part, (u32) vert_off[i] + p.voff, at->second + p.ioff});
+            n_rec += p.icount / 3;
         }
+        if (n_rec >= (1u << 30) - 1u) throw std::runtime_error("too many triangles for the raster keys");
+        if (indices.size() > 0xffffffffull || vert_off[n_inst] > 0xffffffffull)
+            throw std::runtime_error("too many vertices or indices for one bake");
     }
-    std::vector<float> rt(n_rec * kRT);
-    std::vector<u32> rinst(n_rec);
-    parallel_for(n_rec, 4096, [&](size_t k0, size_t k1) {
-        size_t si = std::upper_bound(segs.begin(), segs.end(), k0, [](size_t k, const Seg& g) { return k < g.first; }) -
-                    segs.begin() - 1;
-        for (size_t k = k0; k < k1; ++k) {
-            while (si + 1 < segs.size() && segs[si + 1].first <= k) ++si;
-            const Seg& g = segs[si];
-            HostInst* mi = S->insts[g.inst];
-            const HostPart& p = mi->mesh->parts[g.part];
-            const u32* ib = &mi->mesh->idx[p.ioff];
-            const u32 t = (u32) (k - g.first) * 3;
-            u32 i1 = p.voff + ib[t], i2 = p.voff + ib[t + 1], i3 = p.voff + ib[t + 2];
-            float lmarea = tri_area2(mi->ltex[i1], mi->ltex[i2], mi->ltex[i3]);
-            float coarea = tri_area3(mi->vpos[i1], mi->vpos[i2], mi->vpos[i3]);
-            float sa = lmarea > 0 ? coarea / lmarea : 0;
-            const u32 ids[3] = {i1, i2, i3};
-            float* o = &rt[k * kRT];
-            for (u32 v : ids) { *o++ = mi->ltex[v].x; *o++ = mi->ltex[v].y; }
-            for (u32 v : ids) { *o++ = mi->vpos[v].x; *o++ = mi->vpos[v].y; *o++ = mi->vpos[v].z; }
-            for (u32 v : ids) { *o++ = mi->vnrm[v].x; *o++ = mi->vnrm[v].y; *o++ = mi->vnrm[v].z; }
-            for (u32 v : ids) { *o++ = mi->vtex[v].x; *o++ = mi->vtex[v].y; }
-            *o++ = (float) g.part;
-            *o++ = sa;
-            rinst[k] = (u32) g.inst;
-        }
-    });
     tex_off[n_inst] = ntex;
-    TRACE("raster records done");
-    const int n_rt = (int) rinst.size();
-    if (n_rt >= (1 << 30) - 1) throw std::runtime_error("too many triangles for the raster keys");
+    const int n_rt = (int) n_rec;
     S->stats.texels = ntex;
-    std::vector<int4> bbox[2];
-    std::vector<unsigned long long> woff[2];
     const float margins[2] = {0.5f + kSmall, 0.0f};
-    for (int pass = 0; pass < 2; ++pass) {
-        bbox[pass].resize(n_rt);
-        woff[pass].resize(n_rt + 1);
-        const float mg = margins[pass];
-        parallel_for((size_t) n_rt, 4096, [&](size_t k0, size_t k1) {
-            for (size_t k = k0; k < k1; ++k) {
-                const float* r = &rt[k * kRT];
-                u32 inst = rinst[k];
-                int w = (int) inst_w[inst], h = (int) inst_h[inst];
-                int maxX = (int) (fmax_(r[0], fmax_(r[2], r[4])) + mg);
-                int minX = (int) (fmin_(r[0], fmin_(r[2], r[4])) - mg);
-                int maxY = (int) (fmax_(r[1], fmax_(r[3], r[5])) + mg);
-                int minY = (int) (fmin_(r[1], fmin_(r[3], r[5])) - mg);
-                bool empty = maxX < 0 || minX >= w || maxY < 0 || minY >= h;
-                if (minX < 0) minX = 0;
-                if (maxX >= w) maxX = w - 1;
-                if (minY < 0) minY = 0;
-                if (maxY >= h) maxY = h - 1;
-                V2 p1 = mk2(r[0], r[1]), p2 = mk2(r[2], r[3]), p3 = mk2(r[4], r[5]);
-                if (cross2(p2 - p1, p3 - p1) == 0) empty = true;
-                if (maxX < minX || maxY < minY) empty = true;
-                bbox[pass][k] = empty ? make_int4(0, 0, 1, 0) : make_int4(minX, minY, maxX - minX + 1, maxY - minY + 1);
-            }
-        });
-        unsigned long long acc = 0;   // work offsets (texels covered by each box), in order
-        for (int k = 0; k < n_rt; ++k) {
-            woff[pass][k] = acc;
-            const int4 b = bbox[pass][k];
-            if (b.w > 0) acc += (unsigned long long) b.z * (unsigned long long) b.w;
-        }
-        woff[pass][n_rt] = acc;
-    }
 
     TRACE("host records done");
     // ---- upload
@@ -2680,14 +2696,17 @@ void run_bake(ltr_Scene* S)
     const u32 n_probe = (u32) S->samples.size();
     unsigned char* d_lit = A.upload(lit);
     DLight* d_lights = A.upload(dl);
-    float* d_rt = A.upload(rt);
-    u32* d_rinst = A.upload(rinst);
     unsigned long long* d_tex_off = A.upload(tex_off);
     u32* d_inst_w = A.upload(inst_w);
     u32* d_inst_h = A.upload(inst_h);
-    int4* d_bbox[2];
-    unsigned long long* d_woff[2];
-    for (int p = 0; p < 2; ++p) { d_bbox[p] = A.upload(bbox[p]); d_woff[p] = A.upload(woff[p]); }
+    RasterSeg* d_segs = A.upload(segs);
+    u32* d_indices = A.upload(indices);
+    float* d_verts = A.alloc<float>(kVert * vert_off[n_inst]);
+    if (vert_off[n_inst]) {
+        const size_t vb = kVert * vert_off[n_inst] * sizeof(float);
+        CK(cudaMemcpyAsync(d_verts, verts.get(), vb, cudaMemcpyHostToDevice, st));
+        note_h2d(vb);
+    }
     // one error word per stage kernel: 0 fixup, 1 direct, 2 radiosity, 3 AO
     u32* d_err = A.zeros<u32>(8);
     Counters* d_cnt = A.zeros<Counters>(1);
@@ -2696,45 +2715,34 @@ void run_bake(ltr_Scene* S)
     check_abort(S);
 
     TRACE("upload issued");
-    // ---- BVH (joined)
-    if (bvh_thread.joinable()) bvh_thread.join();
-    if (bvh_error) std::rethrow_exception(bvh_error);
-    host_counters().launches += bvh_counts.launches;
-    host_counters().h2d += bvh_counts.h2d;
-    host_counters().d2h += bvh_counts.d2h;
-    if (bside.st) CK(cudaStreamWaitEvent(st, bside.e1, 0));
-    S->stats.reserved[0] = (uint64_t) bin.n;   // leaf references
-    BvhView bv = bvh.view();
-    bv.watertight = S->opt.intersect_mode == LTRG_ISECT_WATERTIGHT ? 1 : 0;
-    {
-        // rounding bound of the distance test against the plane distance: a few
-        // single-precision dot products over coordinates up to the scene's largest
-        float mx = 0.0f;
-        for (float v : tri_xyz) mx = fmaxf(mx, fabsf(v));
-        bv.dist_margin = std::isfinite(mx) ? 4e-6f * (1.0f + mx) : INFINITY;
-    }
-    cudaEvent_t e_bvh = clock.mark();
-    // LTRG_VALIDATE=1: re-check the BVH topology after every stage
-    const bool validate = getenv("LTRG_VALIDATE") && getenv("LTRG_VALIDATE")[0] == '1';
-    auto checkpoint = [&](const char* where) {
-        if (!validate) return;
-        CK(cudaStreamSynchronize(st));
-        std::string e = bvh_validate(bvh, st);
-        if (!e.empty()) throw std::runtime_error(std::string("BVH corrupted after ") + where + ": " + e);
-    };
-    checkpoint("build");
-
-    // ---- samples (Job_Samples)
-    TRACE("bvh issued");
+    // ---- samples (Job_Samples): which texels the triangles cover (no BVH needed yet)
     S->stage = "generating samples";
+    cudaEvent_t e_ras0 = clock.mark();
+    float* d_rt = A.alloc<float>((size_t) n_rt * kRT);
+    u32* d_rinst = A.alloc<u32>(n_rt);
     u32* d_keys = A.zeros<u32>(ntex);
-    for (int pass = 0; pass < 2; ++pass) {
-        unsigned long long nw = woff[pass][n_rt];
-        if (nw == 0) continue;
-        k_raster_mark<<<blocks_for(nw), kThreads, 0, st>>>(pass, margins[pass], d_rt, d_rinst, d_bbox[pass],
-                                                           d_woff[pass], n_rt, nw, d_tex_off, d_inst_w, d_keys); note_launch();
+    if (n_rt && ntex) {
+        int4* d_bbox[2];
+        unsigned long long *d_area[2], *d_woff[2];
+        for (int p = 0; p < 2; ++p) {
+            d_bbox[p] = A.alloc<int4>(n_rt);
+            d_area[p] = A.alloc<unsigned long long>(n_rt + 1);
+            d_woff[p] = A.alloc<unsigned long long>(n_rt + 1);
+        }
+        k_raster_setup<<<(n_rt + 1 + kThreads - 1) / kThreads, kThreads, 0, st>>>(
+            (u32) n_rt, d_segs, (int) segs.size(), d_verts, d_indices, d_inst_w, d_inst_h, margins[0], margins[1], d_rt,
+            d_rinst, d_bbox[0], d_bbox[1], d_area[0], d_area[1]); note_launch();
         CK(cudaGetLastError());
-        checkpoint("raster mark");
+        size_t tb = 0;
+        CK(cub::DeviceScan::ExclusiveSum(nullptr, tb, d_area[0], d_woff[0], (int64_t) (n_rt + 1), st));
+        void* tmp = A.alloc<char>(tb);
+        for (int pass = 0; pass < 2; ++pass) {
+            CK(cub::DeviceScan::ExclusiveSum(tmp, tb, d_area[pass], d_woff[pass], (int64_t) (n_rt + 1), st));
+            // the boxes' texels stay on the device; about twice the lightmaps' are usual
+            k_raster_mark<<<blocks_for(2 * ntex), kThreads, 0, st>>>(pass, margins[pass], d_rt, d_rinst, d_bbox[pass],
+                                                                     d_woff[pass], n_rt, d_tex_off, d_inst_w, d_keys); note_launch();
+            CK(cudaGetLastError());
+        }
     }
     float4* d_R1 = A.alloc<float4>(ntex);
     float4* d_R2 = A.alloc<float4>(ntex);
@@ -2746,7 +2754,6 @@ void run_bake(ltr_Scene* S)
         k_raster_resolve<<<blocks_for(ntex), kThreads, 0, st>>>(ntex, d_keys, d_rt, d_rinst, d_tex_off, d_inst_w,
                                                                 d_R1, d_R2, d_R3, d_flags); note_launch();
         CK(cudaGetLastError());
-        checkpoint("raster resolve");
     }
     {
         size_t tb = 0;
@@ -2834,7 +2841,6 @@ void run_bake(ltr_Scene* S)
         k_compact<<<blocks_for(ntex), kThreads, 0, st>>>(ntex, d_flags, d_scan, d_R1, d_R2, d_R3, d_tex_off, n_inst,
                                                          n_probe, d_spos, d_snrm, d_srad, d_sloc, d_sinst); note_launch();
         CK(cudaGetLastError());
-        checkpoint("compaction");
     }
     // trace orders of the two trace stages (null: sample order)
     const u32* d_order_dir = nullptr;
@@ -2870,6 +2876,36 @@ void run_bake(ltr_Scene* S)
         d_order_dir = order_for(tu.direct_order);
         d_order_ao = order_for(tu.ao_order);
     }
+    cudaEvent_t e_ras1 = clock.mark();
+    // ---- BVH (joined)
+    if (bvh_thread.joinable()) bvh_thread.join();
+    if (bvh_error) std::rethrow_exception(bvh_error);
+    host_counters().launches += bvh_counts.launches;
+    host_counters().h2d += bvh_counts.h2d;
+    host_counters().d2h += bvh_counts.d2h;
+    if (bside.st) CK(cudaStreamWaitEvent(st, bside.e1, 0));
+    S->stats.reserved[0] = (uint64_t) bin.n;   // leaf references
+    BvhView bv = bvh.view();
+    bv.watertight = S->opt.intersect_mode == LTRG_ISECT_WATERTIGHT ? 1 : 0;
+    {
+        // rounding bound of the distance test against the plane distance: a few
+        // single-precision dot products over coordinates up to the scene's largest
+        float mx = 0.0f;
+        for (float v : tri_xyz) mx = fmaxf(mx, fabsf(v));
+        bv.dist_margin = std::isfinite(mx) ? 4e-6f * (1.0f + mx) : INFINITY;
+    }
+    // LTRG_VALIDATE=1: re-check the BVH topology after every stage
+    const bool validate = getenv("LTRG_VALIDATE") && getenv("LTRG_VALIDATE")[0] == '1';
+    auto checkpoint = [&](const char* where) {
+        if (!validate) return;
+        CK(cudaStreamSynchronize(st));
+        std::string e = bvh_validate(bvh, st);
+        if (!e.empty()) throw std::runtime_error(std::string("BVH corrupted after ") + where + ": " + e);
+    };
+    checkpoint("build");
+
+    TRACE("bvh issued");
+    cudaEvent_t e_fix0 = clock.mark();
     reftree_thread.join();
     TRACE("reference trees joined");
     if (reftree_error) std::rethrow_exception(reftree_error);
@@ -3500,7 +3536,7 @@ void run_bake(ltr_Scene* S)
     TRACE("outputs assembled");
     S->stats.ms_upload = StageClock::ms(e_up0, e_up1);
     S->stats.ms_bvh = StageClock::ms(bside.e0, bside.e1);
-    S->stats.ms_samples = StageClock::ms(e_bvh, e_samples);
+    S->stats.ms_samples = StageClock::ms(e_ras0, e_ras1) + StageClock::ms(e_fix0, e_samples);
     S->stats.ms_direct = StageClock::ms(e_samples, e_direct);
     S->stats.ms_ao = StageClock::ms(e_ao0, e_ao1);
     S->stats.ms_direct_trace = e_dtr0 ? StageClock::ms(e_dtr0, e_dtr1) : 0.0;

@@ -26,9 +26,7 @@ struct HostInst {
     bool shadow = false;
     bool container = false;
     u32 w = 128, h = 128;      // lightmap size (lighter.cpp:1277-1278 default)
-    // filled by the bake (world space, lightmap texel space)
-    std::vector<V3> vpos, vnrm;
-    std::vector<V2> vtex, ltex;
+    std::vector<V3> vpos;      // filled by the bake: world-space positions
 };
 
 struct HostLight {
