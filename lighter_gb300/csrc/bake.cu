@@ -323,6 +323,10 @@ struct FixupArgs {
     float4* spos;
     const float4* snrm;
     const float4* srad;
+    const u32* slivers;        // nonzero when some triangle has an unbounded tri_box
+    const u32* order;          // samples in k_fix_quick's order (null: as they are)
+    u32* list;                 // the samples that k_fix_quick leaves to k_fixup (null: all), and their number
+    u32* n_list;
 };
 
 // Concave-edge push of TriTree::OffsetSample (lighter_math.cpp:991-1044) for
@@ -352,7 +356,7 @@ __device__ __forceinline__ bool offset_candidate(V3 P1, V3 P2, V3 P3, V3 P, V3 N
 // Boxes of the concave-edge pass's triangles, for its exact rejection test: the
 // box of a well-shaped triangle (height at least 1% of its longest edge); an
 // unbounded box for a thinner one, which the test then never rejects.
-__global__ void k_tri_boxes(const float* __restrict__ tri_xyz, u32 n, float4* __restrict__ box)
+__global__ void k_tri_boxes(const float* __restrict__ tri_xyz, u32 n, float4* __restrict__ box, u32* slivers)
 {
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -366,19 +370,26 @@ __global__ void k_tri_boxes(const float* __restrict__ tri_xyz, u32 n, float4* __
     } else {
         box[2 * i] = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.0f);
         box[2 * i + 1] = make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
+        *slivers = 1u;
     }
 }
 
+// dist plus a margin (1 mm + 1e-5 of P's largest coordinate) far above the rounding
+// of point_tri_dist on a well-shaped triangle: one farther than that from P is
+// not found closer than dist.
+__device__ __forceinline__ float fixup_reach(V3 P, float dist)
+{
+    const float scale = fmaxf(fabsf(P.x), fmaxf(fabsf(P.y), fabsf(P.z)));
+    return dist * 1.0001f + 1e-3f + 1e-5f * scale;
+}
+
 // Whether the concave-edge push of a triangle with box (bmn, bmx) surely does
-// nothing at P: the box lies more than r beyond P along an axis, r being dist
-// plus a margin (1 mm + 1e-5 of P's largest coordinate) far above the rounding
-// of point_tri_dist on a well-shaped triangle. The exact distance is at least
+// nothing at P: the box lies more than r (fixup_reach) beyond P along an axis. The exact distance is at least
 // the box's separation, the computed one within rounding of it, so it is not
 // below dist and offset_candidate would return at its first test.
 __device__ __forceinline__ bool fixup_rejects(float4 bmn, float4 bmx, V3 P, float dist)
 {
-    const float scale = fmaxf(fabsf(P.x), fmaxf(fabsf(P.y), fabsf(P.z)));
-    const float r = dist * 1.0001f + 1e-3f + 1e-5f * scale;
+    const float r = fixup_reach(P, dist);
     return P.x + r < bmn.x || P.x - r > bmx.x || P.y + r < bmn.y || P.y - r > bmx.y || P.z + r < bmn.z ||
            P.z - r > bmx.z;
 }
@@ -458,12 +469,108 @@ __device__ __forceinline__ void fixup_instance_warp(const FixupArgs& a, int k, b
     }
 }
 
+// Pushes a sample in front of overlapping faces (lighter.cpp:449-465); the
+// reference's BSP query is replaced by the closest hit over occluders. Each lane
+// walks alone: a walk shared by the warp also tests triangles whose boxes the lane's
+// own segment misses, and where many meet at one point (the foot of a sphere on the
+// ground) that changes which of the equally close ones is taken.
+__device__ __forceinline__ void fixup_overlap(const FixupArgs& a, V3& P, V3 N)
+{
+    if (a.max_correct_dist == 0.0f) return;
+    int left = 100;
+    float md = a.max_correct_dist;
+    V3 PEnd = P + N * md;
+    while (md > kSmall && left-- > 0) {
+        V3 dn = normalized(PEnd - P);
+        V3 mA = P + dn * kSmall, mB = PEnd - dn * kSmall;
+        int ht = -1;
+        float q = bvh_closest(a.bvh, mA, mB, a.err, &ht);
+        V3 hn = mk(0, 0, 0);
+        if (ht >= 0) {
+            V3 P1, P2, P3; u32 meta, local;
+            load_tri(a.bvh, ht, P1, P2, P3, meta, local);
+            hn = tri_normal_rev(P1, P2, P3);
+        }
+        if (-dot(hn, N) < a.corr_min_dot) break;
+        if (q < kSmall) q = kSmall;
+        P = P * (1.0f - q) + PEnd * q;
+        md *= (1.0f - q);
+    }
+}
+
 constexpr int kFixupThreads = 128;
+
+// The samples that no triangle's concave-edge push can apply to, whatever the order
+// of the reference-shaped trees, found by the scene BVH: a sample starts at P, and
+// as long as every triangle fails offset_candidate there, none ever moves it. Those
+// samples (nearly all) go straight to the overlap correction; the others are
+// listed for k_fixup, which walks the trees. Neither reads the trees, so this runs while
+// the host still builds them. A scene with slivers (see k_tri_boxes), whose computed
+// distances bound nothing, lists every sample.
+__global__ void __launch_bounds__(kFixupThreads) k_fix_quick(FixupArgs a)
+{
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const u32 rank = blockIdx.x * blockDim.x + threadIdx.x;
+    if (!__any_sync(full, rank < a.n_samples)) return;
+    u32 s = 0;
+    if (rank < a.n_samples) s = a.order ? a.order[rank] : rank;
+    const bool active = rank < a.n_samples && s >= a.n_probe;
+    V3 P = mk(0, 0, 0), N = P;
+    float dist = 0.0f;
+    if (active) {
+        P = ld3(a.spos[s]);
+        N = ld3(a.snrm[s]);
+        dist = sqrtf(a.srad[s].w);
+    }
+    bool listed = active && *a.slivers != 0;
+    if (__any_sync(full, active && !listed)) {
+        const float r = fixup_reach(P, dist);
+        float r2 = active && !listed ? r * r : -1.0f;
+        warp_walk_near(a.bvh, P, r2, a.err, [&](int t) {
+            // TPN of offset_candidate is the record's normal (the operands of its cross product
+            // exchanged and negated: the same roundings)
+            const float4 f0 = __ldg(a.bvh.drec + 8 * (size_t) t);
+            const bool steep = r2 >= 0.0f && fabsf(dot(mk(f0.x, f0.y, f0.z), N)) < 0.95f;
+            if (!__any_sync(full, steep)) return true;
+            if (steep) {
+                V3 P1, P2, P3, qo, qe;
+                u32 meta, local;
+                load_tri(a.bvh, t, P1, P2, P3, meta, local);
+                if (offset_candidate(P1, P2, P3, P, N, dist, qo, qe)) {
+                    listed = true;
+                    r2 = -1.0f;
+                }
+            }
+            return __any_sync(full, r2 >= 0.0f) != 0;
+        });
+    }
+    const unsigned ml = __ballot_sync(full, listed);
+    if (ml) {
+        u32 at = 0;
+        if (lane == 0) at = atomicAdd(a.n_list, (u32) __popc(ml));
+        at = __shfl_sync(full, at, 0);
+        if (listed) a.list[at + __popc(ml & ((1u << lane) - 1u))] = s;
+    }
+    if (active && !listed) {
+        fixup_overlap(a, P, N);
+        a.spos[s] = st4(P, 0.0f);
+    }
+}
+
+// Samples from which k_fix_quick pays. Below it a bake's GPU is not full, texels
+// are coarse next to the objects (so most samples near any are listed), and the two
+// kernels run one after the other (a 327k-sample level 1.4 -> 2.1 ms). Above: the
+// benchmark level's 2.4M samples 3.25 -> 1.08 + 1.7 ms, of which the first overlaps the
+// host's tree build, the terrain's 3.9M 9 -> 2.1 + 2.2 ms.
+constexpr u32 kFixQuickMin = 1u << 20;
+
 constexpr int kFixupCand = 256;   // candidate instances listed per warp
 
-// The concave-edge pass tests every instance's tree, in instance order
+// The concave-edge pass and the overlap correction of the listed samples (no list: of all).
+// The pass tests every instance's tree, in instance order
 // (lighter.cpp:445-446); an instance whose root box misses the query box
-// leaves P unchanged. A warp (32 consecutive samples) first lists, in order,
+// leaves P unchanged. A warp (32 samples of the list) first lists, in order,
 // the instances whose root box meets the union of its query boxes grown by
 // G > M, and its lanes walk only those. A lane whose P has moved more than M
 // (per axis) from its start could meet an unlisted instance, so once any lane
@@ -474,87 +581,69 @@ __global__ void __launch_bounds__(kFixupThreads) k_fixup(FixupArgs a)
     __shared__ int cand[kFixupThreads / 32][kFixupCand];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const u32 s = a.n_probe + blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = s < a.n_samples;
-    if (!__any_sync(full, active)) return;
-    V3 P = mk(0, 0, 0), N = mk(0, 0, 0);
-    float dist = 0.0f;
-    if (active) {
-        P = ld3(a.spos[s]);
-        N = ld3(a.snrm[s]);
-        dist = sqrtf(a.srad[s].w);
-    }
-    const V3 P0 = P;
-    float lo[3] = {active ? P.x - dist : 3.0e38f, active ? P.y - dist : 3.0e38f, active ? P.z - dist : 3.0e38f};
-    float hi[3] = {active ? P.x + dist : -3.0e38f, active ? P.y + dist : -3.0e38f, active ? P.z + dist : -3.0e38f};
-    float dmax = dist;
-    for (int o = 16; o > 0; o >>= 1) {
+    const u32 n = a.list ? *a.n_list : a.n_samples - a.n_probe;
+    for (u32 first = blockIdx.x * blockDim.x + w * 32; first < n; first += gridDim.x * blockDim.x) {
+        const bool active = first + lane < n;
+        const u32 s = !active ? 0u : a.list ? a.list[first + lane] : a.n_probe + first + lane;
+        V3 P = mk(0, 0, 0), N = mk(0, 0, 0);
+        float dist = 0.0f;
+        if (active) {
+            P = ld3(a.spos[s]);
+            N = ld3(a.snrm[s]);
+            dist = sqrtf(a.srad[s].w);
+        }
+        const V3 P0 = P;
+        float lo[3] = {active ? P.x - dist : 3.0e38f, active ? P.y - dist : 3.0e38f, active ? P.z - dist : 3.0e38f};
+        float hi[3] = {active ? P.x + dist : -3.0e38f, active ? P.y + dist : -3.0e38f, active ? P.z + dist : -3.0e38f};
+        float dmax = dist;
+        for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            lo[c] = fminf(lo[c], __shfl_xor_sync(full, lo[c], o));
-            hi[c] = fmaxf(hi[c], __shfl_xor_sync(full, hi[c], o));
-        }
-        dmax = fmaxf(dmax, __shfl_xor_sync(full, dmax, o));
-    }
-    const float M = 4.0f * dmax + 0.05f;
-    const float G = 1.5f * M + 1e-3f;   // the extra covers rounding of the box arithmetic
-#pragma unroll
-    for (int c = 0; c < 3; ++c) { lo[c] -= G; hi[c] += G; }
-    int ncand = 0;
-    for (int base = 1; base < a.n_inst; base += 32) {
-        const int k = base + lane;
-        bool hit = false;
-        if (k < a.n_inst) {
-            const float4 b0 = __ldg(&a.inst_box[2 * k]), b1 = __ldg(&a.inst_box[2 * k + 1]);
-            hit = !(lo[0] > b1.x || hi[0] < b0.x || lo[1] > b1.y || hi[1] < b0.y || lo[2] > b1.z || hi[2] < b0.z);
-        }
-        const unsigned m = __ballot_sync(full, hit);
-        if (hit) {
-            const int at = ncand + __popc(m & ((1u << lane) - 1u));
-            if (at < kFixupCand) cand[w][at] = k;
-        }
-        ncand += __popc(m);
-    }
-    __syncwarp();
-    bool slow = ncand > kFixupCand;   // list overflow: every instance
-    int ci = 0, k = 1;
-    for (;;) {
-        if (!slow) {
-            if (ci >= ncand) break;
-            k = cand[w][ci++];
-        } else if (k >= a.n_inst) {
-            break;
-        }
-        fixup_instance_warp(a, k, active, P, N, dist);
-        const bool far = fabsf(P.x - P0.x) > M || fabsf(P.y - P0.y) > M || fabsf(P.z - P0.z) > M;
-        if (!slow && __any_sync(full, far)) slow = true;
-        ++k;
-    }
-    if (!active) return;
-    // push in front of overlapping faces (lighter.cpp:449-465); the
-    // reference's BSP query is replaced by the closest hit over occluders
-    if (a.max_correct_dist != 0.0f) {
-        int left = 100;
-        float md = a.max_correct_dist;
-        V3 PEnd = P + N * md;
-        while (md > kSmall && left-- > 0) {
-            V3 dn = normalized(PEnd - P);
-            V3 mA = P + dn * kSmall, mB = PEnd - dn * kSmall;
-            int ht = -1;
-            float q = bvh_closest(a.bvh, mA, mB, a.err, &ht);
-            V3 hn = mk(0, 0, 0);
-            if (ht >= 0) {
-                V3 P1, P2, P3; u32 meta, local;
-                load_tri(a.bvh, ht, P1, P2, P3, meta, local);
-                hn = tri_normal_rev(P1, P2, P3);
+            for (int c = 0; c < 3; ++c) {
+                lo[c] = fminf(lo[c], __shfl_xor_sync(full, lo[c], o));
+                hi[c] = fmaxf(hi[c], __shfl_xor_sync(full, hi[c], o));
             }
-            if (-dot(hn, N) < a.corr_min_dot) break;
-            if (q < kSmall) q = kSmall;
-            P = P * (1.0f - q) + PEnd * q;
-            md *= (1.0f - q);
+            dmax = fmaxf(dmax, __shfl_xor_sync(full, dmax, o));
+        }
+        const float M = 4.0f * dmax + 0.05f;
+        const float G = 1.5f * M + 1e-3f;   // the extra covers rounding of the box arithmetic
+#pragma unroll
+        for (int c = 0; c < 3; ++c) { lo[c] -= G; hi[c] += G; }
+        int ncand = 0;
+        for (int base = 1; base < a.n_inst; base += 32) {
+            const int k = base + lane;
+            bool hit = false;
+            if (k < a.n_inst) {
+                const float4 b0 = __ldg(&a.inst_box[2 * k]), b1 = __ldg(&a.inst_box[2 * k + 1]);
+                hit = !(lo[0] > b1.x || hi[0] < b0.x || lo[1] > b1.y || hi[1] < b0.y || lo[2] > b1.z || hi[2] < b0.z);
+            }
+            const unsigned m = __ballot_sync(full, hit);
+            if (hit) {
+                const int at = ncand + __popc(m & ((1u << lane) - 1u));
+                if (at < kFixupCand) cand[w][at] = k;
+            }
+            ncand += __popc(m);
+        }
+        __syncwarp();
+        bool slow = ncand > kFixupCand;   // list overflow: every instance
+        int ci = 0, k = 1;
+        for (;;) {
+            if (!slow) {
+                if (ci >= ncand) break;
+                k = cand[w][ci++];
+            } else if (k >= a.n_inst) {
+                break;
+            }
+            fixup_instance_warp(a, k, active, P, N, dist);
+            const bool far = fabsf(P.x - P0.x) > M || fabsf(P.y - P0.y) > M || fabsf(P.z - P0.z) > M;
+            if (!slow && __any_sync(full, far)) slow = true;
+            ++k;
+        }
+        __syncwarp();   // the warp's list is read before the next samples' is written
+        if (active) {
+            fixup_overlap(a, P, N);
+            a.spos[s] = st4(P, 0.0f);
         }
     }
-    a.spos[s] = st4(P, 0.0f);
 }
 
 // ----------------------------------------------------------------------------- direct light
@@ -2906,27 +2995,17 @@ void run_bake(ltr_Scene* S)
 
     TRACE("bvh issued");
     cudaEvent_t e_fix0 = clock.mark();
-    reftree_thread.join();
-    TRACE("reference trees joined");
-    if (reftree_error) std::rethrow_exception(reftree_error);
-    float4* d_ref_nodes = A.upload(ref_nodes);
-    int* d_ref_items = A.upload(ref_items);
-    int4* d_ref_inst = A.upload(ref_inst);
-    float4* d_fix_box = A.upload(fix_box);
+    FixupArgs fa;
     if (n_cov) {
-        FixupArgs fa;
-        fa.bvh = bv;
-        fa.err = err_fix;
-        fa.ref_nodes = d_ref_nodes;
-        fa.ref_items = d_ref_items;
-        fa.ref_inst = d_ref_inst;
-        fa.inst_box = d_fix_box;
-        fa.tri_xyz = d_tri_xyz;
         const u32 n_fix_tris = (u32) (tri_xyz.size() / 9);
         float4* d_tri_box = A.alloc<float4>(2 * (size_t) std::max<u32>(n_fix_tris, 1));
+        u32* d_fix_words = A.zeros<u32>(2);   // slivers, listed samples
         if (n_fix_tris) {
-            k_tri_boxes<<<(n_fix_tris + 255) / 256, 256, 0, st>>>(d_tri_xyz, n_fix_tris, d_tri_box); note_launch();
+            k_tri_boxes<<<(n_fix_tris + 255) / 256, 256, 0, st>>>(d_tri_xyz, n_fix_tris, d_tri_box, d_fix_words); note_launch();
         }
+        fa.bvh = bv;
+        fa.err = err_fix;
+        fa.tri_xyz = d_tri_xyz;
         fa.tri_box = d_tri_box;
         fa.n_inst = n_inst;
         fa.n_probe = n_probe;
@@ -2936,7 +3015,27 @@ void run_bake(ltr_Scene* S)
         fa.spos = d_spos;
         fa.snrm = d_snrm;
         fa.srad = d_srad;
-        k_fixup<<<(n_cov + kFixupThreads - 1) / kFixupThreads, kFixupThreads, 0, st>>>(fa); note_launch();
+        fa.slivers = d_fix_words;
+        fa.order = d_order_ao ? d_order_ao : d_order_dir;
+        fa.n_list = d_fix_words + 1;
+        fa.list = n_cov >= kFixQuickMin ? A.alloc<u32>(n_cov) : nullptr;
+        if (fa.list) {
+            k_fix_quick<<<(n_samples + kFixupThreads - 1) / kFixupThreads, kFixupThreads, 0, st>>>(fa); note_launch();
+            CK(cudaGetLastError());
+        }
+    }
+    reftree_thread.join();
+    TRACE("reference trees joined");
+    if (reftree_error) std::rethrow_exception(reftree_error);
+    if (n_cov) {
+        fa.ref_nodes = A.upload(ref_nodes);
+        fa.ref_items = A.upload(ref_items);
+        fa.ref_inst = A.upload(ref_inst);
+        fa.inst_box = A.upload(fix_box);
+        // the number of listed samples stays on the device: a few waves of blocks
+        unsigned grid = (n_cov + kFixupThreads - 1) / kFixupThreads;
+        if (fa.list) grid = std::min(grid, 152u * 16u);
+        k_fixup<<<grid, kFixupThreads, 0, st>>>(fa); note_launch();
         CK(cudaGetLastError());
         checkpoint("sample fixup");
     }

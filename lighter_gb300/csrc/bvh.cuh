@@ -650,6 +650,40 @@ __device__ __forceinline__ float warp_distance(const BvhView& b, V3 p, float d0,
     return active ? dist : d0;
 }
 
+// Calls leaf(t) for the leaves whose box lies within a lane's radius of its point
+// (radius2: squared; negative in lanes that ask for nothing), for all lanes alike,
+// until it returns false (uniformly).
+template <class Leaf>
+__device__ __forceinline__ void warp_walk_near(const BvhView& b, V3 p, float radius2, ErrFlag err, Leaf&& leaf)
+{
+    const unsigned full = 0xffffffffu;
+    if (b.n_tris <= 0 || !__any_sync(full, radius2 >= 0.0f)) return;
+    const F2 px = f2_make(p.x, p.x), py = f2_make(p.y, p.y), pz = f2_make(p.z, p.z), minus1 = f2_make(-1.0f, -1.0f);
+    int s0 = 0, s1 = 0, sp = 0;
+    int cur = b.root;
+    for (;;) {
+        if (cur >= 0) {
+            const NodePairs nd = load_pairs(b, cur);
+            const F2 gx = gap_pair(nd.mnx, nd.mxx, px, minus1), gy = gap_pair(nd.mny, nd.mxy, py, minus1),
+                     gz = gap_pair(nd.mnz, nd.mxz, pz, minus1);
+            float dl, dr;
+            f2_get(f2_fma(gx, gx, f2_fma(gy, gy, f2_mul(gz, gz))), dl, dr);
+            const bool hl = __any_sync(full, dl <= radius2), hr = __any_sync(full, dr <= radius2);
+            if (hl && hr) {
+                wstack_push(s0, s1, sp, nd.r, err);
+                cur = nd.l;
+                continue;
+            }
+            if (hl) { cur = nd.l; continue; }
+            if (hr) { cur = nd.r; continue; }
+        } else if (!leaf(~cur)) {
+            return;
+        }
+        if (sp == 0) return;
+        cur = wstack_pop(s0, s1, sp);
+    }
+}
+
 // bvh_any_hit for the active lanes' segments: a lane stops searching at its
 // first occluder hit (r < 1); the walk ends when no lane searches any more.
 __device__ __forceinline__ bool warp_any_hit(const BvhView& b, V3 o, V3 e, bool active, ErrFlag err)
@@ -689,12 +723,14 @@ __device__ __forceinline__ bool warp_any_hit(const BvhView& b, V3 o, V3 e, bool 
 
 // bvh_closest for the active lanes' segments (the smallest occluder hit
 // fraction, ties to the lower leaf -- a rule that does not depend on the
-// visiting order), each lane shrinking its own limit.
-__device__ __forceinline__ float warp_closest(const BvhView& b, V3 o, V3 e, bool active, ErrFlag err)
+// visiting order), each lane shrinking its own limit; *leaf gets the hit
+// triangle's leaf (or -1).
+__device__ __forceinline__ float warp_closest(const BvhView& b, V3 o, V3 e, bool active, ErrFlag err, int* leaf = nullptr)
 {
     const unsigned full = 0xffffffffu;
     float best = kNoHit;
     int bt = -1;
+    if (leaf) *leaf = -1;
     if (b.n_tris <= 0 || !__any_sync(full, active)) return best;
     const SlabPairs seg(inv_dir(e - o), o);
     float tlimit = active ? 1.0f : -1.0f;
@@ -728,6 +764,7 @@ __device__ __forceinline__ float warp_closest(const BvhView& b, V3 o, V3 e, bool
         if (sp == 0) break;
         cur = wstack_pop(s0, s1, sp);
     }
+    if (leaf) *leaf = bt;
     return best;
 }
 
