@@ -52,6 +52,8 @@
 #include "radiosity.cuh"
 
 namespace lg {
+void keep_pool_memory(int device);   // bake.cu
+
 namespace {
 
 void gck(cudaError_t e, const char* what, int line)
@@ -353,62 +355,81 @@ __device__ __forceinline__ int x_scale_exp(const u32* emax_bits)
 //             j >= n or r >= R
 // The G operand holds 2^g_exp G, the X operand 2^x_exp X (exact scalings).
 // B_out and xh may be null (not wanted); partial null means B = E.
-template <class T>
-__global__ void __launch_bounds__(256) k_combine(u32 n, u32 ld, u32 R, u32 Rpad, const float* __restrict__ partial,
-                                                 u32 max_slots, const u32* __restrict__ rp_cnt,
-                                                 const float* __restrict__ E, const float* __restrict__ albedo,
-                                                 float* __restrict__ B_out, T* __restrict__ xh, T* __restrict__ xl,
-                                                 int g_exp, const u32* __restrict__ emax_bits)
+//
+// With few row blocks (small n) a row block has a dozen slots, and their sum is a
+// chain of loads: SLOTS of them are in flight at a time, for PER elements per thread.
+// err: the products' error word; after a failed product B_out is left alone.
+template <class T, int PER, int SLOTS>
+__global__ void __launch_bounds__(1024 / PER) k_combine(u32 n, u32 ld, u32 R, u32 Rpad, const float* __restrict__ partial,
+                                                        u32 max_slots, const u32* __restrict__ rp_cnt,
+                                                        const float* __restrict__ E, const float* __restrict__ albedo,
+                                                        float* __restrict__ B_out, T* __restrict__ xh, T* __restrict__ xl,
+                                                        int g_exp, const u32* __restrict__ emax_bits, const u32* __restrict__ err)
 {
+    constexpr int ROWSTEP = 32 / PER;
     __shared__ float tile[32][33];
     const u32 j0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int x_exp = x_scale_exp(emax_bits);
     const float unscale = ldexpf(1.0f, -(g_exp + x_exp)), xscale = ldexpf(1.0f, x_exp);
+    const bool store = B_out && *err == 0u;
     // the loads of the second phase (E, albedo) go out together with those of the first,
     // so a block waits for about one memory round trip instead of three
-    float e[4], al[4];
+    float e[PER], al[PER];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {   // tx along r
-        const u32 j = j0 + ty + 8 * i, r = r0 + tx;
+    for (int i = 0; i < PER; ++i) {   // tx along r
+        const u32 j = j0 + ty + ROWSTEP * i, r = r0 + tx;
         const bool in = j < n && r < R;
         e[i] = in ? __ldg(&E[(size_t) j * R + r]) : 0.0f;
         al[i] = in ? __ldg(&albedo[3 * j + r % 3]) : 0.0f;
     }
     // the 32 patches of a tile lie in one 256-row block (j0 is a multiple of 32)
     const u32 rp = j0 / ROWS, cnt = (partial && j0 < n) ? __ldg(&rp_cnt[rp]) : 0u;
-    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    for (u32 s = 0; s < cnt; ++s) {
+    float v[PER];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {   // tx along j
-            const u32 r = r0 + ty + 8 * i, j = j0 + tx;
-            if (j < n && r < R) v[i] += __ldg(&partial[(((size_t) rp * max_slots + s) * R + r) * ROWS + (j % ROWS)]);
-        }
+    for (int i = 0; i < PER; ++i) v[i] = 0.0f;
+    const size_t step = (size_t) R * ROWS;
+    const float* P = partial + ((size_t) rp * max_slots * R + r0 + ty) * ROWS + (j0 + tx) % ROWS;   // tx along j
+    for (u32 s = 0; s < cnt; s += SLOTS) {
+        float q[SLOTS][PER];
+#pragma unroll
+        for (u32 u = 0; u < SLOTS; ++u)
+#pragma unroll
+            for (int i = 0; i < PER; ++i)
+                q[u][i] = s + u < cnt && r0 + ty + ROWSTEP * i < R && j0 + tx < n
+                              ? __ldg(P + (s + u) * step + ROWSTEP * i * ROWS) : 0.0f;
+#pragma unroll
+        for (u32 u = 0; u < SLOTS; ++u)
+#pragma unroll
+            for (int i = 0; i < PER; ++i)
+                if (s + u < cnt) v[i] += q[u][i];
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) tile[ty + 8 * i][tx] = v[i];
+    for (int i = 0; i < PER; ++i) tile[ty + ROWSTEP * i][tx] = v[i];
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {   // tx along r
-        const int k = ty + 8 * i;
+    for (int i = 0; i < PER; ++i) {   // tx along r
+        const int k = ty + ROWSTEP * i;
         const u32 j = j0 + k, r = r0 + tx;
         float x = 0.0f;
         if (j < n && r < R) {
             const float b = e[i] + tile[tx][k] * unscale;
-            if (B_out) B_out[(size_t) j * R + r] = b;
+            if (store) B_out[(size_t) j * R + r] = b;
             x = al[i] * b * xscale;
         }
-        tile[tx][k] = x;
+        tile[tx][k] = x;   // the element that this thread read
     }
-    __syncthreads();
     if (!xh) return;
-    for (int k = ty; k < 32; k += 8) {   // tx along j
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {   // tx along j
+        const int k = ty + ROWSTEP * i;
         const u32 r = r0 + k, j = j0 + tx;
         if (r < Rpad && j < ld) {
-            const float v = tile[k][tx];
-            const T h = to16<T>(v);
+            const float w = tile[k][tx];
+            const T h = to16<T>(w);
             xh[(size_t) r * ld + j] = h;
-            if (xl) xl[(size_t) r * ld + j] = to16<T>(v - from16(h));
+            if (xl) xl[(size_t) r * ld + j] = to16<T>(w - from16(h));
         }
     }
 }
@@ -606,37 +627,87 @@ int sgemm_tn(u32 R)
 
 // ----------------------------------------------------------------------------- G preparation
 
-// G_ij = F_ij * area_j, in place (row stride ldg; the padding columns stay 0).
-__global__ void k_scale_cols(u32 n, u32 ldg, float* __restrict__ G, const float* __restrict__ area)
-{
-    const size_t t = blockIdx.x * (size_t) blockDim.x + threadIdx.x;
-    if (t >= (size_t) n * ldg) return;
-    const u32 j = (u32) (t % ldg);
-    if (j < n) G[t] *= area[j];
-}
-
-// *out = max |x| as float bits (non-negative floats order like their bits); *out starts at 0.
-__global__ void k_absmax(const float* __restrict__ x, size_t count, u32* out)
+// G_ij = F_ij * area_j, in place, and *out = max G_ij as float bits (non-negative
+// floats order like their bits; *out starts at 0). Rows of ldg floats, a multiple of
+// 4; the padding columns stay 0. One pass over G, 16 bytes at a time (as two passes
+// of single floats with a 64-bit remainder each, 4,096 patches took 81 us).
+__global__ void __launch_bounds__(256) k_scale_cols(u32 n, u32 ldg, float* __restrict__ G, const float* __restrict__ area, u32* out)
 {
     float m = 0.0f;
-    for (size_t t = blockIdx.x * (size_t) blockDim.x + threadIdx.x; t < count; t += (size_t) gridDim.x * blockDim.x)
-        m = fmaxf(m, fabsf(x[t]));
+    for (u32 i = blockIdx.x; i < n; i += gridDim.x) {
+        float4* row = reinterpret_cast<float4*>(G + (size_t) i * ldg);
+        for (u32 c = threadIdx.x; c < ldg / 4; c += 256) {
+            float4 g = row[c];
+            const u32 j = 4 * c;
+            g.x *= __ldg(&area[j]);   // j < n: the padding is less than four columns
+            if (j + 1 < n) g.y *= __ldg(&area[j + 1]);
+            if (j + 2 < n) g.z *= __ldg(&area[j + 2]);
+            if (j + 3 < n) g.w *= __ldg(&area[j + 3]);
+            row[c] = g;
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(g.x), fabsf(g.y)), fmaxf(fabsf(g.z), fabsf(g.w))));
+        }
+    }
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
+    if ((threadIdx.x & 31) == 0 && m > 0.0f) atomicMax(out, __float_as_uint(m));
+}
+
+// The right-hand sides on their way in: *out = max |x| as float bits (*out starts at
+// 0) and, with copy, copy = x; with alb, alb_copy = alb (na floats). x and alb are
+// then the caller's host arrays where kernels can address pageable host memory
+// (cudaDevAttrPageableMemoryAccess, e.g. Grace systems: the GPU walks the host page
+// tables over the CPU-GPU link). 16-byte vectors when both sides are aligned.
+__device__ __forceinline__ float copy_max(const float* __restrict__ x, float* __restrict__ copy, size_t count)
+{
+    float m = 0.0f;
+    const size_t stride = (size_t) gridDim.x * blockDim.x, t0 = blockIdx.x * (size_t) blockDim.x + threadIdx.x;
+    size_t t = t0;
+    if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(copy)) & 15u) == 0) {
+        for (size_t k = t0; k < count / 4; k += stride) {
+            const float4 v = reinterpret_cast<const float4*>(x)[k];
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+            if (copy) reinterpret_cast<float4*>(copy)[k] = v;
+        }
+        t = count / 4 * 4 + t0;
+    }
+    for (; t < count; t += stride) {
+        const float v = x[t];
+        m = fmaxf(m, fabsf(v));
+        if (copy) copy[t] = v;
+    }
+    return m;
+}
+
+__global__ void __launch_bounds__(256) k_take_in(const float* __restrict__ x, float* __restrict__ copy, size_t count,
+                                                 const float* __restrict__ alb, float* __restrict__ alb_copy, size_t na,
+                                                 u32* out)
+{
+    if (alb) copy_max(alb, alb_copy, na);
+    float m = copy_max(x, copy, count);
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0 && m > 0.0f) atomicMax(out, __float_as_uint(m));
 }
 
 // hi = 16-bit 2^g_exp G (row stride ld, zero columns j >= n); lo = 16-bit residual when requested.
+// Four columns per thread: 16 bytes in, 8 out.
 template <class T>
-__global__ void k_g_to_16(u32 n, u32 ld, u32 ldg, const float* __restrict__ G, T* __restrict__ hi, T* __restrict__ lo,
-                          float gscale)
+__global__ void __launch_bounds__(256) k_g_to_16(u32 n, u32 ld, u32 ldg, const float* __restrict__ G, T* __restrict__ hi,
+                                                 T* __restrict__ lo, float gscale)
 {
-    const size_t t = blockIdx.x * (size_t) blockDim.x + threadIdx.x;
-    if (t >= (size_t) n * ld) return;
-    const u32 i = (u32) (t / ld), j = (u32) (t % ld);
-    const float g = j < n ? G[(size_t) i * ldg + j] * gscale : 0.0f;
-    const T h = to16<T>(g);
-    hi[t] = h;
-    if (lo) lo[t] = to16<T>(g - from16(h));
+    for (u32 i = blockIdx.x; i < n; i += gridDim.x) {
+        const float4* row = reinterpret_cast<const float4*>(G + (size_t) i * ldg);
+        for (u32 c = threadIdx.x; c < ld / 4; c += 256) {
+            const float4 g = 4 * c < ldg ? __ldcs(&row[c]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float v[4] = {g.x * gscale, g.y * gscale, g.z * gscale, g.w * gscale};
+            alignas(8) T h[4], l[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                h[k] = to16<T>(v[k]);
+                l[k] = to16<T>(v[k] - from16(h[k]));
+            }
+            reinterpret_cast<uint2*>(hi + (size_t) i * ld)[c] = *reinterpret_cast<const uint2*>(h);
+            if (lo) reinterpret_cast<uint2*>(lo + (size_t) i * ld)[c] = *reinterpret_cast<const uint2*>(l);
+        }
+    }
 }
 
 // ----------------------------------------------------------------------------- host helpers
@@ -683,21 +754,23 @@ CUtensorMap make_map(const void* ptr, CUtensorMapDataType dt, u32 ld, u32 rows, 
 // 0.738 ms; it also lets that mode take R = 256).
 u32 stage_k(int refine) { return refine == LTRG_REFINE_FULL ? 32u : 64u; }
 
+// Device buffer from the device's memory pool (which the bakes keep filled between
+// objects, see keep_pool_memory: mapping and unmapping a gather's matrices took
+// most of a millisecond), allocated and freed on the gather's stream.
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
-    void ensure(size_t b)
+    bool ensure(size_t b, cudaStream_t st)   // whether it was allocated anew
     {
-        if (b <= bytes) return;
-        if (p) cudaFree(p);
-        p = nullptr;
-        bytes = 0;
-        GCK(cudaMalloc(&p, b));
+        if (b <= bytes) return false;
+        release(st);
+        GCK(cudaMallocAsync(&p, b, st));
         bytes = b;
+        return true;
     }
-    void release()
+    void release(cudaStream_t st)
     {
-        if (p) cudaFree(p);
+        if (p) cudaFreeAsync(p, st);
         p = nullptr;
         bytes = 0;
     }
@@ -724,26 +797,6 @@ struct PinBuf {
         bytes = 0;
     }
 };
-
-// Copy of `n` floats by the GPU where the host's pageable memory is directly
-// addressable by kernels (cudaDevAttrPageableMemoryAccess, e.g. Grace systems:
-// the GPU walks the host page tables over the CPU-GPU link): one of src and
-// dst is the caller's pageable host buffer. 16-byte vectors when both are
-// aligned, single floats otherwise.
-__global__ void k_copy_floats(float* __restrict__ dst, const float* __restrict__ src, size_t n)
-{
-    const size_t stride = (size_t) gridDim.x * blockDim.x;
-    const size_t t0 = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
-    if (((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15u) == 0) {
-        const size_t n4 = n / 4;
-        float4* d4 = reinterpret_cast<float4*>(dst);
-        const float4* s4 = reinterpret_cast<const float4*>(src);
-        for (size_t i = t0; i < n4; i += stride) d4[i] = s4[i];
-        for (size_t i = 4 * n4 + t0; i < n; i += stride) dst[i] = src[i];
-    } else {
-        for (size_t i = t0; i < n; i += stride) dst[i] = src[i];
-    }
-}
 
 // Whether kernels on `device` may address pageable host memory (queried once).
 bool pageable_access(int device)
@@ -892,9 +945,13 @@ struct ltrg_Gather {
     u32 kchunk = 0;               // k blocks per TMEM accumulation (0: whole range of a CTA)
     DevBuf rp_tab;                // rp_first[n_rp], rp_cnt[n_rp]
     // solve scratch
-    DevBuf partial, xh, xl, x32, err, emax;
+    DevBuf partial, xh, xl, x32;
+    DevBuf words;                 // [0] error word of the products, [1] largest emission
     DevBuf h_alb, h_E, h_out;     // device copies for the host-buffer entry point
     PinBuf pin_in, pin_out;       // its page-locked staging
+    PinBuf pin_err;               // the error word as read back
+    std::vector<cudaEvent_t> events;   // of a solve's timings, used again by the next
+    bool grown = false;           // a buffer was allocated since the last wait for `st`
     std::unique_ptr<StagePool> pool;   // its host copy threads (started by the first host-buffer solve)
     int pool_threads = 0;
     uint64_t links = 0, vis_rays = 0, pairs = 0;
@@ -909,12 +966,23 @@ struct ltrg_Gather {
         if (!st) return;
         cudaSetDevice(device);
         cudaStreamSynchronize(st);
-        DevBuf* all[] = {&G32,  &G16, &G16lo, &rp_tab, &partial, &xh,    &xl,
-                         &x32,  &err,  &emax,   &h_alb,   &h_E,   &h_out};
-        for (DevBuf* b : all) b->release();
+        DevBuf* all[] = {&G32, &G16, &G16lo, &rp_tab, &partial, &xh, &xl, &x32, &words, &h_alb, &h_E, &h_out};
+        for (DevBuf* b : all) b->release(st);
+        for (cudaEvent_t e : events) cudaEventDestroy(e);
         pin_in.release();
         pin_out.release();
+        pin_err.release();
+        cudaStreamSynchronize(st);
+        // as a destroyed scene does: the pool gives back what it holds beyond 8 GiB
+        cudaMemPool_t pool;
+        if (cudaDeviceGetDefaultMemPool(&pool, device) != cudaSuccess || cudaMemPoolTrimTo(pool, 8ull << 30) != cudaSuccess)
+            (void) cudaGetLastError();
         cudaStreamDestroy(st);
+    }
+
+    void need(DevBuf& b, size_t bytes)
+    {
+        if (b.ensure(bytes, st)) grown = true;
     }
 
     void schedule()
@@ -936,35 +1004,67 @@ struct ltrg_Gather {
         for (u32 rp = 0; rp < n_rp; ++rp) max_slots = std::max(max_slots, cnt[rp]);
         std::vector<u32> tab(first);
         tab.insert(tab.end(), cnt.begin(), cnt.end());
-        rp_tab.ensure(tab.size() * 4);
-        GCK(cudaMemcpy(rp_tab.p, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice));
+        need(rp_tab, tab.size() * 4);
+        GCK(cudaMemcpyAsync(rp_tab.p, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice, st));
+        GCK(cudaStreamSynchronize(st));
     }
 
-    // B for R right-hand sides; all pointers on this device, enqueued on `s`.
-    void solve(const float* alb, const float* E, u32 R, int bounces, int precision, int refine, float* out,
-               ltrg_GatherStats* stats, cudaStream_t s);
+    // B for R right-hand sides, enqueued on `s`; all pointers are addressable by this
+    // device's kernels. alb_host/E_host (or null): host arrays to be copied to alb
+    // and E first, by kernels; `out` may then be a host array too.
+    void solve(float* alb, float* E, u32 R, int bounces, int precision, int refine, float* out, ltrg_GatherStats* stats,
+               cudaStream_t s, const float* alb_host = nullptr, const float* E_host = nullptr);
 };
 
-void ltrg_Gather::solve(const float* alb, const float* E, u32 R, int bounces, int precision, int refine, float* out,
-                        ltrg_GatherStats* stats, cudaStream_t s)
+void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision, int refine, float* out,
+                        ltrg_GatherStats* stats, cudaStream_t s, const float* alb_host, const float* E_host)
 {
     const bool tc = precision != LTRG_F_FP32;
     if (tc && R > (u32) MAX_BN) throw std::runtime_error("tensor-core gather takes at most 256 right-hand sides");
     if (refine < LTRG_REFINE_NONE || refine > LTRG_REFINE_FULL) throw std::runtime_error("invalid refine level");
-    err.ensure(4);
-    GCK(cudaMemsetAsync(err.p, 0, 4, s));
-    std::vector<cudaEvent_t> ev;
+    need(words, 8);
+    pin_err.ensure(4);
+    u32* d_err = words.as<u32>();
+    u32* d_emax = words.as<u32>() + 1;
+    size_t ev_used = 0;
     auto event = [&]() {
-        cudaEvent_t e;
-        GCK(cudaEventCreate(&e));
-        ev.push_back(e);
-        GCK(cudaEventRecord(e, s));
-        return e;
+        if (ev_used == events.size()) {
+            cudaEvent_t e;
+            GCK(cudaEventCreate(&e));
+            events.push_back(e);
+        }
+        GCK(cudaEventRecord(events[ev_used], s));
+        return events[ev_used++];
     };
-    struct EvGuard {
-        std::vector<cudaEvent_t>& v;
-        ~EvGuard() { for (cudaEvent_t e : v) cudaEventDestroy(e); }
-    } evg{ev};
+    // buffers allocated on the gather's stream are used on `s`
+    auto begin = [&]() {
+        if (grown) {
+            GCK(cudaStreamSynchronize(st));
+            grown = false;
+        }
+        GCK(cudaMemsetAsync(words.p, 0, 8, s));
+        if (tc || E_host) {
+            const size_t count = (size_t) n * R;
+            k_take_in<<<(unsigned) std::min<size_t>((size_t) sm_count * 8, (count + 1023) / 1024), 256, 0, s>>>(
+                E_host ? E_host : E, E_host ? E : nullptr, count, alb_host, alb, (size_t) n * 3, d_emax); note_launch();
+            GCK(cudaGetLastError());
+        }
+    };
+    // nothing of a solve that ends by an exception runs on after it
+    struct Wait {
+        cudaStream_t s;
+        bool on;
+        ~Wait() { if (on) cudaStreamSynchronize(s); }
+    } wait{s, true};
+    // the end of a solve: one wait, after which the error word is on the host
+    auto finish = [&]() {
+        GCK(cudaMemcpyAsync(pin_err.p, d_err, 4, cudaMemcpyDeviceToHost, s));
+        GCK(cudaStreamSynchronize(s));
+        wait.on = false;
+        const u32 herr = *(const u32*) pin_err.p;
+        if (herr)
+            throw std::runtime_error("tensor-core gather: a pipeline wait expired (error word " + std::to_string(herr) + ")");
+    };
     double ms_convert = 0, ms_gemm = 0, ms_bounces = 0;
     int stages = 0, products = 1;
     int32_t ctas32 = 0;
@@ -978,8 +1078,9 @@ void ltrg_Gather::solve(const float* alb, const float* E, u32 R, int bounces, in
         const u32 sg_cta = (u32) std::min<uint64_t>((uint64_t) sm_count * SGBlocksPerSM, total);
         // slots: the most ranges that one tile's units can fall into
         const u32 slots = (u32) std::min<uint64_t>(sg_cta, ((uint64_t) skb * sg_cta + total - 1) / total + 1);
-        partial.ensure((size_t) tiles_m * tiles_n * slots * SGM * bn * 4);
-        x32.ensure((size_t) tiles_n * bn * ldx * 4);
+        need(partial, (size_t) tiles_m * tiles_n * slots * SGM * bn * 4);
+        need(x32, (size_t) tiles_n * bn * ldx * 4);
+        begin();
         const dim3 cb(32, 8), cg((ldx + 31) / 32, tiles_n * bn / 32);
         auto combine = [&](bool with_partial, bool last) {
             k_combine32<<<cg, cb, 0, s>>>(n, ldx, R, bn, tiles_n, skb, total, sg_cta, slots,
@@ -1004,7 +1105,7 @@ void ltrg_Gather::solve(const float* alb, const float* E, u32 R, int bounces, in
             combine(true, b + 1 == bounces);
         }
         cudaEvent_t e1 = event();
-        GCK(cudaStreamSynchronize(s));
+        finish();
         float m = 0;
         cudaEventElapsedTime(&m, e0, e1);
         ms_bounces = m;
@@ -1012,29 +1113,6 @@ void ltrg_Gather::solve(const float* alb, const float* E, u32 R, int bounces, in
         bytes_bounce = (uint64_t) n * n * 4;
     } else {
         const bool need_lo = refine == LTRG_REFINE_FULL;
-        if (g16_kind != precision || (need_lo && !g16_has_lo)) {
-            cudaEvent_t c0 = event();
-            G16.ensure((size_t) n * ld * 2);
-            if (need_lo) G16lo.ensure((size_t) n * ld * 2);
-            const size_t tot = (size_t) n * ld;
-            const unsigned grid = (unsigned) ((tot + 255) / 256);
-            const float gscale = ldexpf(1.0f, g_exp);
-            if (precision == LTRG_F_FP16)
-                k_g_to_16<__half><<<grid, 256, 0, s>>>(n, ld, ldg, G32.as<float>(), G16.as<__half>(),
-                                                       need_lo ? G16lo.as<__half>() : nullptr, gscale);
-            else
-                k_g_to_16<__nv_bfloat16><<<grid, 256, 0, s>>>(n, ld, ldg, G32.as<float>(), G16.as<__nv_bfloat16>(),
-                                                              need_lo ? G16lo.as<__nv_bfloat16>() : nullptr, gscale);
-            note_launch();
-            GCK(cudaGetLastError());
-            cudaEvent_t c1 = event();
-            GCK(cudaEventSynchronize(c1));
-            float m = 0;
-            cudaEventElapsedTime(&m, c0, c1);
-            ms_convert = m;
-            g16_kind = precision;
-            g16_has_lo = need_lo;
-        }
         const u32 BN = std::max<u32>(32, (R + 31) / 32 * 32);
         const u32 KB = stage_k(refine);
         const u32 b_bytes = BN * KB * 2, a_bytes = ROWS * KB * 2;
@@ -1044,9 +1122,28 @@ void ltrg_Gather::solve(const float* alb, const float* E, u32 R, int bounces, in
         const size_t smem = (size_t) stages * stage_bytes + kSmemExtra;
         products = 1 + (refine >= LTRG_REFINE_RHS) + (refine == LTRG_REFINE_FULL);
         // every element of X^T (padding included) is written by the first k_combine
-        xh.ensure((size_t) BN * ld * 2);
-        xl.ensure((size_t) BN * ld * 2);
-        partial.ensure((size_t) n_rp * max_slots * R * ROWS * 4);
+        need(G16, (size_t) n * ld * 2);
+        if (need_lo) need(G16lo, (size_t) n * ld * 2);
+        need(xh, (size_t) BN * ld * 2);
+        need(xl, (size_t) BN * ld * 2);
+        need(partial, (size_t) n_rp * max_slots * R * ROWS * 4);
+        begin();
+        cudaEvent_t c0 = nullptr, c1 = nullptr;
+        if (g16_kind != precision || (need_lo && !g16_has_lo)) {
+            c0 = event();
+            const unsigned grid = (unsigned) std::min<u32>(n, (u32) sm_count * 8);
+            const float gscale = ldexpf(1.0f, g_exp);
+            if (precision == LTRG_F_FP16)
+                k_g_to_16<__half><<<grid, 256, 0, s>>>(n, ld, ldg, G32.as<float>(), G16.as<__half>(),
+                                                       need_lo ? G16lo.as<__half>() : nullptr, gscale);
+            else
+                k_g_to_16<__nv_bfloat16><<<grid, 256, 0, s>>>(n, ld, ldg, G32.as<float>(), G16.as<__nv_bfloat16>(),
+                                                              need_lo ? G16lo.as<__nv_bfloat16>() : nullptr, gscale);
+            note_launch();
+            GCK(cudaGetLastError());
+            c1 = event();
+            g16_kind = -1;   // until the conversion is known to be done
+        }
         const CUtensorMapDataType dt =
             precision == LTRG_F_FP16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
         const CUtensorMap mG = make_map(G16.p, dt, ld, n, ROWS, KB);
@@ -1063,7 +1160,7 @@ void ltrg_Gather::solve(const float* alb, const float* E, u32 R, int bounces, in
         ua.kchunk = kchunk;
         ua.rp_first = rp_tab.as<u32>();
         ua.partial = partial.as<float>();
-        ua.err = err.as<u32>();
+        ua.err = d_err;
         ua.wait_cycles = kWaitCycles;
         ua.issue = 1;
         if (stall_us) {   // test hook: copies never issued, waits cut short
@@ -1072,24 +1169,26 @@ void ltrg_Gather::solve(const float* alb, const float* E, u32 R, int bounces, in
             stall_us = 0;
         }
         const u32* rp_cnt = rp_tab.as<u32>() + n_rp;
-        emax.ensure(4);
-        GCK(cudaMemsetAsync(emax.p, 0, 4, s));
-        k_absmax<<<std::max<u32>(1, std::min<u32>(1024, (u32) (((size_t) n * R + 255) / 256))), 256, 0, s>>>(
-            E, (size_t) n * R, emax.as<u32>()); note_launch();
-        dim3 cb(32, 8), cg((ld + 31) / 32, (BN + 31) / 32);
-        auto combine = [&](bool with_partial, bool last) {
-            float* bo = last ? out : nullptr;
-            const float* P = with_partial ? partial.as<float>() : nullptr;
-            if (precision == LTRG_F_FP16)
-                k_combine<__half><<<cg, cb, 0, s>>>(n, ld, R, BN, P, max_slots, rp_cnt, E, alb, bo,
-                                                    last ? nullptr : xh.as<__half>(),
-                                                    (last || refine == LTRG_REFINE_NONE) ? nullptr : xl.as<__half>(),
-                                                    g_exp, emax.as<u32>());
-            else
-                k_combine<__nv_bfloat16><<<cg, cb, 0, s>>>(
-                    n, ld, R, BN, P, max_slots, rp_cnt, E, alb, bo, last ? nullptr : xh.as<__nv_bfloat16>(),
-                    (last || refine == LTRG_REFINE_NONE) ? nullptr : xl.as<__nv_bfloat16>(), g_exp, emax.as<u32>());
+        // Up to one tile per SM, a block's own chain of slots is the time: one element per
+        // thread, eight slots in flight (1,500 patches, R = 45, 26 slots: 7.8 us; four
+        // elements and one slot 11.0, four and four 9.5). While the blocks of all tiles are
+        // resident at once, four elements and four slots (3,000 patches, R = 45: 7.9 us;
+        // one at a time 9.3). Beyond, the blocks that wait their turn cover the loads and
+        // more registers only cost occupancy (16,384 patches, R = 192: 15.6 us with one slot
+        // at a time, 16.8 with four, 28.2 with one element per thread).
+        const dim3 cg((ld + 31) / 32, (BN + 31) / 32);
+        const u32 tiles = cg.x * cg.y, per = tiles <= (u32) sm_count ? 1 : 4, slots = tiles <= 8u * (u32) sm_count ? 4 : 1;
+        auto combine_as = [&](auto type, bool with_partial, bool last) {
+            using T = decltype(type);
+            (per == 1 ? k_combine<T, 1, 8> : slots == 4 ? k_combine<T, 4, 4> : k_combine<T, 4, 1>)<<<cg, dim3(32, 32 / per), 0, s>>>(
+                n, ld, R, BN, with_partial ? partial.as<float>() : nullptr, max_slots, rp_cnt, E, alb, last ? out : nullptr,
+                last ? nullptr : xh.as<T>(), (last || refine == LTRG_REFINE_NONE) ? nullptr : xl.as<T>(), g_exp, d_emax,
+                d_err);
             note_launch();
+        };
+        auto combine = [&](bool with_partial, bool last) {
+            if (precision == LTRG_F_FP16) combine_as(__half(), with_partial, last);
+            else combine_as(__nv_bfloat16(), with_partial, last);
         };
         cudaEvent_t e0 = event();
         combine(false, bounces == 0);
@@ -1103,13 +1202,14 @@ void ltrg_Gather::solve(const float* alb, const float* E, u32 R, int bounces, in
             combine(true, b + 1 == bounces);
         }
         cudaEvent_t e1 = event();
-        GCK(cudaStreamSynchronize(s));
-        u32 herr = 0;
-        GCK(cudaMemcpy(&herr, err.p, 4, cudaMemcpyDeviceToHost));
-        if (herr)
-            throw std::runtime_error("tensor-core gather: a pipeline wait expired (error word " + std::to_string(herr) +
-                                     ")");
+        finish();
         float m = 0;
+        if (c0) {
+            g16_kind = precision;
+            g16_has_lo = need_lo;
+            cudaEventElapsedTime(&m, c0, c1);
+            ms_convert = m;
+        }
         cudaEventElapsedTime(&m, e0, e1);
         ms_bounces = m;
         for (auto& p : ge) { cudaEventElapsedTime(&m, p.first, p.second); ms_gemm += m; }
@@ -1149,6 +1249,7 @@ LTRAPI ltrg_Gather* ltrg_GatherCreate(const float* tri_xyz, u32 n_tris, const fl
         if (device < 0 || device >= ndev) throw std::runtime_error("device out of range");
         g->device = device;
         GCK(cudaSetDevice(device));
+        keep_pool_memory(device);
         GCK(cudaDeviceGetAttribute(&g->sm_count, cudaDevAttrMultiProcessorCount, device));
         GCK(cudaStreamCreateWithFlags(&g->st, cudaStreamNonBlocking));
         g->n = n;
@@ -1206,7 +1307,7 @@ LTRAPI ltrg_Gather* ltrg_GatherCreate(const float* tri_xyz, u32 n_tris, const fl
         const float* da = (const float*) up(area, n * sizeof(float));
         u32* derr = (u32*) up(nullptr, 0);
         GCK(cudaMemsetAsync(derr, 0, 4, st));
-        g->G32.ensure((size_t) n * g->ldg * 4);
+        g->need(g->G32, (size_t) n * g->ldg * 4);
 
         cudaEvent_t e0, e1;
         GCK(cudaEventCreate(&e0));
@@ -1214,13 +1315,11 @@ LTRAPI ltrg_Gather* ltrg_GatherCreate(const float* tri_xyz, u32 n_tris, const fl
         GCK(cudaEventRecord(e0, st));
         BvhView view = bin.n ? bvh.view() : BvhView{nullptr, nullptr, nullptr, nullptr, 0, 0};
         RadFormFactors ff = radiosity_form_factors_f32(n, g->ldg, dp, dn, view, ErrFlag{derr}, links, g->G32.as<float>(), st);
-        const size_t nn2 = (size_t) n * g->ldg;
-        k_scale_cols<<<(unsigned) ((nn2 + 255) / 256), 256, 0, st>>>(n, g->ldg, g->G32.as<float>(), da); note_launch();
-        GCK(cudaGetLastError());
-        GCK(cudaEventRecord(e1, st));
         u32* dgmax = (u32*) up(nullptr, 0);
         GCK(cudaMemsetAsync(dgmax, 0, 4, st));
-        k_absmax<<<1024, 256, 0, st>>>(g->G32.as<float>(), nn2, dgmax); note_launch();
+        k_scale_cols<<<std::min<u32>(n, (u32) g->sm_count * 8), 256, 0, st>>>(n, g->ldg, g->G32.as<float>(), da, dgmax); note_launch();
+        GCK(cudaGetLastError());
+        GCK(cudaEventRecord(e1, st));
         u32 herr = 0, hgmax = 0;
         int hbvh = 0;
         if (bin.n) GCK(cudaMemcpyAsync(&hbvh, bvh.status, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1315,8 +1414,8 @@ LTRAPI LTRBOOL ltrg_GatherSolveDevice(ltrg_Gather* g, const float* albedo_rgb, c
             precision > LTRG_F_BF16)
             throw std::runtime_error("invalid arguments");
         GCK(cudaSetDevice(g->device));
-        g->solve(albedo_rgb, emission, R, bounces, precision, refine, out, stats,
-                 stream ? (cudaStream_t) stream : g->st);
+        g->solve(const_cast<float*>(albedo_rgb), const_cast<float*>(emission), R, bounces, precision, refine, out, stats,
+                 stream ? (cudaStream_t) stream : g->st);   // (without host arrays, alb and E are only read)
     } catch (const std::exception& e) {
         g->error = e.what();
         cudaGetLastError();   // the error is reported here; none is left for the caller's next CUDA call
@@ -1338,34 +1437,29 @@ LTRAPI LTRBOOL ltrg_GatherSolve(ltrg_Gather* g, const float* albedo_rgb, const f
         GCK(cudaSetDevice(g->device));
         const u32 n = g->n;
         cudaStream_t s = g->st;
-        g->h_alb.ensure((size_t) n * 3 * 4);
-        g->h_E.ensure((size_t) n * R * 4);
-        g->h_out.ensure((size_t) n * R * 4);
+        g->need(g->h_alb, (size_t) n * 3 * 4);
+        g->need(g->h_E, (size_t) n * R * 4);
         const bool direct = g->host_path ? g->host_path == 2 : pageable_access(g->device);
-        const unsigned cgrid = (unsigned) g->sm_count * 8;
-        if (direct) {
-            // the GPU reads the caller's arrays over the CPU-GPU link: no host copies
-            k_copy_floats<<<cgrid, 256, 0, s>>>(g->h_alb.as<float>(), albedo_rgb, (size_t) n * 3); note_launch();
-            k_copy_floats<<<cgrid, 256, 0, s>>>(g->h_E.as<float>(), emission, (size_t) n * R); note_launch();
-            GCK(cudaGetLastError());
-        } else {
-            GCK(cudaMemcpyAsync(g->h_alb.p, albedo_rgb, (size_t) n * 3 * 4, cudaMemcpyHostToDevice, s));
-            if (!g->pool) {
-                g->pool_threads = std::max(1, std::min(16, (int) std::thread::hardware_concurrency()));
-                g->pool.reset(new StagePool);
-                g->pool->start(g->pool_threads - 1);   // the calling thread works too
-            }
-            stage_h2d(g->h_E.p, emission, (size_t) n * R * 4, g->pin_in, s, *g->pool, g->pool_threads);
-        }
         note_h2d((size_t) n * (3 + R) * 4);
-        g->solve(g->h_alb.as<float>(), g->h_E.as<float>(), R, bounces, precision, refine, g->h_out.as<float>(), stats,
-                 s);
         if (direct) {
-            k_copy_floats<<<cgrid, 256, 0, s>>>(out, g->h_out.as<float>(), (size_t) n * R); note_launch();
-            GCK(cudaGetLastError());
-        } else {
-            stage_d2h(out, g->h_out.p, (size_t) n * R * 4, g->pin_out, s, *g->pool, g->pool_threads);
+            // the GPU reads and writes the caller's arrays over the CPU-GPU link: no host
+            // copies; the emission's maximum is taken on its way in, and the last bounce
+            // writes its result where it belongs
+            g->solve(g->h_alb.as<float>(), g->h_E.as<float>(), R, bounces, precision, refine, out, stats, s, albedo_rgb,
+                     emission);
+            note_d2h((size_t) n * R * 4);
+            return 1;
         }
+        g->need(g->h_out, (size_t) n * R * 4);
+        GCK(cudaMemcpyAsync(g->h_alb.p, albedo_rgb, (size_t) n * 3 * 4, cudaMemcpyHostToDevice, s));
+        if (!g->pool) {
+            g->pool_threads = std::max(1, std::min(16, (int) std::thread::hardware_concurrency()));
+            g->pool.reset(new StagePool);
+            g->pool->start(g->pool_threads - 1);   // the calling thread works too
+        }
+        stage_h2d(g->h_E.p, emission, (size_t) n * R * 4, g->pin_in, s, *g->pool, g->pool_threads);
+        g->solve(g->h_alb.as<float>(), g->h_E.as<float>(), R, bounces, precision, refine, g->h_out.as<float>(), stats, s);
+        stage_d2h(out, g->h_out.p, (size_t) n * R * 4, g->pin_out, s, *g->pool, g->pool_threads);
         note_d2h((size_t) n * R * 4);
         GCK(cudaStreamSynchronize(s));
     } catch (const std::exception& e) {
