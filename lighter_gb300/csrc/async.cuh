@@ -30,27 +30,50 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(bar)) : "memory");
 }
 
+// An arrival on the barrier at the same place in CTA `rank` of this cluster.
+__device__ __forceinline__ void mbar_arrive_rank(uint64_t* bar, uint32_t rank)
+{
+    asm volatile(
+        "{\n\t.reg .b32 a;\n\t"
+        "mapa.shared::cluster.u32 a, %0, %1;\n\t"
+        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [a];\n\t}" ::"r"(saddr(bar)),
+        "r"(rank)
+        : "memory");
+}
+
+// CLUSTER: arrivals by other CTAs of the cluster are acquired too.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity)
 {
     uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(saddr(bar)), "r"(parity)
-        : "memory");
+    if (CLUSTER)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(saddr(bar)), "r"(parity)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(saddr(bar)), "r"(parity)
+            : "memory");
     return ok != 0;
 }
 
 // Bounded wait for the phase of parity `parity`: false (and the error bit)
 // after `limit` SM clock cycles.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t* err, uint32_t bit,
                                           unsigned long long limit)
 {
-    if (mbar_try(bar, parity)) return true;
+    if (mbar_try<CLUSTER>(bar, parity)) return true;
     const long long t0 = clock64();
-    while (!mbar_try(bar, parity)) {
+    while (!mbar_try<CLUSTER>(bar, parity)) {
         if (clock64() - t0 > (long long) limit) {
             if (err) atomicOr(err, bit);
             return false;

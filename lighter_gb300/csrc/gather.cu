@@ -24,6 +24,7 @@
 //               128-row halves into two FP32 accumulators (columns 0 and 256)
 //   warps 2-5   epilogue: tcgen05.ld of the accumulators, partial sums of each
 //               row block written to a workspace slot
+// Wide split right-hand sides run on pairs of CTAs instead (cta_group::2, M=256).
 // k_combine then adds E and the slots of every row block in a fixed order
 // (deterministic) and writes B and the next bounce's X^T. Every mbarrier wait
 // is bounded: on expiry the kernel sets a bit of the error word, stops its
@@ -90,46 +91,87 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
         : "memory");
 }
 
+// The same into this CTA of a pair, completing on the barrier in its even CTA (an
+// address from mapa).
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint32_t even_bar, int x, int y)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];" ::"r"(
+            saddr(dst)),
+        "l"(map), "r"(even_bar), "r"(x), "r"(y)
+        : "memory");
+}
+
+__device__ __forceinline__ uint32_t even_cta_addr(const void* p)
+{
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(saddr(p)));
+    return a;
+}
+
 // Matrix descriptor of a K-major operand tile written by TMA with the swizzle
 // of its row length KB x 2 bytes: 128-byte rows (KB = 64, 128-byte swizzle) or
 // 64-byte rows (KB = 32, 64-byte swizzle), groups of 8 rows 8 x row bytes
 // apart. Advancing K by 16 elements inside a row adds 32 bytes to the start.
+// Only the low word depends on the address, and no offset inside shared memory
+// (below 256 KB) carries out of its 14 bits: a tile's descriptors are its low word
+// plus constants.
+__device__ __forceinline__ uint32_t sdesc_lo(uint32_t addr)
+{
+    return ((addr >> 4) & 0x3FFFu) | 1u << 16;   // start address >> 4; leading byte offset (unused for swizzled K-major)
+}
 template <int KB>
-__device__ __forceinline__ uint64_t sdesc(uint32_t addr)
+__device__ __forceinline__ uint64_t sdesc(uint32_t lo)
 {
     static_assert(KB == 64 || KB == 32, "stage k must be 64 or 32");
-    uint64_t d = 0;
-    d |= (uint64_t) ((addr >> 4) & 0x3FFFu);          // start address >> 4
-    d |= (uint64_t) 1u << 16;                          // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t) ((8u * KB * 2) >> 4) << 32;        // stride byte offset: 8 rows
-    d |= (uint64_t) 1u << 46;                          // descriptor version
-    d |= (uint64_t) (KB == 64 ? 2u : 4u) << 61;        // 128-byte or 64-byte swizzle
-    return d;
+    const uint32_t hi = ((8u * KB * 2) >> 4)          // stride byte offset: 8 rows
+                        | 1u << 14                    // descriptor version
+                        | (KB == 64 ? 2u : 4u) << 29; // 128-byte or 64-byte swizzle
+    return (uint64_t) hi << 32 | lo;
 }
 
 // Instruction descriptor of kind::f16: FP32 accumulator (bits 4-5 = 1), A and
 // B of format `fmt` (0 FP16, 1 BF16; bits 7-9 and 10-12), both K-major
 // (bits 15, 16 = 0), N >> 3 in bits 17-22, M >> 4 in bits 24-28.
-uint32_t idesc_f16(uint32_t fmt, uint32_t bn)
+uint32_t idesc_f16(uint32_t fmt, uint32_t m, uint32_t bn)
 {
-    return (1u << 4) | (fmt << 7) | (fmt << 10) | ((bn >> 3) << 17) | ((uint32_t) (BM >> 4) << 24);
+    return (1u << 4) | (fmt << 7) | (fmt << 10) | ((bn >> 3) << 17) | ((m >> 4) << 24);
 }
 
+// CTAS = 2: one product over the CTA pair, issued by its even CTA (see k_umma_gather).
+template <int CTAS>
 __device__ __forceinline__ void umma(uint32_t tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc)
 {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
-        : "memory");
+    if (CTAS == 2)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
+            : "memory");
 }
 
-// Arrives on `bar` once every tcgen05.mma issued so far by this thread completes.
-__device__ __forceinline__ void umma_commit(uint64_t* bar)
+// Arrives on `bar` (CTAS = 2: in the CTAs of `mask`) once every tcgen05.mma issued so far by
+// this thread completes.
+template <int CTAS>
+__device__ __forceinline__ void umma_commit(uint64_t* bar, uint16_t mask = 3)
 {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(saddr(bar))
-                 : "memory");
+    if (CTAS == 2)
+        asm volatile(
+            "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                saddr(bar)),
+            "h"(mask)
+            : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(saddr(bar))
+                     : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* v)
@@ -148,6 +190,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* v)
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// All threads of the block, or of the pair.
+template <int CTAS>
+__device__ __forceinline__ void group_sync()
+{
+    if (CTAS == 2) {
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+    } else __syncthreads();
+}
+
 // ----------------------------------------------------------------------------- tcgen05 gather
 
 struct UmmaArgs {
@@ -155,11 +207,10 @@ struct UmmaArgs {
     u32 n_rp;             // 256-row blocks
     u32 R, BN;            // right-hand sides, MMA N (multiple of 32, >= R)
     u32 stages, stage_bytes;
-    u32 mode;             // LTRG_REFINE_*
     u32 idesc;
     u32 max_slots;
     u32 kchunk;           // k blocks accumulated in TMEM before moving to the FP32 workspace (0: no limit)
-    const u32* rp_first;  // first CTA whose range touches each row block
+    const u32* rp_first;  // first range (CTA or pair) that touches each row block
     float* partial;       // [rp][slot][R][256]
     u32* err;
     unsigned long long wait_cycles;   // limit of every mbarrier wait (kWaitCycles)
@@ -167,7 +218,16 @@ struct UmmaArgs {
 };
 
 // KB: k per pipeline stage (a 64-wide work unit takes 64 / KB stages).
-template <int KB>
+//
+// CTAS = 2: a pair of CTAs (a cluster, on one pair of SMs) takes units of two row
+// blocks. Each holds the G tile of its own row block and half of the rows of the
+// X tile; the even CTA issues products with M = 256 (cta_group::2) that read both
+// CTAs' tiles and leave each CTA its own 128 rows x BN in its own tensor memory.
+// X, which every row block reads again, costs half the L2 reads and half the shared
+// memory, so the ring has twice the stages (figures at gather_plan).
+// Both CTAs' copies complete on the even CTA's `full`; commits arrive in both CTAs;
+// both epilogues arrive on the even CTA's `acce`.
+template <int KB, int CTAS, int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
     k_umma_gather(const __grid_constant__ CUtensorMap tmG, const __grid_constant__ CUtensorMap tmGl,
                   const __grid_constant__ CUtensorMap tmXh, const __grid_constant__ CUtensorMap tmXl, UmmaArgs a)
@@ -185,96 +245,128 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accf + 3);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint64_t total = (uint64_t) a.n_rp * a.nkb;
-    const uint64_t lo = (uint64_t) blockIdx.x * total / gridDim.x;
-    const uint64_t hi = (uint64_t) (blockIdx.x + 1) * total / gridDim.x;
-    const u32 b_bytes = a.BN * KB * 2;
-    const u32 off_gl = A_BYTES;
-    const u32 off_xh = a.mode == LTRG_REFINE_FULL ? 2 * A_BYTES : A_BYTES;
+    const u32 rank = CTAS == 2 ? blockIdx.x & 1u : 0u, range = blockIdx.x / CTAS;   // clusters are consecutive blocks
+    const uint64_t total = (uint64_t) ((a.n_rp + CTAS - 1) / CTAS) * a.nkb;   // a unit: CTAS row blocks x one k block
+    const uint64_t lo = (uint64_t) range * total / (gridDim.x / CTAS);
+    const uint64_t hi = (uint64_t) (range + 1) * total / (gridDim.x / CTAS);
+    const u32 n_units = (u32) (hi - lo);   // below 2^32: at most 8,192 row blocks x 32,768 k blocks
+    const u32 b_bytes = a.BN / CTAS * KB * 2;
+    constexpr u32 off_gl = A_BYTES;
+    constexpr u32 off_xh = MODE == LTRG_REFINE_FULL ? 2 * A_BYTES : A_BYTES;
     const u32 off_xl = off_xh + b_bytes;
-    const u32 tx_bytes = (a.mode == LTRG_REFINE_FULL ? 2 : 1) * A_BYTES + (a.mode >= LTRG_REFINE_RHS ? 2 : 1) * b_bytes;
+    const u32 tx_bytes = (MODE == LTRG_REFINE_FULL ? 2 : 1) * A_BYTES + (MODE >= LTRG_REFINE_RHS ? 2 : 1) * b_bytes;
 
     if (threadIdx.x == 0) {
         for (u32 s = 0; s < a.stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         mbar_init(accf, 1);
-        mbar_init(acce, 4);
+        mbar_init(acce, 4 * CTAS);
         mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(tmem_slot)),
-                     "r"(TMEM_COLS)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (CTAS == 2) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(tmem_slot)),
+                         "r"(TMEM_COLS)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(tmem_slot)),
+                         "r"(TMEM_COLS)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
-    __syncthreads();
+    group_sync<CTAS>();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
     if (warp == 0) {
         if (lane == 0) {
-            // producer: stage counter i runs over the units' stages
-            uint64_t i = 0;
+            // producer: stage s, whose use number has parity ph
+            u32 s = 0, ph = 0, used = 0, ru = (u32) (lo / a.nkb), kb = (u32) (lo % a.nkb);
+            const int rx = (int) (rank * a.BN / CTAS);   // this CTA's rows of X
+            const uint32_t full_even = CTAS == 2 ? even_cta_addr(full) : 0u;
             bool ok = true;
-            for (uint64_t u = a.issue ? lo : hi; u < hi && ok; ++u) {
-                for (int q = 0; q < SPU; ++q, ++i) {
-                    const u32 s = (u32) (i % a.stages);
-                    if (i >= a.stages &&
-                        !mbar_wait(&empty[s], (u32) ((i / a.stages) - 1) & 1u, a.err, kErrProducer, a.wait_cycles)) {
-                        ok = false;
-                        break;
-                    }
-                    const int kx = (int) ((u % a.nkb) * BK + q * KB), ry = (int) ((u / a.nkb) * ROWS);
+            for (u32 left = a.issue ? n_units : 0; left && ok; --left) {
+                for (int q = 0; q < SPU; ++q) {
+                    if (used == a.stages) {
+                        if (!mbar_wait(&empty[s], ph ^ 1u, a.err, kErrProducer, a.wait_cycles)) {
+                            ok = false;
+                            break;
+                        }
+                    } else ++used;
+                    const int kx = (int) (kb * BK + q * KB), ry = (int) ((ru * CTAS + rank) * ROWS);
                     unsigned char* st = base + (size_t) s * a.stage_bytes;
-                    mbar_expect_tx(&full[s], tx_bytes);
-                    tma_load_2d(st, &tmG, &full[s], kx, ry);
-                    if (a.mode == LTRG_REFINE_FULL) tma_load_2d(st + off_gl, &tmGl, &full[s], kx, ry);
-                    tma_load_2d(st + off_xh, &tmXh, &full[s], kx, 0);
-                    if (a.mode >= LTRG_REFINE_RHS) tma_load_2d(st + off_xl, &tmXl, &full[s], kx, 0);
+                    // the even CTA's barrier counts both CTAs' bytes; the odd CTA's copies cannot
+                    // run ahead into its next phase, since they wait for this one's products
+                    if (rank == 0) mbar_expect_tx(&full[s], CTAS * tx_bytes);
+                    auto load = [&](uint32_t off, const CUtensorMap* m, int x, int y) {
+                        if (CTAS == 2) tma_load_2d_pair(st + off, m, full_even + 8 * s, x, y);
+                        else tma_load_2d(st + off, m, &full[s], x, y);
+                    };
+                    load(0, &tmG, kx, ry);
+                    if (MODE == LTRG_REFINE_FULL) load(off_gl, &tmGl, kx, ry);
+                    load(off_xh, &tmXh, kx, rx);
+                    if (MODE >= LTRG_REFINE_RHS) load(off_xl, &tmXl, kx, rx);
+                    if (++s == a.stages) { s = 0; ph ^= 1u; }
                 }
+                if (++kb == a.nkb) { kb = 0; ++ru; }
             }
             // wait for the copies still in flight (complete already unless a wait above expired)
-            const uint64_t issued = i;
-            for (uint64_t j = issued > a.stages ? issued - a.stages : 0; j < issued; ++j)
-                if (!mbar_wait(&full[j % a.stages], (u32) (j / a.stages) & 1u, a.err, kErrDrain, a.wait_cycles)) break;
+            // the last `used` stages issued end at stage s, so stage t was last used in
+            // this round of the ring (t < s) or the one before
+            for (u32 t = 0; rank == 0 && t < used; ++t)
+                if (!mbar_wait(&full[t], t < s ? ph : ph ^ 1u, a.err, kErrDrain, a.wait_cycles)) break;
+            // in a pair, also for the issuer's last commits into this CTA; where they do not
+            // come, the odd CTA gives its own copies (microseconds at most) a millisecond or so
+            if (CTAS == 2)
+                for (u32 t = 0; t < used; ++t)
+                    if (!mbar_wait(&empty[t], t < s ? ph : ph ^ 1u, a.err, kErrDrain, a.wait_cycles)) {
+                        for (const long long t0 = clock64(); clock64() - t0 < 2000000;) {}
+                        break;
+                    }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // MMA issuer
-            uint64_t i = 0;
-            u32 seg = 0;
-            bool ok = true;
-            for (uint64_t u = lo; u < hi && ok; ++u) {
-                const u32 kb = (u32) (u % a.nkb);
-                const bool first = u == lo || kb == 0 || (a.kchunk && kb % a.kchunk == 0);
-                const bool last = u + 1 == hi || kb + 1 == a.nkb || (a.kchunk && (kb + 1) % a.kchunk == 0);
-                if (first && seg > 0 && !mbar_wait(acce, (seg - 1) & 1u, a.err, kErrMma, a.wait_cycles)) break;
-                for (int q = 0; q < SPU; ++q, ++i) {
-                    const u32 s = (u32) (i % a.stages);
-                    if (!mbar_wait(&full[s], (u32) (i / a.stages) & 1u, a.err, kErrMma, a.wait_cycles)) {
+        if (lane == 0 && rank == 0) {
+            // MMA issuer. One thread issues everything, so its own instructions count: no
+            // divisions, descriptors by adding constants (with a 64-bit remainder per unit and
+            // stage and descriptors built from addresses, a product of any width took 155
+            // cycles: 32,768 patches, 0.56 ms per sweep even for R = 3)
+            u32 s = 0, ph = 0, seg = 0, kb = (u32) (lo % a.nkb), kc = a.kchunk ? kb % a.kchunk : 0;
+            bool ok = true, first = true;
+            for (u32 left = n_units; left && ok; --left) {
+                const bool last = left == 1 || kb + 1 == a.nkb || (a.kchunk && kc + 1 == a.kchunk);
+                if (first && seg > 0 && !mbar_wait<CTAS == 2>(acce, (seg - 1) & 1u, a.err, kErrMma, a.wait_cycles)) break;
+                for (int q = 0; q < SPU; ++q) {
+                    if (!mbar_wait(&full[s], ph, a.err, kErrMma, a.wait_cycles)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t st = saddr(base + (size_t) s * a.stage_bytes);
+                    const uint32_t lg = sdesc_lo(saddr(base) + s * a.stage_bytes), lh = lg + (off_xh >> 4), ll = lg + (off_xl >> 4);
+                    uint32_t acc = first && q == 0 ? 0u : 1u;
+#pragma unroll
                     for (int k = 0; k < KB / UK; ++k) {
-                        const uint64_t bh = sdesc<KB>(st + off_xh + k * UK * 2);
-                        const uint64_t bl = sdesc<KB>(st + off_xl + k * UK * 2);
+                        const uint64_t bh = sdesc<KB>(lh + k * (UK * 2 / 16)), bl = sdesc<KB>(ll + k * (UK * 2 / 16));
+#pragma unroll
                         for (int h = 0; h < 2; ++h) {
-                            const uint32_t d = tmem + h * 256;
-                            const uint32_t ao = h * (BM * KB * 2) + k * UK * 2;
-                            const uint64_t ad = sdesc<KB>(st + ao);
-                            umma(d, ad, bh, a.idesc, (first && q == 0 && k == 0) ? 0u : 1u);
-                            if (a.mode >= LTRG_REFINE_RHS) umma(d, ad, bl, a.idesc, 1u);
-                            if (a.mode == LTRG_REFINE_FULL) umma(d, sdesc<KB>(st + off_gl + ao), bh, a.idesc, 1u);
+                            const uint32_t d = tmem + h * 256, ao = lg + h * (BM * KB * 2 / 16) + k * (UK * 2 / 16);
+                            umma<CTAS>(d, sdesc<KB>(ao), bh, a.idesc, acc);
+                            if (MODE >= LTRG_REFINE_RHS) umma<CTAS>(d, sdesc<KB>(ao), bl, a.idesc, 1u);
+                            if (MODE == LTRG_REFINE_FULL) umma<CTAS>(d, sdesc<KB>(ao + A_BYTES / 16), bh, a.idesc, 1u);
                         }
+                        acc = 1u;
                     }
-                    umma_commit(&empty[s]);
+                    umma_commit<CTAS>(&empty[s]);
+                    if (++s == a.stages) { s = 0; ph ^= 1u; }
                 }
-                if (ok && last) { umma_commit(accf); ++seg; }
+                if (ok && last) { umma_commit<CTAS>(accf); ++seg; }
+                first = last;
+                if (++kc == a.kchunk) kc = 0;
+                if (++kb == a.nkb) kb = kc = 0;
             }
-            umma_commit(done);
+            umma_commit<CTAS>(done, 1);
             mbar_wait(done, 0, a.err, kErrDrain, a.wait_cycles);
         }
     } else {
@@ -285,18 +377,19 @@ __global__ void __launch_bounds__(kThreads, 1)
         // first segment of a row block writes its workspace slot, later ones add to it.
         uint64_t u = lo;
         for (u32 seg = 0; u < hi; ++seg) {
-            const u32 rp = (u32) (u / a.nkb), kb = (u32) (u % a.nkb);
+            const u32 ru = (u32) (u / a.nkb), rp = ru * CTAS + rank, kb = (u32) (u % a.nkb);
             const u32 kend = a.kchunk ? min(a.nkb, (kb / a.kchunk + 1) * a.kchunk) : a.nkb;
             const bool fresh = u == lo || kb == 0;
-            u = min(hi, (uint64_t) rp * a.nkb + kend);
+            u = min(hi, (uint64_t) ru * a.nkb + kend);
             // every lane waits; the warp goes on only if all of them saw the phase, so the
             // .sync.aligned loads below always run converged
             const bool ok = mbar_wait(accf, seg & 1u, a.err, kErrEpilogue, a.wait_cycles);
             if (!__all_sync(0xffffffffu, ok)) break;
             tc_fence_after();
-            const u32 slot = blockIdx.x - __ldg(&a.rp_first[rp]);
+            const bool real = rp < a.n_rp;   // the odd row block of the last pair may not be one
+            const u32 slot = real ? range - __ldg(&a.rp_first[rp]) : 0u;
             float* P = a.partial + ((size_t) rp * a.max_slots + slot) * a.R * ROWS;
-            for (int h = 0; h < 2; ++h) {
+            for (int h = 0; h < 2 && real; ++h) {
                 const u32 row = h * BM + q * 32 + lane;
                 for (u32 c0 = 0; c0 < a.BN; c0 += 32) {
                     uint32_t v[32];
@@ -316,15 +409,23 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(acce);
+            if (lane == 0) {
+                if (rank == 0) mbar_arrive(acce);
+                else mbar_arrive_rank(acce, 0);
+            }
         }
     }
+    // nothing of the pair is in flight beyond this point: every copy and product was
+    // waited for (within the limit) by the CTA that issued it
     tc_fence_before();
-    __syncthreads();
+    group_sync<CTAS>();
     if (warp == 1) {
         __syncwarp();
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+        if (CTAS == 2)
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+        else
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
     }
 }
 
@@ -747,12 +848,38 @@ CUtensorMap make_map(const void* ptr, CUtensorMapDataType dt, u32 ld, u32 rows, 
     return m;
 }
 
-// k per pipeline stage of the tensor-core gather for a refine level. Measured
-// on GB300 (32,768 patches, R = 192): 64 for one and two products (0.388 and
-// 0.606 ms per contraction against 0.463 and 0.652 with 32); 32 for three
-// products, whose stages hold two G tiles and two X tiles (0.719 against
-// 0.738 ms; it also lets that mode take R = 256).
-u32 stage_k(int refine) { return refine == LTRG_REFINE_FULL ? 32u : 64u; }
+// How a product runs, from the refine level and the MMA N (measured on GB300, us per
+// product of 32,768 patches unless noted).
+//
+// k per stage: 64 for one and two products on single CTAs (R = 192: 360 and 538 against
+// 363 and 462 with 32, R = 3: 320 and 328 against 315 and 353; where 64 leaves two
+// stages, pairs are taken instead, below); 32 for three products, whose stages hold
+// two G tiles and two X tiles (R = 192: 691 against 746; it also lets that mode take
+// R = 256).
+//
+// Pairs of CTAs with split right-hand sides, where a single CTA has room for two stages
+// only (N > 160), from 16 units per SM on: R = 192, one CTA / pair: 538 / 430, 8,192
+// patches 46.0 / 41.9, 6,000 30.6 / 30.5, 4,096 20.8 / 22.8; R = 256: 675 / 547, 4,096
+// patches 25.5 / 27.2. With three stages or more both are the same at large sizes
+// (R = 144: 386 / 390) and a pair's start and end cost a microsecond or two at small
+// ones. A pair's stages are 32 wide (R = 192, 256: 430, 547; 64 wide 438, 565).
+struct GatherPlan {
+    bool pair;
+    u32 kb, stages, stage_bytes;
+};
+GatherPlan gather_plan(int refine, u32 bn, uint64_t units, int sm_count)
+{
+    auto stage = [&](u32 kb, u32 ctas) {
+        return (refine == LTRG_REFINE_FULL ? 2u : 1u) * ROWS * kb * 2 + (refine >= LTRG_REFINE_RHS ? 2u : 1u) * (bn / ctas) * kb * 2;
+    };
+    GatherPlan p;
+    p.kb = refine == LTRG_REFINE_FULL ? 32u : 64u;
+    p.pair = refine == LTRG_REFINE_RHS && 3 * stage(p.kb, 1) + kSmemExtra > (u32) kSmemLimit && units >= 16ull * (u32) sm_count;
+    if (p.pair) p.kb = 32;
+    p.stage_bytes = stage(p.kb, p.pair ? 2 : 1);
+    p.stages = std::min<u32>(kMaxStages, (kSmemLimit - kSmemExtra) / p.stage_bytes);
+    return p;
+}
 
 // Device buffer from the device's memory pool (which the bakes keep filled between
 // objects, see keep_pool_memory: mapping and unmapping a gather's matrices took
@@ -941,9 +1068,10 @@ struct ltrg_Gather {
     int g_exp = 0;                // G16 holds 2^g_exp G: max |G| maps below 2^14
     bool g16_has_lo = false;
     // stream-K schedule of the tcgen05 kernel (fixed by n and the SM count)
-    u32 n_rp = 0, nkb = 0, n_cta = 0, max_slots = 0;
+    u32 n_rp = 0, nkb = 0;
+    u32 n_ranges[2] = {}, max_slots[2] = {};   // stream-K ranges and most slots of a row block: single CTAs, pairs
     u32 kchunk = 0;               // k blocks per TMEM accumulation (0: whole range of a CTA)
-    DevBuf rp_tab;                // rp_first[n_rp], rp_cnt[n_rp]
+    DevBuf rp_tab;                // rp_first[n_rp], rp_cnt[n_rp] of single CTAs, then of pairs
     // solve scratch
     DevBuf partial, xh, xl, x32;
     DevBuf words;                 // [0] error word of the products, [1] largest emission
@@ -989,21 +1117,27 @@ struct ltrg_Gather {
     {
         n_rp = (n + ROWS - 1) / ROWS;
         nkb = ld / BK;
-        const uint64_t total = (uint64_t) n_rp * nkb;
-        n_cta = (u32) std::min<uint64_t>((uint64_t) sm_count, total);
-        std::vector<u32> first(n_rp, UINT32_MAX), cnt(n_rp, 0);
-        for (u32 c = 0; c < n_cta; ++c) {
-            const uint64_t lo = (uint64_t) c * total / n_cta, hi = (uint64_t) (c + 1) * total / n_cta;
-            if (hi <= lo) continue;
-            for (uint64_t rp = lo / nkb; rp <= (hi - 1) / nkb; ++rp) {
-                if (first[rp] == UINT32_MAX) first[rp] = c;
-                cnt[rp] = c - first[rp] + 1;
+        std::vector<u32> tab;
+        for (u32 ctas = 1; ctas <= 2; ++ctas) {
+            const uint64_t total = (uint64_t) ((n_rp + ctas - 1) / ctas) * nkb;
+            const u32 ranges = (u32) std::min<uint64_t>((uint64_t) sm_count / ctas, total);
+            std::vector<u32> first(n_rp, UINT32_MAX), cnt(n_rp, 0);
+            u32 most = 0;
+            for (u32 c = 0; c < ranges; ++c) {
+                const uint64_t lo = (uint64_t) c * total / ranges, hi = (uint64_t) (c + 1) * total / ranges;
+                if (hi <= lo) continue;
+                for (uint64_t ru = lo / nkb; ru <= (hi - 1) / nkb; ++ru)
+                    for (u32 rp = (u32) ru * ctas; rp < std::min<u32>(n_rp, ((u32) ru + 1) * ctas); ++rp) {
+                        if (first[rp] == UINT32_MAX) first[rp] = c;
+                        cnt[rp] = c - first[rp] + 1;
+                        most = std::max(most, cnt[rp]);
+                    }
             }
+            n_ranges[ctas - 1] = ranges;
+            max_slots[ctas - 1] = most;
+            tab.insert(tab.end(), first.begin(), first.end());
+            tab.insert(tab.end(), cnt.begin(), cnt.end());
         }
-        max_slots = 0;
-        for (u32 rp = 0; rp < n_rp; ++rp) max_slots = std::max(max_slots, cnt[rp]);
-        std::vector<u32> tab(first);
-        tab.insert(tab.end(), cnt.begin(), cnt.end());
         need(rp_tab, tab.size() * 4);
         GCK(cudaMemcpyAsync(rp_tab.p, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice, st));
         GCK(cudaStreamSynchronize(st));
@@ -1067,7 +1201,7 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
     };
     double ms_convert = 0, ms_gemm = 0, ms_bounces = 0;
     int stages = 0, products = 1;
-    int32_t ctas32 = 0;
+    int32_t ctas_run = 0;
     uint64_t bytes_bounce = 0;
 
     if (!tc) {
@@ -1092,7 +1226,7 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
         auto kern = tn == 6 ? k_sgemm_bounce<6> : tn == 4 ? k_sgemm_bounce<4> : k_sgemm_bounce<2>;
         const size_t sg_smem = (size_t) SGStages * (SGM + bn) * SGS * 4;
         GCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sg_smem));
-        ctas32 = (int32_t) sg_cta;
+        ctas_run = (int32_t) sg_cta;
         cudaEvent_t e0 = event();
         combine(false, bounces == 0);
         std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ge;
@@ -1114,10 +1248,11 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
     } else {
         const bool need_lo = refine == LTRG_REFINE_FULL;
         const u32 BN = std::max<u32>(32, (R + 31) / 32 * 32);
-        const u32 KB = stage_k(refine);
-        const u32 b_bytes = BN * KB * 2, a_bytes = ROWS * KB * 2;
-        const u32 stage_bytes = (need_lo ? 2 : 1) * a_bytes + (refine >= LTRG_REFINE_RHS ? 2 : 1) * b_bytes;
-        stages = std::min<int>(kMaxStages, (kSmemLimit - kSmemExtra) / (int) stage_bytes);
+        const GatherPlan plan = gather_plan(refine, BN, (uint64_t) n_rp * nkb, sm_count);
+        const bool pair = plan.pair;
+        const u32 KB = plan.kb, ctas = pair ? 2 : 1, slots_max = max_slots[pair];
+        const u32 stage_bytes = plan.stage_bytes;
+        stages = (int) plan.stages;
         if (stages < 2) throw std::runtime_error("tensor-core gather: stage does not fit in shared memory");
         const size_t smem = (size_t) stages * stage_bytes + kSmemExtra;
         products = 1 + (refine >= LTRG_REFINE_RHS) + (refine == LTRG_REFINE_FULL);
@@ -1126,7 +1261,7 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
         if (need_lo) need(G16lo, (size_t) n * ld * 2);
         need(xh, (size_t) BN * ld * 2);
         need(xl, (size_t) BN * ld * 2);
-        need(partial, (size_t) n_rp * max_slots * R * ROWS * 4);
+        need(partial, (size_t) n_rp * slots_max * R * ROWS * 4);
         begin();
         cudaEvent_t c0 = nullptr, c1 = nullptr;
         if (g16_kind != precision || (need_lo && !g16_has_lo)) {
@@ -1148,17 +1283,20 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
             precision == LTRG_F_FP16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
         const CUtensorMap mG = make_map(G16.p, dt, ld, n, ROWS, KB);
         const CUtensorMap mGl = make_map(need_lo ? G16lo.p : G16.p, dt, ld, n, ROWS, KB);
-        const CUtensorMap mXh = make_map(xh.p, dt, ld, BN, BN, KB);
-        const CUtensorMap mXl = make_map(xl.p, dt, ld, BN, BN, KB);
-        auto kern = KB == 64 ? k_umma_gather<64> : k_umma_gather<32>;
+        const CUtensorMap mXh = make_map(xh.p, dt, ld, BN, BN / ctas, KB);
+        const CUtensorMap mXl = make_map(xl.p, dt, ld, BN, BN / ctas, KB);
+        auto kern = refine == LTRG_REFINE_NONE   ? k_umma_gather<64, 1, LTRG_REFINE_NONE>
+                    : refine == LTRG_REFINE_FULL ? k_umma_gather<32, 1, LTRG_REFINE_FULL>
+                    : pair                       ? k_umma_gather<32, 2, LTRG_REFINE_RHS>
+                                                 : k_umma_gather<64, 1, LTRG_REFINE_RHS>;
         GCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
         UmmaArgs ua;
         ua.nkb = nkb; ua.n_rp = n_rp; ua.R = R; ua.BN = BN;
-        ua.stages = (u32) stages; ua.stage_bytes = stage_bytes; ua.mode = (u32) refine;
-        ua.idesc = idesc_f16(precision == LTRG_F_BF16 ? 1u : 0u, BN);
-        ua.max_slots = max_slots;
+        ua.stages = (u32) stages; ua.stage_bytes = stage_bytes;
+        ua.idesc = idesc_f16(precision == LTRG_F_BF16 ? 1u : 0u, BM * ctas, BN);
+        ua.max_slots = slots_max;
         ua.kchunk = kchunk;
-        ua.rp_first = rp_tab.as<u32>();
+        ua.rp_first = rp_tab.as<u32>() + (pair ? 2 * n_rp : 0);
         ua.partial = partial.as<float>();
         ua.err = d_err;
         ua.wait_cycles = kWaitCycles;
@@ -1168,7 +1306,19 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
             ua.wait_cycles = (unsigned long long) stall_us * 2000ull;
             stall_us = 0;
         }
-        const u32* rp_cnt = rp_tab.as<u32>() + n_rp;
+        const u32* rp_cnt = ua.rp_first + n_rp;
+        cudaLaunchConfig_t lc = {};
+        cudaLaunchAttribute la[1];
+        la[0].id = cudaLaunchAttributeClusterDimension;
+        la[0].val.clusterDim.x = ctas;
+        la[0].val.clusterDim.y = la[0].val.clusterDim.z = 1;
+        lc.gridDim = dim3(n_ranges[pair] * ctas);
+        lc.blockDim = dim3(kThreads);
+        lc.dynamicSmemBytes = smem;
+        lc.stream = s;
+        lc.attrs = la;
+        lc.numAttrs = 1;
+        ctas_run = (int32_t) lc.gridDim.x;
         // Up to one tile per SM, a block's own chain of slots is the time: one element per
         // thread, eight slots in flight (1,500 patches, R = 45, 26 slots: 7.8 us; four
         // elements and one slot 11.0, four and four 9.5). While the blocks of all tiles are
@@ -1181,7 +1331,7 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
         auto combine_as = [&](auto type, bool with_partial, bool last) {
             using T = decltype(type);
             (per == 1 ? k_combine<T, 1, 8> : slots == 4 ? k_combine<T, 4, 4> : k_combine<T, 4, 1>)<<<cg, dim3(32, 32 / per), 0, s>>>(
-                n, ld, R, BN, with_partial ? partial.as<float>() : nullptr, max_slots, rp_cnt, E, alb, last ? out : nullptr,
+                n, ld, R, BN, with_partial ? partial.as<float>() : nullptr, slots_max, rp_cnt, E, alb, last ? out : nullptr,
                 last ? nullptr : xh.as<T>(), (last || refine == LTRG_REFINE_NONE) ? nullptr : xl.as<T>(), g_exp, d_emax,
                 d_err);
             note_launch();
@@ -1195,7 +1345,7 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
         std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ge;
         for (int b = 0; b < bounces; ++b) {
             cudaEvent_t g0 = event();
-            kern<<<n_cta, kThreads, smem, s>>>(mG, mGl, mXh, mXl, ua); note_launch();
+            GCK(cudaLaunchKernelEx(&lc, kern, mG, mGl, mXh, mXl, ua)); note_launch();
             cudaEvent_t g1 = event();
             ge.push_back({g0, g1});
             GCK(cudaGetLastError());
@@ -1229,7 +1379,7 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
         stats->pairs = pairs;
         stats->tensor_cores = tc ? 1 : 0;
         stats->stages = stages;
-        stats->ctas = tc ? (int32_t) n_cta : ctas32;
+        stats->ctas = ctas_run;
         stats->products = tc ? products : 1;
     }
 }
