@@ -24,6 +24,7 @@
 #include <condition_variable>
 #include <memory>
 #include <mutex>
+#include <numeric>
 #include <thread>
 #include <cstring>
 #include <stdexcept>
@@ -57,12 +58,21 @@ void ck(cudaError_t e, const char* what, int line)
 constexpr int kThreads = 256;
 constexpr u32 kNoLoc = 0xffffffffu;
 
-// f(i) for i in [0, n) on up to 16 host threads taking items one at a time;
-// the first exception is rethrown after all threads end.
-template <class F>
-void parallel_items(int n, F&& f)
+// Host threads for `work` units of which a thread should have `per_thread` at least:
+// starting and joining one takes 20 to 30 us (room with 34 boxes and 16 threads for
+// each of two passes: 1.6 ms of its 3.9).
+inline int host_threads(size_t work, size_t per_thread, int cap)
 {
-    int nt = std::min({16, (int) std::max(1u, std::thread::hardware_concurrency()), n});
+    const int hw = (int) std::max(1u, std::thread::hardware_concurrency());
+    return std::max(1, (int) std::min<size_t>((size_t) std::min(cap, hw), work / per_thread));
+}
+
+// f(i) for i in [0, n) on nt host threads (this one among them) taking items one at a
+// time; the first exception is rethrown after all threads end.
+template <class F>
+void parallel_items(int n, int nt, F&& f)
+{
+    nt = std::min(nt, n);
     if (nt <= 1) {
         for (int i = 0; i < n; ++i) f(i);
         return;
@@ -70,19 +80,26 @@ void parallel_items(int n, F&& f)
     std::atomic<int> next(0);
     std::exception_ptr err;
     std::mutex mu;
-    std::vector<std::thread> th;
-    for (int t = 0; t < nt; ++t)
-        th.emplace_back([&]() {
-            for (int i = next++; i < n; i = next++) {
-                try {
-                    f(i);
-                } catch (...) {
-                    std::lock_guard<std::mutex> lk(mu);
-                    if (!err) err = std::current_exception();
-                }
+    auto run = [&]() {
+        for (int i = next++; i < n; i = next++) {
+            try {
+                f(i);
+            } catch (...) {
+                std::lock_guard<std::mutex> lk(mu);
+                if (!err) err = std::current_exception();
             }
-        });
-    for (auto& x : th) x.join();
+        }
+    };
+    std::vector<std::thread> th;
+    struct Join {   // also when a thread cannot be started
+        std::vector<std::thread>& th;
+        ~Join() { for (auto& x : th) if (x.joinable()) x.join(); }
+    };
+    {
+        Join join{th};
+        for (int t = 1; t < nt; ++t) th.emplace_back(run);
+        run();
+    }
     if (err) std::rethrow_exception(err);
 }
 
@@ -2001,44 +2018,67 @@ struct ClipPoly {
     int n = 0;
 };
 
-inline float axis_of(V3 p, int a) { return a == 0 ? p.x : (a == 1 ? p.y : p.z); }
+// The pieces found so far: arrays that grow ahead of what is written.
+struct RefOut {
+    std::vector<u32>& tri;
+    std::vector<float>& box;   // 6 per reference
+    size_t n = 0;
+    void add(u32 t, V3 mn, V3 mx)
+    {
+        if (n == tri.size()) {
+            tri.resize(2 * n + 64);
+            box.resize(6 * (2 * n + 64));
+        }
+        float* b = &box[6 * n];
+        b[0] = mn.x; b[1] = mn.y; b[2] = mn.z;
+        b[3] = mx.x; b[4] = mx.y; b[5] = mx.z;
+        tri[n++] = t;
+    }
+};
 
-void clip_half(const ClipPoly& in, int axis, float c, bool below, ClipPoly& out)
+// Both halves of `in` at coordinate AXIS = c; a cut edge gives both the same point.
+template <int AXIS>
+void clip_halves(const ClipPoly& in, float c, ClipPoly& lo, ClipPoly& hi)
 {
-    out.n = 0;
+    auto at = [](const V3& p) { return AXIS == 0 ? p.x : AXIS == 1 ? p.y : p.z; };
+    lo.n = hi.n = 0;
+    V3 a = in.v[0];
+    float da = at(a) - c;
     for (int i = 0; i < in.n; ++i) {
-        V3 a = in.v[i], b = in.v[(i + 1) % in.n];
-        float da = axis_of(a, axis) - c, db = axis_of(b, axis) - c;
-        bool ia = below ? da <= 0 : da >= 0, ib = below ? db <= 0 : db >= 0;
-        if (ia && out.n < 24) out.v[out.n++] = a;
-        if (ia != ib && out.n < 24) {
+        const V3 b = in.v[i + 1 < in.n ? i + 1 : 0];
+        const float db = at(b) - c;
+        const bool la = da <= 0, lb = db <= 0, ha = da >= 0, hb = db >= 0;
+        if (la && lo.n < 24) lo.v[lo.n++] = a;
+        if (ha && hi.n < 24) hi.v[hi.n++] = a;
+        if (la != lb || ha != hb) {
             float t = da / (da - db);
             V3 p = a + (b - a) * t;
-            // pin the cut coordinate on the plane
-            if (axis == 0) p.x = c; else if (axis == 1) p.y = c; else p.z = c;
-            out.v[out.n++] = p;
+            (AXIS == 0 ? p.x : AXIS == 1 ? p.y : p.z) = c;   // pinned on the plane
+            if (la != lb && lo.n < 24) lo.v[lo.n++] = p;
+            if (ha != hb && hi.n < 24) hi.v[hi.n++] = p;
         }
+        a = b;
+        da = db;
     }
 }
 
-void split_ref(const ClipPoly& p, float limit, int depth, u32 tri, std::vector<u32>& ref_tri, std::vector<float>& ref_box)
+void split_ref(const ClipPoly& p, float limit, int depth, u32 tri, RefOut& out)
 {
     V3 mn = splat(FLT_MAX), mx = splat(-FLT_MAX);
     for (int i = 0; i < p.n; ++i) { mn = vmin(mn, p.v[i]); mx = vmax(mx, p.v[i]); }
     V3 e = mx - mn;
     int axis = (e.x >= e.y && e.x >= e.z) ? 0 : (e.y >= e.z ? 1 : 2);
-    float ext = axis_of(e, axis);
+    float ext = axis == 0 ? e.x : (axis == 1 ? e.y : e.z);
     if (ext <= limit || depth >= 12 || p.n < 3) {
-        ref_tri.push_back(tri);
-        ref_box.insert(ref_box.end(), {mn.x, mn.y, mn.z, mx.x, mx.y, mx.z});
+        out.add(tri, mn, mx);
         return;
     }
-    float c = (axis_of(mn, axis) + axis_of(mx, axis)) * 0.5f;
     ClipPoly lo, hi;
-    clip_half(p, axis, c, true, lo);
-    clip_half(p, axis, c, false, hi);
-    if (lo.n) split_ref(lo, limit, depth + 1, tri, ref_tri, ref_box);
-    if (hi.n) split_ref(hi, limit, depth + 1, tri, ref_tri, ref_box);
+    if (axis == 0) clip_halves<0>(p, (mn.x + mx.x) * 0.5f, lo, hi);
+    else if (axis == 1) clip_halves<1>(p, (mn.y + mx.y) * 0.5f, lo, hi);
+    else clip_halves<2>(p, (mn.z + mx.z) * 0.5f, lo, hi);
+    if (lo.n) split_ref(lo, limit, depth + 1, tri, out);
+    if (hi.n) split_ref(hi, limit, depth + 1, tri, out);
 }
 
 // References for all triangles; the split limit is four times the median
@@ -2066,24 +2106,35 @@ void build_refs(const std::vector<float>& xyz, std::vector<u32>& ref_tri, std::v
     }
     ref_tri.clear();
     ref_box.clear();
-    ref_tri.reserve(n);
-    ref_box.reserve(6 * n);
+    ref_tri.resize(n);
+    ref_box.resize(6 * n);
+    RefOut out{ref_tri, ref_box};
     for (size_t i = 0; i < n; ++i) {
         const float* q = &xyz[9 * i];
+        const V3 a = mk(q[0], q[1], q[2]), b = mk(q[3], q[4], q[5]), c = mk(q[6], q[7], q[8]);
+        const V3 mn = vmin(vmin(vmin(splat(FLT_MAX), a), b), c), mx = vmax(vmax(vmax(splat(-FLT_MAX), a), b), c), e = mx - mn;
+        if (e.x <= limit && e.y <= limit && e.z <= limit) {   // most triangles: what split_ref finds for them
+            out.add((u32) i, mn, mx);
+            continue;
+        }
         ClipPoly p;
         p.n = 3;
-        p.v[0] = mk(q[0], q[1], q[2]);
-        p.v[1] = mk(q[3], q[4], q[5]);
-        p.v[2] = mk(q[6], q[7], q[8]);
-        split_ref(p, limit, 0, (u32) i, ref_tri, ref_box);
+        p.v[0] = a;
+        p.v[1] = b;
+        p.v[2] = c;
+        split_ref(p, limit, 0, (u32) i, out);
     }
-    for (int c = 0; c < 3; ++c) { cmin[c] = FLT_MAX; cmax[c] = -FLT_MAX; }
-    for (size_t r = 0; r < ref_tri.size(); ++r)
+    ref_tri.resize(out.n);
+    ref_box.resize(6 * out.n);
+    // bounds of the boxes' centres (a NaN bounds nothing)
+    float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+    for (size_t r = 0; r < out.n; ++r)
         for (int c = 0; c < 3; ++c) {
-            float m = (ref_box[6 * r + c] + ref_box[6 * r + 3 + c]) * 0.5f;
-            cmin[c] = fminf(cmin[c], m);
-            cmax[c] = fmaxf(cmax[c], m);
+            const float m = (ref_box[6 * r + c] + ref_box[6 * r + 3 + c]) * 0.5f;
+            lo[c] = m < lo[c] ? m : lo[c];
+            hi[c] = m > hi[c] ? m : hi[c];
         }
+    for (int c = 0; c < 3; ++c) { cmin[c] = lo[c]; cmax[c] = hi[c]; }
 }
 
 // Gaussian taps (Generate_Gaussian_Kernel, lighter_math.cpp:357-365), on the
@@ -2475,7 +2526,7 @@ void run_bake(ltr_Scene* S)
     for (int i = 0; i < n_inst; ++i)
         vert_off[i + 1] = vert_off[i] + (S->insts[i]->container ? 0 : S->insts[i]->mesh->pos.size());
     std::unique_ptr<float[]> verts(new float[kVert * std::max<size_t>(vert_off[n_inst], 1)]);
-    parallel_items(n_inst - 1, [&](int k) { prexform(S, S->insts[k + 1], verts.get() + kVert * vert_off[k + 1]); });
+    parallel_items(n_inst - 1, host_threads(vert_off[n_inst], 1024, 16), [&](int k) { prexform(S, S->insts[k + 1], verts.get() + kVert * vert_off[k + 1]); });
     check_abort(S);
 
     // ---- host: triangle soup of shadow parts (Job_ColInfo) + instance boxes
@@ -2488,7 +2539,9 @@ void run_bake(ltr_Scene* S)
     };
     std::vector<InstSoup> soup(n_inst);
     std::vector<float> inst_box(6 * n_inst);
-    parallel_items(n_inst, [&](int i) {
+    size_t n_index = 0;
+    for (HostInst* mi : S->insts) n_index += mi->container ? 0 : mi->mesh->idx.size();
+    parallel_items(n_inst, host_threads(n_index, 3072, 16), [&](int i) {
         HostInst* mi = S->insts[i];
         InstSoup& o = soup[i];
         V3 bmn = splat(FLT_MAX), bmx = splat(-FLT_MAX);
@@ -2498,14 +2551,13 @@ void run_bake(ltr_Scene* S)
                 if (!p.shadow) continue;
                 const V3* vb = &mi->vpos[p.voff];
                 const u32* ib = &me->idx[p.ioff];
+                o.xyz.reserve(o.xyz.size() + 3 * (size_t) p.icount);
                 for (u32 t = 0; t < p.icount; t += 3) {
                     V3 P1 = vb[ib[t]], P2 = vb[ib[t + 1]], P3 = vb[ib[t + 2]];
                     if (near_zero(cross(P2 - P1, P3 - P1))) continue;   // Triangle::CheckIsUseful
                     const V3 ps[3] = {P1, P2, P3};
-                    for (const V3& q : ps) {
-                        o.xyz.push_back(q.x); o.xyz.push_back(q.y); o.xyz.push_back(q.z);
-                        bmn = vmin(bmn, q); bmx = vmax(bmx, q);
-                    }
+                    for (const V3& q : ps) { bmn = vmin(bmn, q); bmx = vmax(bmx, q); }
+                    o.xyz.insert(o.xyz.end(), {P1.x, P1.y, P1.z, P2.x, P2.y, P2.z, P3.x, P3.y, P3.z});
                     float cx = (P1.x + P2.x + P3.x) * (1.0f / 3.0f), cy = (P1.y + P2.y + P3.y) * (1.0f / 3.0f),
                           cz = (P1.z + P2.z + P3.z) * (1.0f / 3.0f);
                     o.smin[0] = fminf(o.smin[0], cx); o.smin[1] = fminf(o.smin[1], cy); o.smin[2] = fminf(o.smin[2], cz);
@@ -2530,10 +2582,9 @@ void run_bake(ltr_Scene* S)
             const u32 nt_i = (u32) (o.xyz.size() / 9);
             tri_xyz.insert(tri_xyz.end(), o.xyz.begin(), o.xyz.end());
             const u32 meta = (u32) i | (S->insts[i]->shadow ? kOccluderBit : 0u);
-            for (u32 t = 0; t < nt_i; ++t) {
-                tri_meta.push_back(meta);
-                tri_local.push_back(t);
-            }
+            tri_meta.insert(tri_meta.end(), nt_i, meta);
+            tri_local.resize(tri_local.size() + nt_i);
+            std::iota(tri_local.end() - nt_i, tri_local.end(), 0u);
             for (int c = 0; c < 3; ++c) {
                 smin[c] = fminf(smin[c], o.smin[c]);
                 smax[c] = fmaxf(smax[c], o.smax[c]);
@@ -2573,18 +2624,18 @@ void run_bake(ltr_Scene* S)
     std::thread reftree_thread([&]() {
         try {
             std::vector<RefTree> rtrees(n_inst);
-            {
-                std::vector<std::thread> pool;
-                std::atomic<int> next(1);
-                int nth = std::max(1, std::min({8, (int) std::thread::hardware_concurrency(), n_inst - 1}));
-                for (int t = 0; t < nth; ++t)
-                    pool.emplace_back([&]() {
-                        for (int i = next++; i < n_inst; i = next++)
-                            build_ref_tree(tri_xyz.data() + 9 * (size_t) inst_tri_off[i],
-                                           (size_t) (inst_tri_off[i + 1] - inst_tri_off[i]), rtrees[i]);
-                    });
-                for (auto& th : pool) th.join();
+            parallel_items(n_inst - 1, host_threads((size_t) n_tris, 256, 8), [&](int k) {
+                const int i = k + 1;
+                build_ref_tree(tri_xyz.data() + 9 * (size_t) inst_tri_off[i],
+                               (size_t) (inst_tri_off[i + 1] - inst_tri_off[i]), rtrees[i]);
+            });
+            size_t all_nodes = 0, all_items = 0;
+            for (const RefTree& t : rtrees) {
+                all_nodes += t.nodes.size();
+                all_items += t.items.size();
             }
+            ref_nodes.reserve(2 * all_nodes);
+            ref_items.reserve(all_items);
             for (int i = 0; i < n_inst; ++i) {
                 fix_box[2 * i] = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.0f);
                 fix_box[2 * i + 1] = make_float4(-3.0e38f, -3.0e38f, -3.0e38f, 0.0f);

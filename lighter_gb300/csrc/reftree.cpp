@@ -59,22 +59,22 @@ struct Builder {
         Box nb = {mn, mx};
         float nvol = volume(nb);
         if (n > 4 && depth < 16) {
-            int nsplit = 0;
+            std::vector<int32_t> self, split;
+            split.reserve(n);
             V3 smn = splat(FLT_MAX), smx = splat(-FLT_MAX);
             for (size_t i = 0; i < n; ++i) {
                 const Box& b = boxes[ids[i]];
-                if (volume(b) * 3 < nvol) { nsplit++; smn = vmin(smn, b.mn); smx = vmax(smx, b.mx); }
+                if (volume(b) * 3 < nvol) {
+                    split.push_back(ids[i]);
+                    smn = vmin(smn, b.mn);
+                    smx = vmax(smx, b.mx);
+                } else self.push_back(ids[i]);
             }
             V3 ss = smx - smn;
             V3 axis = mk(0, 0, 1);
             if (ss.x > ss.y && ss.x > ss.z) axis = mk(1, 0, 0);
             else if (ss.y > ss.x && ss.y > ss.z) axis = mk(0, 1, 0);
-            if (nsplit >= 4) {
-                std::vector<int32_t> self, split;
-                for (size_t i = 0; i < n; ++i) {
-                    if (volume(boxes[ids[i]]) * 3 < nvol) split.push_back(ids[i]);
-                    else self.push_back(ids[i]);
-                }
+            if (split.size() >= 4) {
                 if (!self.empty()) emit(node, self.data(), self.size());
                 // the keys are the values the comparison dot(axis, centre(a)) < dot(axis,
                 // centre(b)) would compute, so std::sort sees the same comparisons;
