@@ -537,14 +537,18 @@ __global__ void __launch_bounds__(1024 / PER) k_combine(u32 n, u32 ld, u32 R, u3
 
 // ----------------------------------------------------------------------------- FP32 SIMT gather
 
-// Partial sums of G X for FP32 (G n x n, row stride ldg a multiple of 4; X^T rows
-// of ldx floats, zero past n and past R). Bound by the FP32 pipes (G streams at a
-// fifth of HBM's rate), so the shape serves the multiply-adds:
-//  * both operands lie k-contiguous in shared memory (no transposition on the way
-//    in); a thread owns 16 rows ty + 8 i and TN columns tx + 16 j and reads four k at a
-//    time, 16 + TN 16-byte loads for 64 TN multiply-adds. A warp spans 4 x 8 threads,
-//    so with rows padded to 36 floats its loads touch 4 (G) or 8 (X) different rows
-//    on different banks.
+// Partial sums of G X for FP32 (G n x n, row stride ldg a multiple of 4; X rows of ldr
+// floats, zero past n and past R). Bound by the FP32 pipes (G streams at a fifth of
+// HBM's rate), so the shape serves the multiply-adds:
+//  * G lies k-contiguous in shared memory, X as it is, k by k (no transposition on the
+//    way in); a thread owns 16 rows ty + 8 i and TN columns, four neighbours 4 tx .. of
+//    each 64 and two of the last 32, and reads four k at a time, 16 + 8 loads of up to 16
+//    bytes for 384 multiply-adds (TN = 6). A warp spans 4 x 8 threads, so with G's
+//    rows padded to 36 floats its loads touch 4 rows on different banks, and 128
+//    contiguous bytes of X. Neighbouring columns also keep an X value's register
+//    bank the same for every k, so accumulators can sit in the other: with X
+//    k-contiguous too, half the issue slots lost were register conflicts
+//    (dispatch stalls 0.48 per instruction against 0.21, issue 73% against 79%).
 //  * 128 x (16 TN) tiles, k blocks of 32 in three cp.async stages, 128 threads, two
 //    blocks per SM.
 //  * the (tile, k block) units are cut into equal contiguous ranges, one per
@@ -552,18 +556,19 @@ __global__ void __launch_bounds__(1024 / PER) k_combine(u32 n, u32 ld, u32 R, u3
 //    sums of each tile it touches into its slot of that tile and k_combine32 adds
 //    the slots in order (deterministic, and shorter sums than one range of n).
 // TN by R (sgemm_tn): the least padding wins, with a charge per tile for G's re-read.
-// Measured, n = 8192: R = 96 1541 -> 262 us a bounce (50 TFLOP/s; the 128 x 192 tile on
-// 64 blocks before), R = 192 515 us. Tried: fma.rn.f32x2 on k pairs 46 TFLOP/s (its
-// 64-bit operands cost the register ports what it saves in issue slots); 8 x 6 and
-// 8 x 12 per thread 47 and 49.
+// Measured, n = 8192: R = 96 1541 -> 254 us a bounce with both operands k-contiguous and
+// 241 now (54 TFLOP/s; the 128 x 192 tile on 64 blocks at first), R = 192 515 -> 472.
+// Tried: fma.rn.f32x2 on column pairs 252 and 496 (its 64-bit operands cost the
+// register ports what it saves in issue slots), on k pairs 46 TFLOP/s; 8 x 6 and 8 x 12
+// per thread 47 and 49.
 constexpr int SGM = 128, SGK = 32, SGS = SGK + 4, SGStages = 3, SGThreads = 128, SGBlocksPerSM = 2;
 
 struct SgemmArgs {
-    u32 n, ldg, ldx, nkb;     // rows, strides of G and X^T, k blocks
+    u32 n, ldg, ldr, nkb;     // rows, strides of G and X, k blocks
     u32 tiles_n, max_slots;
     uint64_t total;           // (tile, k block) units
     const float* G;
-    const float* XT;
+    const float* X;           // [k][ldr], zero rows up to nkb SGK
     float* partial;           // [tile][slot][SGM][16 TN]
 };
 
@@ -583,7 +588,7 @@ __device__ __forceinline__ float f4at(const float4& v, int k) { return k == 0 ? 
 template <int TN>
 __global__ void __launch_bounds__(SGThreads, SGBlocksPerSM) k_sgemm_bounce(SgemmArgs a)
 {
-    constexpr int BN = 16 * TN, TM = SGM / 8, STAGE = (SGM + BN) * SGS, CG = SGM / 16, CX = BN / 16;
+    constexpr int BN = 16 * TN, TM = SGM / 8, STAGE = SGM * SGS + SGK * BN, CG = SGM / 16;
     extern __shared__ __align__(16) float sm[];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int ty = (w >> 1) * 4 + (lane >> 3), tx = (w & 1) * 8 + (lane & 7);
@@ -594,6 +599,13 @@ __global__ void __launch_bounds__(SGThreads, SGBlocksPerSM) k_sgemm_bounce(Sgemm
     const float* gp[CG];
     bool gin[CG];
     const float* xp;
+    // X rows of BN floats: chunks tid + 128 t of the stage's SGK x BN / 4
+    u32 xoff[TN];
+#pragma unroll
+    for (int t = 0; t < TN; ++t) {
+        const u32 c = tid + SGThreads * t;
+        xoff[t] = c / (BN / 4) * a.ldr + c % (BN / 4) * 4;
+    }
     auto seek = [&]() {
         const u32 m0 = ft / a.tiles_n * SGM, n0 = ft % a.tiles_n * BN;
 #pragma unroll
@@ -602,11 +614,12 @@ __global__ void __launch_bounds__(SGThreads, SGBlocksPerSM) k_sgemm_bounce(Sgemm
             gin[t] = m < a.n;
             gp[t] = a.G + (gin[t] ? (size_t) m * a.ldg : 0) + fk * SGK + cc;
         }
-        xp = a.XT + (size_t) (n0 + cr) * a.ldx + fk * SGK + cc;
+        xp = a.X + (size_t) fk * SGK * a.ldr + n0;
     };
     seek();
     auto fetch = [&](int stage) {
         float* S = sm + stage * STAGE + cr * SGS + cc;
+        float* SX = sm + stage * STAGE + SGM * SGS + 4 * tid;
         const bool kin = fk * SGK + cc < a.ldg;
 #pragma unroll
         for (int t = 0; t < CG; ++t) {
@@ -614,14 +627,16 @@ __global__ void __launch_bounds__(SGThreads, SGBlocksPerSM) k_sgemm_bounce(Sgemm
             gp[t] += SGK;
         }
 #pragma unroll
-        for (int t = 0; t < CX; ++t) cp16(S + (SGM + 16 * t) * SGS, xp + (size_t) (16 * t) * a.ldx, true);
-        xp += SGK;
+        for (int t = 0; t < TN; ++t) cp16(SX + 4 * SGThreads * t, xp + xoff[t], true);
+        xp += (size_t) SGK * a.ldr;
         if (++fk == a.nkb) {
             fk = 0;
             ++ft;
             seek();
         }
     };
+    // this thread's column j of the tile: four and two neighbouring ones
+    auto col = [&](int j) { return j < (TN & ~3) ? 16 * (j & ~3) + 4 * tx + (j & 3) : 16 * (TN & ~3) + 2 * tx + (j & 1); };
     float acc[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
@@ -640,19 +655,29 @@ __global__ void __launch_bounds__(SGThreads, SGBlocksPerSM) k_sgemm_bounce(Sgemm
         if (u + SGStages - 1 < hi) fetch(stage == 0 ? SGStages - 1 : stage - 1);
         asm volatile("cp.async.commit_group;" ::: "memory");
         const float* As = sm + stage * STAGE + ty * SGS;
-        const float* Bs = sm + stage * STAGE + (SGM + tx) * SGS;
-#pragma unroll 2
+        const float* Bs = sm + stage * STAGE + SGM * SGS;
+#pragma unroll 4
         for (int k = 0; k < SGK; k += 4) {
-            float4 b[TN];
+            float b[4][TN];
 #pragma unroll
-            for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const float4*>(Bs + 16 * j * SGS + k);
+            for (int h = 0; h < 4; ++h) {
+#pragma unroll
+                for (int j = 0; j + 4 <= TN; j += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(Bs + (k + h) * BN + 16 * j + 4 * tx);
+                    b[h][j] = v.x; b[h][j + 1] = v.y; b[h][j + 2] = v.z; b[h][j + 3] = v.w;
+                }
+                if (TN % 4) {
+                    const float2 v = *reinterpret_cast<const float2*>(Bs + (k + h) * BN + 16 * (TN & ~3) + 2 * tx);
+                    b[h][TN - 2] = v.x; b[h][TN - 1] = v.y;
+                }
+            }
 #pragma unroll
             for (int i = 0; i < TM; ++i) {
                 const float4 av = *reinterpret_cast<const float4*>(As + 8 * i * SGS + k);
 #pragma unroll
                 for (int h = 0; h < 4; ++h)
 #pragma unroll
-                    for (int j = 0; j < TN; ++j) acc[i][j] = __fmaf_rn(f4at(av, h), f4at(b[j], h), acc[i][j]);
+                    for (int j = 0; j < TN; ++j) acc[i][j] = __fmaf_rn(f4at(av, h), b[h][j], acc[i][j]);
             }
         }
         stage = stage + 1 == SGStages ? 0 : stage + 1;
@@ -664,7 +689,7 @@ __global__ void __launch_bounds__(SGThreads, SGBlocksPerSM) k_sgemm_bounce(Sgemm
             for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < TN; ++j) {
-                    P[(ty + 8 * i) * BN + tx + 16 * j] = acc[i][j];
+                    P[(ty + 8 * i) * BN + col(j)] = acc[i][j];
                     acc[i][j] = 0.0f;
                 }
             ck = 0;
@@ -673,44 +698,38 @@ __global__ void __launch_bounds__(SGThreads, SGBlocksPerSM) k_sgemm_bounce(Sgemm
     }
 }
 
-// One 32 (patches) x 32 (right-hand sides) tile of a bounce: B = E + the tile's
-// slots in order (no slots: B = E), and the next X^T[r][j] = albedo_j(r mod 3) B,
-// zero for j >= n or r >= R. B_out and xt may be null (not wanted).
-__global__ void __launch_bounds__(256) k_combine32(u32 n, u32 ldx, u32 R, u32 BN, u32 tiles_n, u32 nkb, uint64_t total,
+// A bounce's sums: B = E + the tile's slots in order (no slots: B = E), and the next
+// X[j][r] = albedo_j(r mod 3) B (rows of ldr), zero for j >= n or r >= R. B_out and x
+// may be null (not wanted). 32 right-hand sides x 8 patches per block.
+__global__ void __launch_bounds__(256) k_combine32(u32 n, u32 ldx, u32 ldr, u32 R, u32 BN, u32 tiles_n, u32 nkb, uint64_t total,
                                                    u32 n_cta, u32 max_slots, const float* __restrict__ partial,
                                                    const float* __restrict__ E, const float* __restrict__ albedo,
-                                                   float* __restrict__ B_out, float* __restrict__ xt)
+                                                   float* __restrict__ B_out, float* __restrict__ x_out)
 {
-    __shared__ float tile[32][33];
-    const u32 j0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    // 32 divides the tile's rows and its BN columns: one product tile for the block
-    const u32 t = j0 / SGM * tiles_n + r0 / BN;
-    u32 cnt = 0;
-    if (partial && j0 < n)
-        cnt = range_of((uint64_t) (t + 1) * nkb - 1, total, n_cta) - range_of((uint64_t) t * nkb, total, n_cta) + 1;
-    const float* P = partial ? partial + (size_t) t * max_slots * (SGM * BN) + (size_t) (j0 % SGM) * BN + r0 % BN + tx : nullptr;
-    const u32 r = r0 + tx;
+    const u32 j = blockIdx.x * 8 + threadIdx.y, r0 = blockIdx.y * 32, r = r0 + threadIdx.x;
+    float x = 0.0f;
+    if (j < n && r < R) {
+        const float e = __ldg(&E[(size_t) j * R + r]), al = __ldg(&albedo[3 * j + r % 3]);
+        float v = 0.0f;
+        if (partial) {
+            // 8 divides the tile's rows and 32 its BN columns: one product tile for the block
+            const u32 t = j / SGM * tiles_n + r0 / BN;
+            const u32 cnt = range_of((uint64_t) (t + 1) * nkb - 1, total, n_cta) - range_of((uint64_t) t * nkb, total, n_cta) + 1;
+            const float* P = partial + (size_t) t * max_slots * (SGM * BN) + (size_t) (j % SGM) * BN + r % BN;
+            for (u32 s = 0; s < cnt; s += 4) {   // four slots in flight
+                float q[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const u32 k = ty + 8 * i, j = j0 + k;
-        float x = 0.0f;
-        if (j < n && r < R) {
-            float v = 0.0f;
-            for (u32 s = 0; s < cnt; ++s) v += __ldg(&P[(size_t) s * (SGM * BN) + (size_t) k * BN]);
-            const float b = E[(size_t) j * R + r] + v;
-            if (B_out) B_out[(size_t) j * R + r] = b;
-            x = albedo[3 * j + r % 3] * b;
+                for (u32 u = 0; u < 4; ++u) q[u] = s + u < cnt ? __ldg(&P[(size_t) (s + u) * (SGM * BN)]) : 0.0f;
+#pragma unroll
+                for (u32 u = 0; u < 4; ++u)
+                    if (s + u < cnt) v += q[u];
+            }
         }
-        tile[k][tx] = x;
+        const float b = e + v;
+        if (B_out) B_out[(size_t) j * R + r] = b;
+        x = al * b;
     }
-    if (!xt) return;
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const u32 rr = r0 + ty + 8 * i, j = j0 + tx;
-        if (j < ldx) xt[(size_t) rr * ldx + j] = tile[tx][ty + 8 * i];
-    }
+    if (x_out && j < ldx) x_out[(size_t) j * ldr + r] = x;
 }
 
 // Column groups of 16 per tile (TN of k_sgemm_bounce) for R right-hand sides: the
@@ -1215,16 +1234,17 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
         need(partial, (size_t) tiles_m * tiles_n * slots * SGM * bn * 4);
         need(x32, (size_t) tiles_n * bn * ldx * 4);
         begin();
-        const dim3 cb(32, 8), cg((ldx + 31) / 32, tiles_n * bn / 32);
+        const u32 ldr = tiles_n * bn;
+        const dim3 cb(32, 8), cg((ldx + 7) / 8, ldr / 32);
         auto combine = [&](bool with_partial, bool last) {
-            k_combine32<<<cg, cb, 0, s>>>(n, ldx, R, bn, tiles_n, skb, total, sg_cta, slots,
+            k_combine32<<<cg, cb, 0, s>>>(n, ldx, ldr, R, bn, tiles_n, skb, total, sg_cta, slots,
                                           with_partial ? partial.as<float>() : nullptr, E, alb, last ? out : nullptr,
                                           last ? nullptr : x32.as<float>()); note_launch();
             GCK(cudaGetLastError());
         };
-        const SgemmArgs sa{n, ldg, ldx, skb, tiles_n, slots, total, G32.as<float>(), x32.as<float>(), partial.as<float>()};
+        const SgemmArgs sa{n, ldg, ldr, skb, tiles_n, slots, total, G32.as<float>(), x32.as<float>(), partial.as<float>()};
         auto kern = tn == 6 ? k_sgemm_bounce<6> : tn == 4 ? k_sgemm_bounce<4> : k_sgemm_bounce<2>;
-        const size_t sg_smem = (size_t) SGStages * (SGM + bn) * SGS * 4;
+        const size_t sg_smem = (size_t) SGStages * (SGM * SGS + SGK * bn) * 4;
         GCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sg_smem));
         ctas_run = (int32_t) sg_cta;
         cudaEvent_t e0 = event();
