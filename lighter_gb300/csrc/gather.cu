@@ -459,13 +459,15 @@ __device__ __forceinline__ int x_scale_exp(const u32* emax_bits)
 //
 // With few row blocks (small n) a row block has a dozen slots, and their sum is a
 // chain of loads: SLOTS of them are in flight at a time, for PER elements per thread.
-// err: the products' error word; after a failed product B_out is left alone.
+// err: the products' error word; after a failed product B_out is left alone. err_host:
+// null, or host memory that the last call copies it to.
 template <class T, int PER, int SLOTS>
 __global__ void __launch_bounds__(1024 / PER) k_combine(u32 n, u32 ld, u32 R, u32 Rpad, const float* __restrict__ partial,
                                                         u32 max_slots, const u32* __restrict__ rp_cnt,
                                                         const float* __restrict__ E, const float* __restrict__ albedo,
                                                         float* __restrict__ B_out, T* __restrict__ xh, T* __restrict__ xl,
-                                                        int g_exp, const u32* __restrict__ emax_bits, const u32* __restrict__ err)
+                                                        int g_exp, const u32* __restrict__ emax_bits, const u32* __restrict__ err,
+                                                        u32* __restrict__ err_host)
 {
     constexpr int ROWSTEP = 32 / PER;
     __shared__ float tile[32][33];
@@ -473,7 +475,9 @@ __global__ void __launch_bounds__(1024 / PER) k_combine(u32 n, u32 ld, u32 R, u3
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int x_exp = x_scale_exp(emax_bits);
     const float unscale = ldexpf(1.0f, -(g_exp + x_exp)), xscale = ldexpf(1.0f, x_exp);
-    const bool store = B_out && *err == 0u;
+    const u32 failed = *err;
+    const bool store = B_out && failed == 0u;
+    if (err_host && blockIdx.x == 0 && blockIdx.y == 0 && tx == 0 && ty == 0) *err_host = failed;
     // the loads of the second phase (E, albedo) go out together with those of the first,
     // so a block waits for about one memory round trip instead of three
     float e[PER], al[PER];
@@ -1096,7 +1100,7 @@ struct ltrg_Gather {
     DevBuf words;                 // [0] error word of the products, [1] largest emission
     DevBuf h_alb, h_E, h_out;     // device copies for the host-buffer entry point
     PinBuf pin_in, pin_out;       // its page-locked staging
-    PinBuf pin_err;               // the error word as read back
+    u32 h_err = 0;                // the error word as read back
     std::vector<cudaEvent_t> events;   // of a solve's timings, used again by the next
     bool grown = false;           // a buffer was allocated since the last wait for `st`
     std::unique_ptr<StagePool> pool;   // its host copy threads (started by the first host-buffer solve)
@@ -1118,7 +1122,6 @@ struct ltrg_Gather {
         for (cudaEvent_t e : events) cudaEventDestroy(e);
         pin_in.release();
         pin_out.release();
-        pin_err.release();
         cudaStreamSynchronize(st);
         // as a destroyed scene does: the pool gives back what it holds beyond 8 GiB
         cudaMemPool_t pool;
@@ -1176,7 +1179,6 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
     if (tc && R > (u32) MAX_BN) throw std::runtime_error("tensor-core gather takes at most 256 right-hand sides");
     if (refine < LTRG_REFINE_NONE || refine > LTRG_REFINE_FULL) throw std::runtime_error("invalid refine level");
     need(words, 8);
-    pin_err.ensure(4);
     u32* d_err = words.as<u32>();
     u32* d_emax = words.as<u32>() + 1;
     size_t ev_used = 0;
@@ -1209,14 +1211,15 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
         bool on;
         ~Wait() { if (on) cudaStreamSynchronize(s); }
     } wait{s, true};
-    // the end of a solve: one wait, after which the error word is on the host
+    // the end of a solve: one wait, after which the products' error word is on the host
+    // (the last slot sum wrote it there where the device can)
+    const bool err_direct = tc && pageable_access(device);
     auto finish = [&]() {
-        GCK(cudaMemcpyAsync(pin_err.p, d_err, 4, cudaMemcpyDeviceToHost, s));
+        if (tc && !err_direct) GCK(cudaMemcpyAsync(&h_err, d_err, 4, cudaMemcpyDeviceToHost, s));
         GCK(cudaStreamSynchronize(s));
         wait.on = false;
-        const u32 herr = *(const u32*) pin_err.p;
-        if (herr)
-            throw std::runtime_error("tensor-core gather: a pipeline wait expired (error word " + std::to_string(herr) + ")");
+        if (tc && h_err)
+            throw std::runtime_error("tensor-core gather: a pipeline wait expired (error word " + std::to_string(h_err) + ")");
     };
     double ms_convert = 0, ms_gemm = 0, ms_bounces = 0;
     int stages = 0, products = 1;
@@ -1353,7 +1356,7 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
             (per == 1 ? k_combine<T, 1, 8> : slots == 4 ? k_combine<T, 4, 4> : k_combine<T, 4, 1>)<<<cg, dim3(32, 32 / per), 0, s>>>(
                 n, ld, R, BN, with_partial ? partial.as<float>() : nullptr, slots_max, rp_cnt, E, alb, last ? out : nullptr,
                 last ? nullptr : xh.as<T>(), (last || refine == LTRG_REFINE_NONE) ? nullptr : xl.as<T>(), g_exp, d_emax,
-                d_err);
+                d_err, last && err_direct ? &h_err : nullptr);
             note_launch();
         };
         auto combine = [&](bool with_partial, bool last) {
