@@ -278,8 +278,9 @@ def run_ours(args, world, rank, local, dist):
     return rays, dev_ms, wall, stats, clocks, stats[-1]["bytes_h2d"], stats[-1]["bytes_d2h"], launches, tuning
 
 
-# algorithmic bytes per lightmap texel of the finalize stage: scatter 13, three dilations x 26, two blur passes x 24
-TEXEL_STAGE_BYTES = 13 + 3 * 26 + 2 * 24
+# algorithmic bytes per lightmap texel of the finalize stage (one kernel): its word of the covered-texel scan, its
+# sample's colour, the finished colour
+TEXEL_STAGE_BYTES = 4 + 16 + 12
 
 # bake radiosity precisions: (name, LTRG_F_*, refine_steps)
 RAD_MODES = (("fp32", 0, 0), ("fp16", 1, 0), ("fp16_refine1", 1, 1), ("bf16", 2, 0), ("bf16_refine1", 2, 1))
@@ -719,11 +720,9 @@ def main():
         "clocks": clocks,
         "s_per_bounce": s0["ms_rad_bounce"] / bounces / 1000.0,
         "texels_per_s": s0["samples"] / (s0["ms_device"] / 1000.0),
-        # the texel stage (scatter, three dilations, two blur passes) over every lightmap texel:
-        # scatter 13 B (colour + mask written), a dilation 26 B (colour + mask read and written),
-        # a blur pass 24 B (colour read and written) per texel
+        # the texel stage (scatter, three dilations and two blur passes in one kernel) over every lightmap texel
         "texel_roofline": {
-            "bound": "hbm", "kernels": "k_scatter, 3 x k_dilate, 2 x k_conv_t (finalize stage)",
+            "bound": "hbm", "kernels": "k_finalize",
             "bytes_per_texel": TEXEL_STAGE_BYTES, "texels": s0["texels"],
             "achieved": s0["texels"] * TEXEL_STAGE_BYTES / (s0["ms_finalize"] / 1000.0) / 1e9 if s0["ms_finalize"] > 0 else 0.0,
             "peak": peak, "unit": "GB/s", "peak_source": peak_kind,

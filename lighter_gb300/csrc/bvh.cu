@@ -298,7 +298,6 @@ __global__ void k_pack_leaves(int nleaf, const u32* __restrict__ ids, const u32*
 // position), so the pairs are totally ordered: the least pair is always mutual
 // (every iteration merges), and a run of equal boxes pairs up (0,1), (2,3), ...
 // and halves each iteration instead of growing a chain.
-
 //
 // All iterations run in one launch: one thread-block cluster, each block owning a
 // contiguous run of the list, with two cluster barriers per iteration (merge
@@ -309,8 +308,9 @@ __global__ void k_pack_leaves(int nleaf, const u32* __restrict__ ids, const u32*
 // many as a cluster takes: 16 where the device can place such a cluster, 8
 // otherwise, fewer for short lists (ploc_launch). Measured, whole kernel: 44,652
 // references 539 us with 8 blocks and a bounds-checked search -> 264 us, the 1.8k-triangle
-// level (22k references) 328 -> 185 us, a 34-triangle room 33 -> 18 us. Launched kernel by kernel (as graphs of eight
-// iterations and a read-back of the count) the same builds took 2.5 and 1.6 ms.
+// level (22k references) 328 -> 185 us, a 34-triangle room 33 -> 18 us. Launched kernel
+// by kernel (as graphs of eight iterations and a read-back of the count) the same
+// builds took 2.5 and 1.6 ms.
 
 constexpr int kPlocR = 16;
 constexpr int kPlocT = 1024;           // threads per block
