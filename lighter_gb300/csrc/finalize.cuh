@@ -10,11 +10,13 @@
 // ext): sweeps and both convolutions run in shared memory, and the tile is
 // written once. The halo re-reads 2.1x the texels, from L2. One lightmap is a
 // block or two per SM, so a block's own chain of latencies is the time: 512
-// threads, four texels per thread read at once, and each thread remembers which
-// of its texels are uncovered, so a sweep touches no others. Measured: 512 x 512
-// at blur 0.5 13.3 us on the device and 16.4 us a call (30.9 and 53.6 as separate
-// kernels; 25.4 a call with 256 threads that rescan the region every sweep),
-// 1024 x 1024 33.8 us (90.5); a bake's stage on four 1024^2 lightmaps 0.34 -> 0.16 ms. The float
+// threads, five texels per thread read at once (the whole region up to ext = 3), and
+// the sweeps go through a list of the uncovered texels, so all lanes have one.
+// Measured: 512 x 512 at blur 0.5 11.0 us on the device and 12.4 us a call (13.3 and 16.4
+// with every thread looking after its own texels, 30.9 and 53.6 as separate
+// kernels), 1024 x 1024 30.8 us (33.8; 90.5); 256 threads 14.1 us at 512 x 512, 384
+// 11.7, 1024 11.0 but 32.3 at 1024 x 1024. A bake's stage on four 1024^2 lightmaps took
+// 0.34 ms as separate kernels and 0.16 with the first form of this. The float
 // expressions and their order are those of the separate kernels, so the
 // results are the same bits.
 #pragma once
@@ -28,13 +30,13 @@ constexpr int kFinMaxExt = 16;   // largest ceil(blur_size) the tile's shared me
 
 struct FinTaps { float k[2 * kFinMaxExt + 1]; };
 
-// Region side (tile + halo) and shared memory: colours, masks, and the rows of
-// the first convolution.
+// Region side (tile + halo) and shared memory: colours, masks, the rows of the
+// first convolution, and the list of uncovered texels.
 inline __host__ __device__ int fin_side(int ext) { return kFinTile + 2 * (6 + ext); }
 inline size_t fin_smem(int ext)
 {
     const size_t s = (size_t) fin_side(ext);
-    return s * s * 12 + (s * s + 15) / 16 * 16 + (ext ? (size_t) kFinTile * (kFinTile + 2 * ext) * 12 : 0);
+    return s * s * 12 + (s * s + 15) / 16 * 16 + (ext ? (size_t) kFinTile * (kFinTile + 2 * ext) * 12 : 0) + s * s * 2;
 }
 
 #ifdef __CUDACC__
@@ -81,24 +83,27 @@ __device__ __forceinline__ void fin_tile(int bx, int by, int w, int h, int ext, 
     float* col = reinterpret_cast<float*>(smem);
     unsigned char* msk = smem + (size_t) side * side * 12;
     float* tmp = reinterpret_cast<float*>(msk + (side * side + 15) / 16 * 16);
+    unsigned short* list = reinterpret_cast<unsigned short*>(tmp + (ext ? kFinTile * (kFinTile + 2 * ext) * 3 : 0));
+    __shared__ unsigned n_open;
+    if (threadIdx.x == 0) n_open = 0;
+    __syncthreads();
     const int x0 = bx * kFinTile - halo, y0 = by * kFinTile - halo;   // the region's corner
     const int n = side * side;
     // i / side for i < n: n < 2^13 and side < 2^7, so the rounded-up reciprocal of 20 bits is exact
     const unsigned rcp = (0xfffffu + (unsigned) side) / (unsigned) side;
-    unsigned open = 0;   // bit k: this thread's texel k (threadIdx.x + k kFinThreads) is uncovered
-    constexpr int kBatch = 4;
+    constexpr int kBatch = 5;   // up to ext = 3 one batch: one wait for memory
     for (int k0 = 0; k0 * kFinThreads < n; k0 += kBatch) {
         float c[kBatch][3];
-        bool set[kBatch];
+        bool set[kBatch], open[kBatch];   // covered; uncovered, and within a sweep's reach
 #pragma unroll
         for (int k = 0; k < kBatch; ++k) {
             const int i = (int) threadIdx.x + (k0 + k) * kFinThreads;
             const int y = (int) ((unsigned) i * rcp >> 20), gx = x0 + i - y * side, gy = y0 + y;
             c[k][0] = c[k][1] = c[k][2] = 0.0f;
-            set[k] = false;
+            set[k] = open[k] = false;
             if (i < n && gx >= 0 && gx < w && gy >= 0 && gy < h) {
                 set[k] = load((size_t) gy * w + gx, c[k]);
-                if (!set[k]) open |= 1u << (k0 + k);
+                open[k] = !set[k] && i - y * side >= 2 && i - y * side < side - 2 && y >= 2 && y < side - 2;
             }
         }
 #pragma unroll
@@ -108,19 +113,24 @@ __device__ __forceinline__ void fin_tile(int bx, int by, int w, int h, int ext, 
                 col[3 * i] = c[k][0]; col[3 * i + 1] = c[k][1]; col[3 * i + 2] = c[k][2];
                 msk[i] = set[k] ? 1 : 0;
             }
+            const unsigned who = __ballot_sync(0xffffffffu, open[k]);
+            unsigned at = 0;
+            if (who && lane == 0) at = atomicAdd(&n_open, (unsigned) __popc(who));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (open[k]) list[at + __popc(who & ((1u << lane) - 1u))] = (unsigned short) i;
         }
     }
-    if (__syncthreads_or(open != 0)) {   // some texel of the image in the region is uncovered
+    __syncthreads();
+    const int opened = (int) n_open;   // texels of the image in the region that a sweep may set
+    if (opened)
         for (int s = 1; s <= 3; ++s) {
-            for (unsigned left = open; left; left &= left - 1) {
-                const int k = __ffs(left) - 1, i = (int) threadIdx.x + k * kFinThreads;
-                const int y = (int) ((unsigned) i * rcp >> 20), x = i - y * side;
-                if (x < 2 * s || y < 2 * s || x >= side - 2 * s || y >= side - 2 * s) continue;
-                if (fin_dilate(msk + i, col + 3 * i, side, s)) open &= ~(1u << k);
+            for (int e = (int) threadIdx.x; e < opened; e += kFinThreads) {
+                const int i = list[e], y = (int) ((unsigned) i * rcp >> 20), x = i - y * side;
+                if (msk[i] || x < 2 * s || y < 2 * s || x >= side - 2 * s || y >= side - 2 * s) continue;
+                fin_dilate(msk + i, col + 3 * i, side, s);
             }
             __syncthreads();
         }
-    }
     const int tx = bx * kFinTile + lane;
     float* res = col;   // the finished tile: 32 rows of 96 floats
     int res_stride = 3 * kFinTile;
