@@ -57,6 +57,22 @@ def test_pairs_against_fp64(gpu, n, R, precision):
     assert np.array_equal(B, again)
 
 
+@pytest.mark.parametrize("chunk", [1, 7, 64])
+def test_pairs_in_chunks(gpu, chunk):
+    """Accumulation in chunks of k blocks: more accumulator hand-overs between the pair's issuer and both epilogues."""
+    n, R = 6657, 192
+    pos, nrm, area, rng = _sphere(n, chunk)
+    albedo = rng.uniform(0.3, 0.8, (n, 3)).astype(np.float32)
+    E = rng.uniform(0.0, 5.0, (n, R)).astype(np.float32)
+    with Gather(gpu, np.zeros((0, 9), np.float32), pos, nrm, area) as g:
+        G16 = _round16(g.G(), FP16)
+        g.set_chunk(chunk)
+        B, st = g.solve(albedo, E, 1, FP16, REFINE_RHS)
+    assert st["ctas"] % 2 == 0 and st["stages"] > 2
+    want = E + G16 @ (albedo.astype(np.float64)[:, np.arange(R) % 3] * E)
+    assert (np.abs(B - want) / want).max() <= 2.0 ** -22 + (n + 16) * 2.0 ** -23
+
+
 def test_pair_wait_expires_and_the_next_solve_succeeds(gpu):
     pos, nrm, area, rng = _sphere(6700, 0)
     albedo = np.full((6700, 3), 0.5, np.float32)
