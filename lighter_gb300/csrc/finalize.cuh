@@ -16,7 +16,7 @@
 // with every thread looking after its own texels, 30.9 and 53.6 as separate
 // kernels), 1024 x 1024 30.8 us (33.8; 90.5); 256 threads 14.1 us at 512 x 512, 384
 // 11.7, 1024 11.0 but 32.3 at 1024 x 1024. A bake's stage on four 1024^2 lightmaps took
-// 0.34 ms as separate kernels and 0.16 with the first form of this. The float
+// 0.34 ms as separate kernels, 0.155 with the first form of this and 0.140 now. The float
 // expressions and their order are those of the separate kernels, so the
 // results are the same bits.
 #pragma once
