@@ -1867,9 +1867,14 @@ __global__ void k_normals(u32 n_probe, u32 n_samples, int n_lights, const float4
 // ----------------------------------------------------------------------------- host helpers
 
 // Device arena: every buffer of one bake, freed (stream-ordered) at the end.
+// A copy from pageable memory may still read it after the call that queued it has
+// returned (it does not have to be staged, above all where the device addresses
+// pageable memory), so what upload() copies has to outlive the stream's work: vectors of
+// the bake's own frame do (SyncAtExit), and others are handed over and kept here.
 struct Arena {
     cudaStream_t st = nullptr;
     std::vector<void*> ptrs;
+    std::vector<std::shared_ptr<void>> kept;
     size_t bytes = 0;
     template <class T> T* alloc(size_t n)
     {
@@ -1886,6 +1891,12 @@ struct Arena {
         if (!v.empty()) CK(cudaMemcpyAsync(d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st));
         note_h2d(v.size() * sizeof(T));
         return d;
+    }
+    template <class T> T* upload(std::vector<T>&& v)
+    {
+        auto own = std::make_shared<std::vector<T>>(std::move(v));
+        kept.push_back(own);
+        return upload(static_cast<const std::vector<T>&>(*own));
     }
     template <class T> T* zeros(size_t n)
     {
@@ -1906,6 +1917,13 @@ struct Arena {
             cudaStreamDestroy(st);
         }
     }
+};
+
+// Waits for the stream on every way out of a frame, before the vectors declared
+// ahead of it (and copied from) go.
+struct SyncAtExit {
+    cudaStream_t st;
+    ~SyncAtExit() { cudaStreamSynchronize(st); }
 };
 
 struct StageClock {
@@ -2204,6 +2222,7 @@ struct BatchCtx {
         std::vector<DirectJob> djobs;
         std::vector<AoJob> ajobs;
         std::vector<unsigned long long> rays;   // AO work items per job (ao_items)
+        std::vector<unsigned long long> off;    // and their offsets (copied from, as the jobs are)
         std::vector<cudaEvent_t> ready;
         cudaEvent_t done = nullptr;
     };
@@ -2404,12 +2423,11 @@ struct BatchCtx {
                                                                                        d_next);
                     note_launch();
                 } else {
-                    std::vector<unsigned long long> off(nj + 1, 0);
-                    for (int k = 0; k < nj; ++k) off[k + 1] = off[k] + ph.rays[k];
+                    ph.off.assign(nj + 1, 0);
+                    for (int k = 0; k < nj; ++k) ph.off[k + 1] = ph.off[k] + ph.rays[k];
                     CK(cudaMemcpyAsync(d_jobs, ph.ajobs.data(), jb, cudaMemcpyHostToDevice, bst));
-                    CK(cudaMemcpyAsync(d_off, off.data(), off.size() * sizeof(unsigned long long),
+                    CK(cudaMemcpyAsync(d_off, ph.off.data(), ph.off.size() * sizeof(unsigned long long),
                                        cudaMemcpyHostToDevice, bst));
-                    // the pageable copies above are staged before they return, so `off` may go
                     const ltrg_Tuning tu = get_tuning(device);
                     const unsigned grid = (unsigned) sms * tu.ao_blocks_per_sm;
                     if (tu.ao_packet)
@@ -2682,6 +2700,8 @@ void run_bake(ltr_Scene* S)
     bin.tri_meta = d_tri_meta;
     bin.tri_local = d_tri_local;
     bin.builder = (int) S->opt.bvh_builder;
+    std::vector<u32> ref_tri;      // its leaf references (copied from until its stream is done)
+    std::vector<float> ref_box;
     struct BvhSide {   // its stream, start/end events, and the BVH's storage, released last
         cudaStream_t st_main = nullptr, st = nullptr;
         cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -2709,8 +2729,6 @@ void run_bake(ltr_Scene* S)
             cudaStream_t bs = bside.st ? bside.st : st;
             if (bs != st) CK(cudaStreamWaitEvent(bs, e_tri, 0));
             CK(cudaEventRecord(bside.e0, bs));
-            std::vector<u32> ref_tri;
-            std::vector<float> ref_box;
             float rmin[3], rmax[3];
             build_refs(tri_xyz, ref_tri, ref_box, rmin, rmax);
             u32* d_ref_tri = nullptr;
@@ -2832,6 +2850,7 @@ void run_bake(ltr_Scene* S)
 
     TRACE("host records done");
     // ---- upload
+    SyncAtExit sources{st};   // the copies below read the vectors above
     cudaEvent_t e_up0 = clock.mark();
     const u32 n_probe = (u32) S->samples.size();
     unsigned char* d_lit = A.upload(lit);
@@ -3216,8 +3235,8 @@ void run_bake(ltr_Scene* S)
             std::vector<float> td, te;
             if (tab && tab->diffuse_rgb) td.assign(tab->diffuse_rgb, tab->diffuse_rgb + 3 * (size_t) count);
             if (tab && tab->emissive_rgb) te.assign(tab->emissive_rgb, tab->emissive_rgb + 3 * (size_t) count);
-            float* d_td = td.empty() ? nullptr : A.upload(td);
-            float* d_te = te.empty() ? nullptr : A.upload(te);
+            float* d_td = td.empty() ? nullptr : A.upload(std::move(td));
+            float* d_te = te.empty() ? nullptr : A.upload(std::move(te));
             k_table_samples<<<(n_samples + kThreads - 1) / kThreads, kThreads, 0, st>>>(
                 n_samples, d_srad, d_sinst, cfg.sample_fn != nullptr && tab != nullptr, count, d_td, d_te, d_diff, d_emis); note_launch();
             CK(cudaGetLastError());
@@ -3372,8 +3391,8 @@ void run_bake(ltr_Scene* S)
                 tile = best;
             }
             const u32 nslots = layout(tile);
-            u32* d_slot_base = A.upload(slot_base);
-            u32* d_ntx = A.upload(ntx);
+            u32* d_slot_base = A.upload(std::move(slot_base));
+            u32* d_ntx = A.upload(std::move(ntx));
             u32* d_occ = A.zeros<u32>(nslots + 1);
             u32* d_slot_scan = A.alloc<u32>(nslots + 1);
             k_patch_slots<<<(n_samples + kThreads - 1) / kThreads, kThreads, 0, st>>>(
@@ -3518,13 +3537,14 @@ void run_bake(ltr_Scene* S)
         if (fin_ext) memcpy(ft.k, taps.data(), taps.size() * sizeof(float));
         const size_t smem = fin_smem(fin_ext);
         if (smem > 48 * 1024) CK(cudaFuncSetAttribute(k_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-        FinInst* d_fin = A.upload(fin);
-        k_finalize<<<(unsigned) n_tiles, kFinThreads, smem, st>>>(d_fin, (int) fin.size(), fin_ext, ft, n_probe, d_scan,
+        const int n_fin = (int) fin.size();
+        FinInst* d_fin = A.upload(std::move(fin));
+        k_finalize<<<(unsigned) n_tiles, kFinThreads, smem, st>>>(d_fin, n_fin, fin_ext, ft, n_probe, d_scan,
                                                                   d_lm, d_img); note_launch();
         CK(cudaGetLastError());
     }
     if (blur_ext > kFinMaxExt) {
-        float* d_taps = A.upload(taps);
+        float* d_taps = A.upload(std::move(taps));
         float* d_tmp = A.alloc<float>(3 * ntex);
         k_conv_t<<<blocks_for(ntex), kThreads, 0, st>>>(ntex, n_inst, d_tex_off, d_inst_w, d_inst_h, 0, blur_ext, d_taps,
                                                         d_img, d_tmp); note_launch();
@@ -3549,7 +3569,7 @@ void run_bake(ltr_Scene* S)
     out_off[n_inst] = nout;
     float* d_out = d_img;
     if (cfg.ds2x && nout) {
-        unsigned long long* d_out_off = A.upload(out_off);
+        unsigned long long* d_out_off = A.upload(std::vector<unsigned long long>(out_off));
         d_out = A.alloc<float>(3 * nout);
         k_ds2x<<<blocks_for(nout), kThreads, 0, st>>>(nout, n_inst, d_out_off, d_tex_off, d_inst_w, d_inst_h, d_img, d_out); note_launch();
         CK(cudaGetLastError());
@@ -3558,8 +3578,8 @@ void run_bake(ltr_Scene* S)
     if (want_normals && nout) {
         std::vector<u32> cap(n_inst);
         for (int i = 0; i < n_inst; ++i) cap[i] = out_w[i] * out_h[i];
-        unsigned long long* d_nout_off = A.upload(out_off);
-        u32* d_cap = A.upload(cap);
+        unsigned long long* d_nout_off = A.upload(std::vector<unsigned long long>(out_off));
+        u32* d_cap = A.upload(std::move(cap));
         d_nimg = A.zeros<float>(4 * nout);
         float amb = brightness(mk(cfg.ambient_color[0], cfg.ambient_color[1], cfg.ambient_color[2]));
         if (n_cov && d_ndir) {

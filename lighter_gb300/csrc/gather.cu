@@ -1438,8 +1438,9 @@ LTRAPI ltrg_Gather* ltrg_GatherCreate(const float* tri_xyz, u32 n_tris, const fl
         std::vector<float> ref_box;
         float cmin[3], cmax[3];
         build_refs_host(xyz, ref_tri, ref_box, cmin, cmax);
+        std::vector<float4> hp(n), hn(n);   // patches: position, unit normal
         std::vector<void*> tmp;
-        struct TmpGuard {
+        struct TmpGuard {   // waits for the copies before the vectors above go
             std::vector<void*>& v; cudaStream_t s;
             ~TmpGuard() { for (void* p : v) cudaFreeAsync(p, s); cudaStreamSynchronize(s); }
         } tg{tmp, st};
@@ -1468,8 +1469,7 @@ LTRAPI ltrg_Gather* ltrg_GatherCreate(const float* tri_xyz, u32 n_tris, const fl
             ~BvhGuard() { if (on) bvh_free(b, s); }
         } bg{bvh, st, bin.n > 0};
 
-        // patches: position, unit normal (normalised as the reference's samples are)
-        std::vector<float4> hp(n), hn(n);
+        // (normalised as the reference's samples are)
         for (u32 i = 0; i < n; ++i) {
             hp[i] = make_float4(pos3[3 * i], pos3[3 * i + 1], pos3[3 * i + 2], 0.0f);
             V3 nn = normalized(mk(nrm3[3 * i], nrm3[3 * i + 1], nrm3[3 * i + 2]));

@@ -50,6 +50,9 @@ LTRAPI LTRBOOL ltrdbg_TraceSegments(const float* tri_xyz, u32 n_tris, const floa
     BvhStorage bvh;
     bool built = false;
     LTRBOOL ok = 1;
+    // copied from until the stream is done
+    std::vector<float> xyz, ref_box;
+    std::vector<u32> meta, local, ref_tri;
     try {
         TCK(cudaSetDevice(device));
         TCK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
@@ -61,11 +64,10 @@ LTRAPI LTRBOOL ltrdbg_TraceSegments(const float* tri_xyz, u32 n_tris, const floa
             if (h && bytes) TCK(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, st));
             return d;
         };
-        std::vector<float> xyz(tri_xyz, tri_xyz + 9 * (size_t) n_tris);
-        std::vector<u32> meta(n_tris, kOccluderBit), local(n_tris);
+        xyz.assign(tri_xyz, tri_xyz + 9 * (size_t) n_tris);
+        meta.assign(n_tris, kOccluderBit);
+        local.resize(n_tris);
         for (u32 i = 0; i < n_tris; ++i) local[i] = i;
-        std::vector<u32> ref_tri;
-        std::vector<float> ref_box;
         float cmin[3] = {0, 0, 0}, cmax[3] = {0, 0, 0};
         build_refs_host(xyz, ref_tri, ref_box, cmin, cmax);
         BvhBuildInput in;
