@@ -3536,7 +3536,7 @@ void run_bake(ltr_Scene* S)
         FinTaps ft = {};
         if (fin_ext) memcpy(ft.k, taps.data(), taps.size() * sizeof(float));
         const size_t smem = fin_smem(fin_ext);
-        if (smem > 48 * 1024) CK(cudaFuncSetAttribute(k_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+        if (smem > 48 * 1024) CK(fin_allow_smem(k_finalize));
         const int n_fin = (int) fin.size();
         FinInst* d_fin = A.upload(std::move(fin));
         k_finalize<<<(unsigned) n_tiles, kFinThreads, smem, st>>>(d_fin, n_fin, fin_ext, ft, n_probe, d_scan,

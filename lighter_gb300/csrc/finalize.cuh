@@ -41,6 +41,15 @@ inline size_t fin_smem(int ext)
 
 #ifdef __CUDACC__
 
+// Lets `kernel` be launched with any halo's shared memory. The limit belongs to the kernel,
+// not to a launch, so it is always the largest: set to one call's size, it could
+// drop between another thread's setting and its launch, which would then be refused.
+template <class K>
+inline cudaError_t fin_allow_smem(K kernel)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) fin_smem(kFinMaxExt));
+}
+
 // One dilation of an unset texel from its set 4-neighbours, each extrapolated
 // linearly (2 c1 - c2) when the next texel out is set too; `m` and `col` point
 // at the texel in the region, `sweep` counts from 1, and a mask byte holds one

@@ -151,9 +151,7 @@ extern "C" LTRAPI int ltrg_FinalizeLightmapNoAlloc(const float* rgb, const unsig
     }
     const unsigned tx = (width + kFinTile - 1) / kFinTile, ty = (height + kFinTile - 1) / kFinTile;
     const size_t smem = fin_smem(ext);
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(k_na_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
-        return LTRG_NOALLOC_ECUDA;
+    if (smem > 48 * 1024 && fin_allow_smem(k_na_finalize) != cudaSuccess) return LTRG_NOALLOC_ECUDA;
     k_na_finalize<<<tx * ty, kFinThreads, smem, st>>>(width, height, tx, ext, taps, rgb, mask, out);
     e = cudaGetLastError();
     return e == cudaSuccess ? LTRG_NOALLOC_OK : LTRG_NOALLOC_ECUDA;
