@@ -1312,7 +1312,8 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
                     : refine == LTRG_REFINE_FULL ? k_umma_gather<32, 1, LTRG_REFINE_FULL>
                     : pair                       ? k_umma_gather<32, 2, LTRG_REFINE_RHS>
                                                  : k_umma_gather<64, 1, LTRG_REFINE_RHS>;
-        GCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+        // the limit is the kernel's, and other gathers' threads set it too: always the same value
+        GCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
         UmmaArgs ua;
         ua.nkb = nkb; ua.n_rp = n_rp; ua.R = R; ua.BN = BN;
         ua.stages = (u32) stages; ua.stage_bytes = stage_bytes;
