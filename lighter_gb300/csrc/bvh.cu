@@ -583,7 +583,7 @@ __global__ void __launch_bounds__(kPlocT) k_ploc(PlocArgs p)
 // largest cluster that the current device can place.
 cudaError_t ploc_launch(const PlocArgs& pa, cudaStream_t st)
 {
-    static std::atomic<int> largest[64];   // per device, 0 = not asked yet
+    static std::atomic<int> largest[64];   // per device (a property of its SMs), 0 = not asked yet
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -609,6 +609,12 @@ cudaError_t ploc_launch(const PlocArgs& pa, cudaStream_t st)
     }
     int ctas = 1;
     while (ctas < most && ctas * kPlocT < pa.n) ctas *= 2;
+    // the permission for more than the portable 8 lives in the context, which a device reset
+    // replaces: given anew for each such launch
+    if (ctas > 8 && cudaFuncSetAttribute(k_ploc, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        ctas = 8;
+    }
     at.val.clusterDim.x = (unsigned) ctas;
     cfg.gridDim = dim3((unsigned) ctas);
     return cudaLaunchKernelEx(&cfg, k_ploc, pa);
