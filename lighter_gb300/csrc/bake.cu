@@ -2565,11 +2565,13 @@ void run_bake(ltr_Scene* S)
         V3 bmn = splat(FLT_MAX), bmx = splat(-FLT_MAX);
         if (!mi->container) {
             ltr_Mesh* me = mi->mesh;
+            size_t n_shadow = 0;   // indices of the shadow parts
+            for (const HostPart& p : me->parts) n_shadow += p.shadow ? p.icount : 0;
+            o.xyz.reserve(3 * n_shadow);
             for (const HostPart& p : me->parts) {
                 if (!p.shadow) continue;
                 const V3* vb = &mi->vpos[p.voff];
                 const u32* ib = &me->idx[p.ioff];
-                o.xyz.reserve(o.xyz.size() + 3 * (size_t) p.icount);
                 for (u32 t = 0; t < p.icount; t += 3) {
                     V3 P1 = vb[ib[t]], P2 = vb[ib[t + 1]], P3 = vb[ib[t + 2]];
                     if (near_zero(cross(P2 - P1, P3 - P1))) continue;   // Triangle::CheckIsUseful
