@@ -2784,6 +2784,8 @@ void run_bake(ltr_Scene* S)
     CK(cudaEventCreate(&bside.e1));
     std::exception_ptr bvh_error;
     HostCounters bvh_counts;
+    volatile int* bvh_status = (volatile int*) abort_host + 1;   // page-locked: the build's status word
+    *bvh_status = 0;
     auto bvh_job = [&]() {
         try {
             CK(cudaSetDevice(S->opt.device));
@@ -2810,6 +2812,10 @@ void run_bake(ltr_Scene* S)
             bin.n = (int) ref_tri.size();
             for (int c = 0; c < 3; ++c) { bin.scene_min[c] = bin.n ? rmin[c] : 0; bin.scene_max[c] = bin.n ? rmax[c] : 0; }
             bvh_build(bin, bvh, bs);
+            if (bvh.status) {
+                CK(cudaMemcpyAsync((void*) bvh_status, bvh.status, sizeof(int), cudaMemcpyDeviceToHost, bs));
+                note_d2h(sizeof(int));
+            }
             CK(cudaEventRecord(bside.e1, bs));
         } catch (...) {
             bvh_error = std::current_exception();
@@ -3104,6 +3110,11 @@ void run_bake(ltr_Scene* S)
     host_counters().h2d += bvh_counts.h2d;
     host_counters().d2h += bvh_counts.d2h;
     if (bside.st) CK(cudaStreamWaitEvent(st, bside.e1, 0));
+    // a failed clustering ends the bake here, before the later stages (and the caller's
+    // sample_fn) run over a tree without a scene; the build mostly ended before the sample
+    // counts were read
+    CK(cudaEventSynchronize(bside.e1));
+    bvh_check_status(*bvh_status);
     S->stats.reserved[0] = (uint64_t) bin.n;   // leaf references
     BvhView bv = bvh.view();
     bv.watertight = S->opt.intersect_mode == LTRG_ISECT_WATERTIGHT ? 1 : 0;
@@ -3665,9 +3676,7 @@ void run_bake(ltr_Scene* S)
 
     // ---- readback
     u32 err_words[8] = {0};
-    int bvh_status = 0;
     Counters cnt;
-    if (bvh.status) { CK(cudaMemcpyAsync(&bvh_status, bvh.status, sizeof(int), cudaMemcpyDeviceToHost, st)); note_d2h(sizeof(int)); }
     CK(cudaMemcpyAsync(err_words, d_err, sizeof(err_words), cudaMemcpyDeviceToHost, st)); note_d2h(sizeof(err_words));
     CK(cudaMemcpyAsync(&cnt, d_cnt, sizeof(Counters), cudaMemcpyDeviceToHost, st)); note_d2h(sizeof(Counters));
     // Outputs land directly in the scene's page-locked buffer (kept across
@@ -3714,7 +3723,6 @@ void run_bake(ltr_Scene* S)
     // the host queues the whole bake and waits here; an ltr_Abort during that
     // wait stopped the trace kernels early, so their outputs are incomplete
     check_abort(S);
-    bvh_check_status(bvh_status);
     static const char* kStageName[4] = {"sample fixup", "direct light", "radiosity", "ambient occlusion"};
     for (int k = 0; k < 4; ++k) {
         if (!err_words[k]) continue;
