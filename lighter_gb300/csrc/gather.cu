@@ -704,13 +704,14 @@ __global__ void __launch_bounds__(SGThreads, SGBlocksPerSM) k_sgemm_bounce(Sgemm
 
 // A bounce's sums: B = E + the tile's slots in order (no slots: B = E), and the next
 // X[j][r] = albedo_j(r mod 3) B (rows of ldr), zero for j >= n or r >= R. B_out and x
-// may be null (not wanted). 32 right-hand sides x 8 patches per block.
+// may be null (not wanted). 32 right-hand sides (along the grid's x, which has room for
+// any number) x 8 patches (y: as many as a matrix in device memory has) per block.
 __global__ void __launch_bounds__(256) k_combine32(u32 n, u32 ldx, u32 ldr, u32 R, u32 BN, u32 tiles_n, u32 nkb, uint64_t total,
                                                    u32 n_cta, u32 max_slots, const float* __restrict__ partial,
                                                    const float* __restrict__ E, const float* __restrict__ albedo,
                                                    float* __restrict__ B_out, float* __restrict__ x_out)
 {
-    const u32 j = blockIdx.x * 8 + threadIdx.y, r0 = blockIdx.y * 32, r = r0 + threadIdx.x;
+    const u32 j = blockIdx.y * 8 + threadIdx.y, r0 = blockIdx.x * 32, r = r0 + threadIdx.x;
     float x = 0.0f;
     if (j < n && r < R) {
         const float e = __ldg(&E[(size_t) j * R + r]), al = __ldg(&albedo[3 * j + r % 3]);
@@ -1238,7 +1239,7 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
         need(x32, (size_t) tiles_n * bn * ldx * 4);
         begin();
         const u32 ldr = tiles_n * bn;
-        const dim3 cb(32, 8), cg((ldx + 7) / 8, ldr / 32);
+        const dim3 cb(32, 8), cg(ldr / 32, (ldx + 7) / 8);
         auto combine = [&](bool with_partial, bool last) {
             k_combine32<<<cg, cb, 0, s>>>(n, ldx, ldr, R, bn, tiles_n, skb, total, sg_cta, slots,
                                           with_partial ? partial.as<float>() : nullptr, E, alb, last ? out : nullptr,
