@@ -704,9 +704,9 @@ __global__ void __launch_bounds__(SGThreads, SGBlocksPerSM) k_sgemm_bounce(Sgemm
 
 // A bounce's sums: B = E + the tile's slots in order (no slots: B = E), and the next
 // X[j][r] = albedo_j(r mod 3) B (rows of ldr), zero for j >= n or r >= R. B_out and x
-// may be null (not wanted). 32 right-hand sides (along the grid's x, which has room for
-// any number) x 8 patches (y: as many as a matrix in device memory has) per block.
-__global__ void __launch_bounds__(256) k_combine32(u32 n, u32 ldx, u32 ldr, u32 R, u32 BN, u32 tiles_n, u32 nkb, uint64_t total,
+// may be null (not wanted); E and B_out have rows of ldb floats. 32 right-hand sides (along the grid's x,
+// which has room for any number) x 8 patches (y: as many as a matrix in device memory has) per block.
+__global__ void __launch_bounds__(256) k_combine32(u32 n, u32 ldx, u32 ldr, u32 ldb, u32 R, u32 BN, u32 tiles_n, u32 nkb, uint64_t total,
                                                    u32 n_cta, u32 max_slots, const float* __restrict__ partial,
                                                    const float* __restrict__ E, const float* __restrict__ albedo,
                                                    float* __restrict__ B_out, float* __restrict__ x_out)
@@ -714,7 +714,7 @@ __global__ void __launch_bounds__(256) k_combine32(u32 n, u32 ldx, u32 ldr, u32 
     const u32 j = blockIdx.y * 8 + threadIdx.y, r0 = blockIdx.x * 32, r = r0 + threadIdx.x;
     float x = 0.0f;
     if (j < n && r < R) {
-        const float e = __ldg(&E[(size_t) j * R + r]), al = __ldg(&albedo[3 * j + r % 3]);
+        const float e = __ldg(&E[(size_t) j * ldb + r]), al = __ldg(&albedo[3 * j + r % 3]);
         float v = 0.0f;
         if (partial) {
             // 8 divides the tile's rows and 32 its BN columns: one product tile for the block
@@ -731,7 +731,7 @@ __global__ void __launch_bounds__(256) k_combine32(u32 n, u32 ldx, u32 ldr, u32 
             }
         }
         const float b = e + v;
-        if (B_out) B_out[(size_t) j * R + r] = b;
+        if (B_out) B_out[(size_t) j * ldb + r] = b;
         x = al * b;
     }
     if (x_out && j < ldx) x_out[(size_t) j * ldr + r] = x;
@@ -748,6 +748,15 @@ int sgemm_tn(u32 R)
         if (c < cost) { cost = c; best = tn; }
     }
     return best;
+}
+
+// Right-hand sides solved at a time: the most whose slots (two per tile where there are
+// many) and X take 1 GiB, so that a solve of any width needs little beside its own arrays.
+// A multiple of 96, which keeps the columns' albedo channels (r mod 3) and whole tiles.
+u32 sgemm_columns(u32 tiles_m, u32 ldx)
+{
+    const uint64_t per96 = (2ull * tiles_m * SGM + ldx) * 96 * 4;
+    return 96 * (u32) std::max<uint64_t>(1, std::min<uint64_t>((1ull << 30) / per96, 40000000));
 }
 
 // ----------------------------------------------------------------------------- G preparation
@@ -1228,39 +1237,57 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
     uint64_t bytes_bounce = 0;
 
     if (!tc) {
-        const int tn = sgemm_tn(R);
-        const u32 bn = 16 * (u32) tn, tiles_n = (R + bn - 1) / bn, tiles_m = (n + SGM - 1) / SGM;
-        const u32 skb = (ldg + SGK - 1) / SGK, ldx = skb * SGK;
-        const uint64_t total = (uint64_t) tiles_m * tiles_n * skb;
-        const u32 sg_cta = (u32) std::min<uint64_t>((uint64_t) sm_count * SGBlocksPerSM, total);
-        // slots: the most ranges that one tile's units can fall into
-        const u32 slots = (u32) std::min<uint64_t>(sg_cta, ((uint64_t) skb * sg_cta + total - 1) / total + 1);
-        need(partial, (size_t) tiles_m * tiles_n * slots * SGM * bn * 4);
-        need(x32, (size_t) tiles_n * bn * ldx * 4);
-        begin();
-        const u32 ldr = tiles_n * bn;
-        const dim3 cb(32, 8), cg(ldr / 32, (ldx + 7) / 8);
-        auto combine = [&](bool with_partial, bool last) {
-            k_combine32<<<cg, cb, 0, s>>>(n, ldx, ldr, R, bn, tiles_n, skb, total, sg_cta, slots,
-                                          with_partial ? partial.as<float>() : nullptr, E, alb, last ? out : nullptr,
-                                          last ? nullptr : x32.as<float>()); note_launch();
-            GCK(cudaGetLastError());
+        const u32 tiles_m = (n + SGM - 1) / SGM, skb = (ldg + SGK - 1) / SGK, ldx = skb * SGK;
+        const u32 wide = sgemm_columns(tiles_m, ldx);
+        struct Run {   // the solve of `w` right-hand sides
+            u32 w;
+            int tn;
+            u32 bn, tiles_n, sg_cta, slots;
+            uint64_t total;
         };
-        const SgemmArgs sa{n, ldg, ldr, skb, tiles_n, slots, total, G32.as<float>(), x32.as<float>(), partial.as<float>()};
-        auto kern = tn == 6 ? k_sgemm_bounce<6> : tn == 4 ? k_sgemm_bounce<4> : k_sgemm_bounce<2>;
-        const size_t sg_smem = (size_t) SGStages * (SGM * SGS + SGK * bn) * 4;
-        GCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sg_smem));
-        ctas_run = (int32_t) sg_cta;
+        auto run_of = [&](u32 w) {
+            Run q;
+            q.w = w;
+            q.tn = sgemm_tn(w);
+            q.bn = 16 * (u32) q.tn;
+            q.tiles_n = (w + q.bn - 1) / q.bn;
+            q.total = (uint64_t) tiles_m * q.tiles_n * skb;
+            q.sg_cta = (u32) std::min<uint64_t>((uint64_t) sm_count * SGBlocksPerSM, q.total);
+            // slots: the most ranges that one tile's units can fall into
+            q.slots = (u32) std::min<uint64_t>(q.sg_cta, ((uint64_t) skb * q.sg_cta + q.total - 1) / q.total + 1);
+            return q;
+        };
+        for (const Run& q : {run_of(std::min(R, wide)), run_of(R > wide && R % wide ? R % wide : std::min(R, wide))}) {
+            need(partial, (size_t) tiles_m * q.tiles_n * q.slots * SGM * q.bn * 4);
+            need(x32, (size_t) q.tiles_n * q.bn * ldx * 4);
+        }
+        begin();
         cudaEvent_t e0 = event();
-        combine(false, bounces == 0);
         std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ge;
-        for (int b = 0; b < bounces; ++b) {
-            cudaEvent_t g0 = event();
-            kern<<<sg_cta, SGThreads, sg_smem, s>>>(sa); note_launch();
-            cudaEvent_t g1 = event();
-            ge.push_back({g0, g1});
-            GCK(cudaGetLastError());
-            combine(true, b + 1 == bounces);
+        for (u32 c = 0; c < R; c += std::min(R - c, wide)) {
+            const Run q = run_of(std::min(R - c, wide));
+            const u32 ldr = q.tiles_n * q.bn;
+            const dim3 cb(32, 8), cg(ldr / 32, (ldx + 7) / 8);
+            auto combine = [&](bool with_partial, bool last) {
+                k_combine32<<<cg, cb, 0, s>>>(n, ldx, ldr, R, q.w, q.bn, q.tiles_n, skb, q.total, q.sg_cta, q.slots,
+                                              with_partial ? partial.as<float>() : nullptr, E + c, alb, last ? out + c : nullptr,
+                                              last ? nullptr : x32.as<float>()); note_launch();
+                GCK(cudaGetLastError());
+            };
+            const SgemmArgs sa{n, ldg, ldr, skb, q.tiles_n, q.slots, q.total, G32.as<float>(), x32.as<float>(), partial.as<float>()};
+            auto kern = q.tn == 6 ? k_sgemm_bounce<6> : q.tn == 4 ? k_sgemm_bounce<4> : k_sgemm_bounce<2>;
+            const size_t sg_smem = (size_t) SGStages * (SGM * SGS + SGK * q.bn) * 4;
+            GCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sg_smem));
+            ctas_run = (int32_t) q.sg_cta;
+            combine(false, bounces == 0);
+            for (int b = 0; b < bounces; ++b) {
+                cudaEvent_t g0 = event();
+                kern<<<q.sg_cta, SGThreads, sg_smem, s>>>(sa); note_launch();
+                cudaEvent_t g1 = event();
+                ge.push_back({g0, g1});
+                GCK(cudaGetLastError());
+                combine(true, b + 1 == bounces);
+            }
         }
         cudaEvent_t e1 = event();
         finish();
