@@ -689,11 +689,12 @@ __global__ void __launch_bounds__(SGThreads, SGBlocksPerSM) k_sgemm_bounce(Sgemm
         if (u + 1 == hi || ck == a.nkb) {   // the end of this block's part of the tile
             const u32 slot = blockIdx.x - range_of((uint64_t) ct * a.nkb, a.total, gridDim.x);
             float* P = a.partial + ((size_t) ct * a.max_slots + slot) * (SGM * BN);
+            const u32 rows = a.n - ct / a.tiles_n * SGM;   // rows past n are not read (8 patches: 128 to a tile)
 #pragma unroll
             for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < TN; ++j) {
-                    P[(ty + 8 * i) * BN + col(j)] = acc[i][j];
+                    if (ty + 8 * i < rows) P[(ty + 8 * i) * BN + col(j)] = acc[i][j];
                     acc[i][j] = 0.0f;
                 }
             ck = 0;
@@ -1267,11 +1268,12 @@ void ltrg_Gather::solve(float* alb, float* E, u32 R, int bounces, int precision,
         for (u32 c = 0; c < R; c += std::min(R - c, wide)) {
             const Run q = run_of(std::min(R - c, wide));
             const u32 ldr = q.tiles_n * q.bn;
-            const dim3 cb(32, 8), cg(ldr / 32, (ldx + 7) / 8);
             auto combine = [&](bool with_partial, bool last) {
-                k_combine32<<<cg, cb, 0, s>>>(n, ldx, ldr, R, q.w, q.bn, q.tiles_n, skb, q.total, q.sg_cta, q.slots,
-                                              with_partial ? partial.as<float>() : nullptr, E + c, alb, last ? out + c : nullptr,
-                                              last ? nullptr : x32.as<float>()); note_launch();
+                const u32 rows = with_partial ? n : ldx;   // X's rows past n are zero from the first call on
+                const dim3 grid(ldr / 32, (rows + 7) / 8), block(32, 8);
+                k_combine32<<<grid, block, 0, s>>>(n, rows, ldr, R, q.w, q.bn, q.tiles_n, skb, q.total, q.sg_cta, q.slots,
+                                                   with_partial ? partial.as<float>() : nullptr, E + c, alb,
+                                                   last ? out + c : nullptr, last ? nullptr : x32.as<float>()); note_launch();
                 GCK(cudaGetLastError());
             };
             const SgemmArgs sa{n, ldg, ldr, skb, q.tiles_n, q.slots, q.total, G32.as<float>(), x32.as<float>(), partial.as<float>()};
