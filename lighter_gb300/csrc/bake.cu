@@ -629,11 +629,14 @@ __global__ void __launch_bounds__(kFixupThreads) k_fix_quick(FixupArgs a)
     }
 }
 
-// Samples from which k_fix_quick pays. Below it a bake's GPU is not full, texels
-// are coarse next to the objects (so most samples near any are listed), and the two
-// kernels run one after the other (a 327k-sample level 1.4 -> 2.1 ms). Above: the
-// benchmark level's 2.4M samples 3.25 -> 1.08 + 1.7 ms, of which the first overlaps the
-// host's tree build, the terrain's 3.9M 9 -> 2.1 + 2.2 ms.
+// Samples from which k_fix_quick pays whatever the scene. Below it a bake's GPU is not
+// full, texels are coarse next to the objects (so most samples near any are listed), and the
+// two kernels run one after the other. Above, the first overlaps the host's tree build.
+// Whole bakes with one light, without / with it, ms:
+//   levels    157k 11.9 / 13.7  399k 16.7 / 17.3  586k 13.4 / 12.9  910k 21.5 / 21.1
+//             1.3M 20.6 / 19.8  2.4M 19.7 / 18.0  (few objects: 2.6M 4.8 / 4.8, 5.3M 8.6 / 8.6)
+//   terrains  248k 14.7 / 14.8  484k 17.1 / 15.5  966k 19.0 / 16.5  1.8M 22.1 / 18.6  3.6M 29.2 / 24.2
+// A single sliver lists every sample (in trace order): terrains 22.1 / 20.4 and 29.3 / 28.0.
 constexpr u32 kFixQuickMin = 1u << 20;
 
 constexpr int kFixupCand = 256;   // candidate instances listed per warp
@@ -2822,10 +2825,9 @@ void run_bake(ltr_Scene* S)
         }
     };
     // A scene of a batch builds on its own thread and stream: the other scenes'
-    // work fills the GPU and the host meanwhile, an extra waiting thread per scene
-    // (the build's read-backs) would take host cores from the scenes still
-    // preparing, and with a second stream per scene the 256-scene batch measured
-    // 5.0 s instead of 0.8 s.
+    // work fills the GPU and the host meanwhile, a further thread per scene would take host
+    // cores from the scenes still preparing, and with a second stream per scene the 256-scene
+    // batch measured 5.0 s instead of 0.8 s.
     std::thread bvh_thread;
     if (batch) {
         bvh_job();
@@ -3176,7 +3178,11 @@ void run_bake(ltr_Scene* S)
         fa.inst_box = A.upload(fix_box);
         // the number of listed samples stays on the device: a few waves of blocks
         unsigned grid = (n_cov + kFixupThreads - 1) / kFixupThreads;
-        if (fa.list) grid = std::min(grid, 152u * 16u);
+        if (fa.list) {
+            int sms = 0;
+            CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, S->opt.device));
+            grid = std::min(grid, 16u * (unsigned) sms);
+        }
         k_fixup<<<grid, kFixupThreads, 0, st>>>(fa); note_launch();
         CK(cudaGetLastError());
         checkpoint("sample fixup");

@@ -176,9 +176,11 @@ __device__ __forceinline__ int get_child(const float4* nodes, size_t i, int s, f
     return __float_as_int(f[12 + s]);
 }
 
-// Nodes of the radix hierarchy; or, after a failed clustering, nodes whose boxes
-// no query enters, so that the kernels queued behind the build end at the root
-// (the failure itself reaches the host with their results).
+// Nodes of the radix hierarchy; or, after a failed clustering, nodes whose children are
+// both leaf 0, so that kernels queued behind the build end at once: their boxes are
+// inside out, which a distance query of finite radius does not enter and a segment
+// does (a slab test takes either order of the planes), and then tests that leaf twice. No
+// other child may stand there. The failure itself is the status word.
 __global__ void k_pack_nodes(const int* __restrict__ status, int n_int, const int* left, const int* right,
                              const float* leaf_box, const float* int_box, float4* nodes)
 {

@@ -723,14 +723,12 @@ __device__ __forceinline__ bool warp_any_hit(const BvhView& b, V3 o, V3 e, bool 
 
 // bvh_closest for the active lanes' segments (the smallest occluder hit
 // fraction, ties to the lower leaf -- a rule that does not depend on the
-// visiting order), each lane shrinking its own limit; *leaf gets the hit
-// triangle's leaf (or -1).
-__device__ __forceinline__ float warp_closest(const BvhView& b, V3 o, V3 e, bool active, ErrFlag err, int* leaf = nullptr)
+// visiting order), each lane shrinking its own limit.
+__device__ __forceinline__ float warp_closest(const BvhView& b, V3 o, V3 e, bool active, ErrFlag err)
 {
     const unsigned full = 0xffffffffu;
     float best = kNoHit;
     int bt = -1;
-    if (leaf) *leaf = -1;
     if (b.n_tris <= 0 || !__any_sync(full, active)) return best;
     const SlabPairs seg(inv_dir(e - o), o);
     float tlimit = active ? 1.0f : -1.0f;
@@ -764,7 +762,6 @@ __device__ __forceinline__ float warp_closest(const BvhView& b, V3 o, V3 e, bool
         if (sp == 0) break;
         cur = wstack_pop(s0, s1, sp);
     }
-    if (leaf) *leaf = bt;
     return best;
 }
 
@@ -852,8 +849,8 @@ struct BvhStorage {
 
 // Builds into `out` on `stream` (allocations with cudaMallocAsync on that stream)
 // without waiting for it. A clustering that cannot go on (unordered costs: boxes
-// with NaN or infinities) leaves a tree no query enters and a nonzero
-// status[0], which the caller reads back with its results.
+// with NaN or infinities) leaves a root from which a walk tests leaf 0 twice at most
+// and a nonzero status[0], which the caller reads back before it uses any result.
 void bvh_build(const BvhBuildInput& in, BvhStorage& out, void* stream);
 // Throws when `status` (a build's status[0], read back) says that it failed.
 void bvh_check_status(int status);
