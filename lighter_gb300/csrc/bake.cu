@@ -105,28 +105,30 @@ void parallel_items(int n, int nt, F&& f)
     if (err) std::rethrow_exception(err);
 }
 
-// The same where an item's time is not known beforehand (it runs the caller's code): one
-// thread is started that takes items, and starts the next thread, only once the items
-// have taken 200 us (about what starting the threads takes) and most are still left. Quick
-// ones end before that: with every thread in from the start, two quads took 80 us
-// longer to bake and a room of 40 instances 300 us.
+// The same where an item's time is not known beforehand (it runs the caller's code): beside
+// the `now` threads that the known work is for, one is started that takes items, and
+// starts the next thread up to nt, only once the items have taken 200 us (about what
+// starting the threads takes) and most are still left. Quick ones end before that: with every
+// thread in from the start, two quads took 80 us longer to bake and a room of 40
+// instances 300 us.
 template <class F>
-void parallel_relay(int n, int nt, F&& f)
+void parallel_relay(int n, int now, int nt, F&& f)
 {
     nt = std::min(nt, n);
+    now = std::min(now, nt);
     std::atomic<int> next(0);
     std::exception_ptr err;
     std::mutex mu;
     std::condition_variable cv;
     bool ended = false;
-    std::vector<std::thread> th((size_t) std::max(nt, 1));   // th[t]: started by thread t, runs as t + 1
-    std::function<void(int)> run = [&](int t) {
-        bool more = t > 0 && t + 1 < nt;
+    std::vector<std::thread> th((size_t) std::max(nt - now, 0));   // th[0] watches, th[t + 1] is started by th[t]
+    std::vector<std::thread> known;
+    auto run = [&](std::function<void()> relay) {
         for (int i = next++; i < n; i = next++) {
             try {
-                if (more && next.load() < n) {
-                    more = false;
-                    th[t] = std::thread(run, t + 1);
+                if (relay && next.load() < n) {
+                    relay();
+                    relay = nullptr;
                 }
                 f(i);
             } catch (...) {
@@ -135,24 +137,37 @@ void parallel_relay(int n, int nt, F&& f)
             }
         }
     };
-    if (nt > 1)
-        th[0] = std::thread([&]() {
-            std::unique_lock<std::mutex> lk(mu);
-            do {
-                if (cv.wait_for(lk, std::chrono::microseconds(200), [&]() { return ended; })) return;
-            } while (2 * std::min(next.load(), n) > n);
-            lk.unlock();
-            run(1);
-        });
-    run(0);
+    std::function<void(size_t)> late = [&](size_t t) {
+        run(t + 1 < th.size() ? std::function<void()>([&, t]() { th[t + 1] = std::thread(late, t + 1); }) : nullptr);
+    };
+    struct Join {   // also when a thread cannot be started
+        std::function<void()> f;
+        ~Join() { f(); }
+    };
     {
-        std::lock_guard<std::mutex> lk(mu);
-        ended = true;
-    }
-    cv.notify_one();
-    for (std::thread& x : th) {   // a thread has ended before the one it started is looked at
-        if (!x.joinable()) break;
-        x.join();
+        Join join{[&]() {
+            {
+                std::lock_guard<std::mutex> lk(mu);
+                ended = true;
+            }
+            cv.notify_one();
+            for (std::thread& x : known) x.join();
+            for (std::thread& x : th) {   // a thread has ended before the one it started is looked at
+                if (!x.joinable()) break;
+                x.join();
+            }
+        }};
+        if (!th.empty())
+            th[0] = std::thread([&]() {
+                std::unique_lock<std::mutex> lk(mu);
+                do {
+                    if (cv.wait_for(lk, std::chrono::microseconds(200), [&]() { return ended; })) return;
+                } while (2 * std::min(next.load(), n) > n);
+                lk.unlock();
+                late(0);
+            });
+        for (int t = 1; t < now; ++t) known.emplace_back(run, nullptr);
+        run(nullptr);
     }
     if (err) std::rethrow_exception(err);
 }
@@ -2602,11 +2617,12 @@ void run_bake(ltr_Scene* S)
         vert_off[i + 1] = vert_off[i] + (S->insts[i]->container ? 0 : S->insts[i]->mesh->pos.size());
     std::unique_ptr<float[]> verts(new float[kVert * std::max<size_t>(vert_off[n_inst], 1)]);
     auto pre = [&](int k) { prexform(S, S->insts[k + 1], verts.get() + kVert * vert_off[k + 1]); };
+    const int work_threads = host_threads(vert_off[n_inst], 1024, 16);
     // a size_fn of the caller's may take any time: instances side by side, as many as there are threads
     if (cfg.size_fn && cfg.size_fn != ltr_DefaultSizeFunc)
-        parallel_relay(n_inst - 1, std::min(16, (int) std::max(1u, std::thread::hardware_concurrency())), pre);
+        parallel_relay(n_inst - 1, work_threads, std::min(16, (int) std::max(1u, std::thread::hardware_concurrency())), pre);
     else
-        parallel_items(n_inst - 1, host_threads(vert_off[n_inst], 1024, 16), pre);
+        parallel_items(n_inst - 1, work_threads, pre);
     check_abort(S);
 
     // ---- host: triangle soup of shadow parts (Job_ColInfo) + instance boxes
@@ -3112,11 +3128,6 @@ void run_bake(ltr_Scene* S)
     host_counters().h2d += bvh_counts.h2d;
     host_counters().d2h += bvh_counts.d2h;
     if (bside.st) CK(cudaStreamWaitEvent(st, bside.e1, 0));
-    // a failed clustering ends the bake here, before the later stages (and the caller's
-    // sample_fn) run over a tree without a scene; the build mostly ended before the sample
-    // counts were read
-    CK(cudaEventSynchronize(bside.e1));
-    bvh_check_status(*bvh_status);
     S->stats.reserved[0] = (uint64_t) bin.n;   // leaf references
     BvhView bv = bvh.view();
     bv.watertight = S->opt.intersect_mode == LTRG_ISECT_WATERTIGHT ? 1 : 0;
@@ -3171,6 +3182,10 @@ void run_bake(ltr_Scene* S)
     reftree_thread.join();
     TRACE("reference trees joined");
     if (reftree_error) std::rethrow_exception(reftree_error);
+    // a failed clustering ends the bake here, before the later stages (and the caller's
+    // sample_fn) run over a tree without a scene; the build mostly ended before the trees above
+    CK(cudaEventSynchronize(bside.e1));
+    bvh_check_status(*bvh_status);
     if (n_cov) {
         fa.ref_nodes = A.upload(ref_nodes);
         fa.ref_items = A.upload(ref_items);
