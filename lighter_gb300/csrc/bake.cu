@@ -3515,8 +3515,10 @@ void run_bake(ltr_Scene* S)
             }
             CK(cudaStreamSynchronize(st));
             u32* d_csr_off = A.alloc<u32>(np + 1);
-            k_patch_offsets<<<(n_cov + kThreads - 1) / kThreads, kThreads, 0, st>>>(n_cov, np, d_keys_out, d_csr_off); note_launch();
-            CK(cudaGetLastError());
+            if (n_cov) {   // none with probes alone: no patches
+                k_patch_offsets<<<(n_cov + kThreads - 1) / kThreads, kThreads, 0, st>>>(n_cov, np, d_keys_out, d_csr_off); note_launch();
+                CK(cudaGetLastError());
+            }
             float4* d_ppos = A.alloc<float4>(np);
             float4* d_pnrm = A.alloc<float4>(np);
             float4* d_pda = A.alloc<float4>(np);
