@@ -193,14 +193,16 @@ def _profile_fields(name):
     return out
 
 
-def _trace_roofline(kernel, profile, items, ms, sm_mhz, n_sm, unit_name):
+def _trace_roofline(kernel, profile, items, ms, sm_mhz, n_sm, unit_name, lm):
     """Roofline block of a BVH trace kernel against the resource it is bound by:
     instruction issue (one warp instruction per scheduler and clock, 4 schedulers
-    per SM). achieved = warp instructions per item (ncu, same scene at a quarter
-    of the texels) x items / the kernel's CUDA-event time; the ncu fractions of
-    the captured launch (issue slots, lanes per instruction, L1) come with it."""
+    per SM). achieved = warp instructions per item x items / the kernel's CUDA-event
+    time. The instructions are ncu's count on this scene at 1024^2 lightmaps, or at
+    512^2 for smaller ones (neighbouring samples share more of their walks the closer
+    they lie, so the count follows the texels); the ncu fractions of the 512^2 launch (issue
+    slots of the active cycles, lanes per instruction, L1) come with it."""
     m = _profile_fields(profile)
-    ipi = m.get("warp_inst_per_item")
+    ipi = m.get("warp_inst_per_item_1024" if lm >= 1024 else "warp_inst_per_item")
     block = {"kernel": kernel, "bound": "issue", "unit": "warp-instructions/s", "items": items,
              "item": unit_name, "kernel_ms": ms, "source": "profiles/" + profile, "ncu": m or None}
     if ipi and ms > 0 and sm_mhz:
@@ -746,9 +748,9 @@ def main():
         n_sm = 152
     line["trace_rooflines"] = {
         "shadow": _trace_roofline("k_direct_trace", "k_direct_trace_mid512.md", s0["shadow_pairs"],
-                                  s0["ms_direct_trace"], clocks.get("sm_mhz"), n_sm, "(sample, light) pair"),
+                                  s0["ms_direct_trace"], clocks.get("sm_mhz"), n_sm, "(sample, light) pair", args.lm),
         "ao": _trace_roofline("k_ao_rays", "k_ao_rays_mid512.md", s0["ao_rays"], s0["ms_ao_trace"],
-                              clocks.get("sm_mhz"), n_sm, "AO ray"),
+                              clocks.get("sm_mhz"), n_sm, "AO ray", args.lm),
     }
     # the resource that binds the dominant kernel, beside its HBM figure
     sh = line["trace_rooflines"]["shadow"]
@@ -759,7 +761,8 @@ def main():
         line["sampled_shadows"] = run_sampled(args, local)
         ss = line["sampled_shadows"]
         ss["roofline"] = _trace_roofline("k_direct_trace (sampled shadows)", "k_direct_trace_sampled_mid512.md",
-                                         ss["shadow_rays"], ss["kernel_ms"], clocks.get("sm_mhz"), n_sm, "shadow ray")
+                                         ss["shadow_rays"], ss["kernel_ms"], clocks.get("sm_mhz"), n_sm, "shadow ray",
+                                         args.lm)
     if not args.no_large and args.scene == "mid":
         line["large_scene"] = run_large(args, local)
     if not args.no_rad_precisions:

@@ -8,7 +8,7 @@ if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
 
 # sources of the reference project (read only; absent where the GPU tests run)
-REF_SRC = os.environ.get("LIGHTER_REF_SRC", "/root/reference")
+REF_SRC = os.environ.get("LIGHTER_REF_SRC", os.path.join(os.path.dirname(ROOT), "reference"))
 
 
 def pytest_configure(config):
