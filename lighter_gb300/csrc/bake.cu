@@ -3319,10 +3319,11 @@ void run_bake(ltr_Scene* S)
         S->stage = "calculating radiosity";
         CK(cudaStreamSynchronize(st2));
         TRACE("sample copies done");
-        float4* d_diff = A.alloc<float4>(n_samples);
-        float4* d_emis = A.alloc<float4>(n_samples);
-        std::vector<float4> hdiff, hemis;
+        float4* d_diff = nullptr;
+        float4* d_emis = nullptr;
         if (gpu_sample_fn) {
+            d_diff = A.alloc<float4>(n_samples);
+            d_emis = A.alloc<float4>(n_samples);
             const ltrg_SampleTable* tab = cfg.sample_fn ? (const ltrg_SampleTable*) cfg.userdata : nullptr;
             u32 count = tab ? tab->count : 0;
             std::vector<float> td, te;
@@ -3334,8 +3335,7 @@ void run_bake(ltr_Scene* S)
                 n_samples, d_srad, d_sinst, cfg.sample_fn != nullptr && tab != nullptr, count, d_td, d_te, d_diff, d_emis); note_launch();
             CK(cudaGetLastError());
         } else {
-        hdiff.resize(n_samples);
-        hemis.resize(n_samples);
+        std::vector<float4> hdiff(n_samples), hemis(n_samples);
         for (int i = 0; i < n_inst; ++i) {
             HostInst* mi = S->insts[i];
             for (u32 k = 0; k < scount[i]; ++k) {
@@ -3381,8 +3381,9 @@ void run_bake(ltr_Scene* S)
                 batch->acquire();
             }
         }
-        CK(cudaMemcpyAsync(d_diff, hdiff.data(), n_samples * sizeof(float4), cudaMemcpyHostToDevice, st2)); note_h2d(n_samples * sizeof(float4));
-        CK(cudaMemcpyAsync(d_emis, hemis.data(), n_samples * sizeof(float4), cudaMemcpyHostToDevice, st2)); note_h2d(n_samples * sizeof(float4));
+        // on the bake's own stream, which the patch kernels follow
+        d_diff = A.upload(std::move(hdiff));
+        d_emis = A.upload(std::move(hemis));
         }
         // per-sample radiosity inputs once direct light is done
         float4* d_rpos = A.alloc<float4>(n_samples);
@@ -3418,14 +3419,9 @@ void run_bake(ltr_Scene* S)
             CK(cudaStreamSynchronize(st));
         };
         if (S->opt.radiosity_patches == 0) {
-            cudaEvent_t up = nullptr;
-            CK(cudaEventCreateWithFlags(&up, cudaEventDisableTiming));
-            CK(cudaEventRecord(up, st2));
-            CK(cudaStreamWaitEvent(st, up, 0));
             k_rad_sample_inputs<<<(n_samples + kThreads - 1) / kThreads, kThreads, 0, st>>>(
                 n_samples, d_spos, d_snrm, d_srad, d_sinst, d_diff, d_emis, d_lm, d_rpos, d_rnrm, d_rda, d_remit); note_launch();
             CK(cudaGetLastError());
-            cudaEventDestroy(up);
             RadDevInputs ri{n_samples, d_rpos, d_rnrm, d_rda, d_remit};
             rad_dump_begin(n_samples);
             rr = radiosity_solve_dev(ri, rs, bv, err_rad, st, d_lm, &S->abort_flag);
